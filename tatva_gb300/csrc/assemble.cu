@@ -29,6 +29,7 @@
 
 #include "tg_common.cuh"
 #include "tg_dispatch.cuh"
+#include "tg_hex.cuh"
 #include "tg_internal.h"
 #include "tg_materials.cuh"
 
@@ -139,6 +140,99 @@ __device__ __forceinline__ void element_generic(
         }
     }
   }
+}
+
+// ------------------------------------------------------------------ Hex8 per-QP element
+// Residual or HVP of a general (trilinear) Hex8 element in the modal form of tg_hex.cuh,
+// one z pair of Gauss points per trip.  The element arithmetic bounds these kernels (the
+// issue slots in FP32, the FP64 pipe in FP64).  Against nodal sums at every point, which
+// this replaces, on jittered bricks: linear-elastic FP32 HVP of 872,640 elements 142 ->
+// 94 us, Neo-Hookean FP64 energy and residual of 84,480 elements 1522 -> 1016 us; FP32
+// error against FP64 2.1e-6 -> 1.5e-6 (differences to corner 0).
+template <int MAT, class T, int MODE>
+__device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (&X)[8][3],
+                                                  T (&U)[8][LawDims<MAT, 3>::V],
+                                                  T (&W)[8][LawDims<MAT, 3>::V],
+                                                  T (&Y)[8][LawDims<MAT, 3>::V]) {
+  using L = Law<MAT, 3, T>;
+  constexpr int V = L::V;
+  constexpr bool NEED_U = MODE == TG_MODE_RESIDUAL || !L::LINEAR;
+  hex_modes8<T, 3>(X);
+  hex_scale_gauss<T, 3>(X);
+  if constexpr (NEED_U) {
+    hex_modes8<T, V>(U);
+    hex_scale_gauss<T, V>(U);
+  }
+  if constexpr (MODE == TG_MODE_HVP) {
+    hex_modes8<T, V>(W);
+    hex_scale_gauss<T, V>(W);
+  }
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+#pragma unroll
+    for (int i = 0; i < V; ++i) Y[m][i] = T(0);
+  // not unrolled: the four pairs differ in two signs, and one pair already holds a
+  // Jacobian, a gradient and a flux per point
+#pragma unroll 1
+  for (int p = 0; p < 4; ++p) {
+    T sx, sy;
+    hex_pair_sides<T>(p, sx, sy);
+    HexPair<T, 3> jx;
+    HexPair<T, V> ju, jw;
+    jx.set(X, sx, sy);
+    if constexpr (NEED_U) ju.set(U, sx, sy);
+    if constexpr (MODE == TG_MODE_HVP) jw.set(W, sx, sy);
+    T F[2][3][V];
+#pragma unroll
+    for (int up = 0; up < 2; ++up) {
+      T J[3][3], R[3][3];  // 8 J and its inverse
+      jx.at(up, J);
+      const T wd = inv3(J, R) * T(1.0 / 512);
+      auto physical = [&](const HexPair<T, V>& f, T (&H)[V][3]) {
+        T D[3][V];
+        f.at(up, D);
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            H[i][d] = fma(R[d][2], D[2][i], fma(R[d][1], D[1][i], R[d][0] * D[0][i]));
+      };
+      T H[V][3], P[V][3];
+      if constexpr (NEED_U) physical(ju, H);
+      if constexpr (MODE == TG_MODE_RESIDUAL) {
+        law.flux(H, P);
+      } else {
+        const auto lin = law.linearize(H);
+        T dH[V][3];
+        physical(jw, dH);
+        lin.dflux(dH, P);
+      }
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) P[i][d] *= wd;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          F[up][k][i] = fma(P[i][2], R[2][k], fma(P[i][1], R[1][k], P[i][0] * R[0][k]));
+      }
+      if constexpr (MODE == TG_MODE_RESIDUAL && MAT == TG_POISSON) {
+        // -f N_a(xi_q) wd: the monomials of the point, g folded like the scaled modes
+        const T c = -(wd * law.source()) * T(0.125), cg = c * T(HEX_GAUSS);
+        const T sz = up ? T(1) : T(-1);
+        Y[0][0] += c;
+        Y[1][0] = fma(cg, sx, Y[1][0]);
+        Y[2][0] = fma(cg, sy, Y[2][0]);
+        Y[4][0] = fma(cg, sz, Y[4][0]);
+        Y[3][0] = fma(cg, sx * sy, Y[3][0]);
+        Y[5][0] = fma(cg, sx * sz, Y[5][0]);
+        Y[6][0] = fma(cg, sy * sz, Y[6][0]);
+        Y[7][0] = fma(cg, sx * sy * sz, Y[7][0]);
+      }
+    }
+    hex_pair_adjoint<T, V>(F, sx, sy, Y);
+  }
+  hex_scale_gauss<T, V>(Y);
+  hex_modes8_adjoint<T, V>(Y);
 }
 
 // ------------------------------------------------------------------ Hex8 affine modal path
@@ -503,9 +597,9 @@ __device__ __forceinline__ void hex_le_modal_box(const T (&r)[3], T detJm, T mu,
 
 template <int ET, int MAT, class T, int MODE, bool AFFINE>
 __device__ __forceinline__ void element_apply(
-    T p0, T p1, const T (&X)[Elem<ET>::NN][Elem<ET>::D],
-    const T (&U)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
-    const T (&W)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
+    T p0, T p1, T (&X)[Elem<ET>::NN][Elem<ET>::D],
+    T (&U)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
+    T (&W)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
     T (&Y)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V]) {
   using E = Elem<ET>;
   if constexpr (AFFINE) {
@@ -526,7 +620,10 @@ __device__ __forceinline__ void element_apply(
     }
   } else {
     const Law<MAT, E::D, T> law(p0, p1);
-    element_generic<ET, MAT, T, MODE>(law, X, U, W, Y);
+    if constexpr (ET == TG_HEX8 && MODE != TG_MODE_DIAG)
+      hex_element_modal<MAT, T, MODE>(law, X, U, W, Y);
+    else
+      element_generic<ET, MAT, T, MODE>(law, X, U, W, Y);
   }
 }
 
@@ -962,24 +1059,61 @@ __global__ void energy_kernel(const T* __restrict__ coords, const int32_t* __res
   }
   const Law<MAT, D, T> law(eparam ? eparam[e] : p0, p1);
   T acc = T(0);
+  if constexpr (ET == TG_HEX8) {
+    hex_modes8<T, 3>(X);
+    hex_scale_gauss<T, 3>(X);
+    const T u0 = U[0][0];
+    hex_modes8<T, V>(U);
+    hex_scale_gauss<T, V>(U);
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+      T sx, sy;
+      hex_pair_sides<T>(p, sx, sy);
+      HexPair<T, 3> jx;
+      HexPair<T, V> ju;
+      jx.set(X, sx, sy);
+      ju.set(U, sx, sy);
 #pragma unroll
-  for (int q = 0; q < E::Q; ++q) {
-    T G[NN][D];
-    const T wd = qp_geometry<ET, T>(q, X, G) * E::template w<T>(q);
-    T H[V][D];
+      for (int up = 0; up < 2; ++up) {
+        T J[3][3], R[3][3], Du[3][V], H[V][3];
+        jx.at(up, J);
+        ju.at(up, Du);
+        const T wd = inv3(J, R) * T(1.0 / 512);
 #pragma unroll
-    for (int i = 0; i < V; ++i)
+        for (int i = 0; i < V; ++i)
 #pragma unroll
-      for (int d = 0; d < D; ++d) {
-        T s = T(0);
+          for (int d = 0; d < 3; ++d)
+            H[i][d] = fma(R[d][2], Du[2][i], fma(R[d][1], Du[1][i], R[d][0] * Du[0][i]));
+        T uq = T(0);
+        if constexpr (MAT == TG_POISSON) {
+          T m[8];
 #pragma unroll
-        for (int a = 0; a < NN; ++a) s += G[a][d] * U[a][i];
-        H[i][d] = s;
+          for (int k = 0; k < 8; ++k) m[k] = U[k][0];
+          uq = hex_value<T>(m, u0, sx, sy, up ? T(1) : T(-1));
+        }
+        acc += wd * law.energy(H, uq);
       }
-    T uq = T(0);
+    }
+  } else {
 #pragma unroll
-    for (int a = 0; a < NN; ++a) uq += E::template N<T>(q, a) * U[a][0];
-    acc += wd * law.energy(H, uq);
+    for (int q = 0; q < E::Q; ++q) {
+      T G[NN][D];
+      const T wd = qp_geometry<ET, T>(q, X, G) * E::template w<T>(q);
+      T H[V][D];
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          T s = T(0);
+#pragma unroll
+          for (int a = 0; a < NN; ++a) s += G[a][d] * U[a][i];
+          H[i][d] = s;
+        }
+      T uq = T(0);
+#pragma unroll
+      for (int a = 0; a < NN; ++a) uq += E::template N<T>(q, a) * U[a][0];
+      acc += wd * law.energy(H, uq);
+    }
   }
   out[e] = acc;
 }
