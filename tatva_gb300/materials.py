@@ -75,7 +75,9 @@ class Energy:
         return self.op.n_nodes * self.n_values
 
     def plan(self):
-        return self._plan_override if self._plan_override is not None else self.op.plan()
+        if self._plan_override is not None:
+            return self._plan_override
+        return self.op.plan(box_kernels=self.kind == _lib.TG_LINEAR_ELASTIC)
 
     def use_plan(self, plan) -> None:
         self._plan_override = plan

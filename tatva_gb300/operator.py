@@ -39,10 +39,12 @@ from typing import Callable, Sequence
 import numpy as np
 import torch
 
-from . import _lib
+from . import _lib, autotune
 from ._device import prec_of, ptr, require_cuda, stream, workspace
 from .element import Element
 from .mesh import Mesh
+from .plan import (DEFAULT_BLOCK_ELEMS, DEFAULT_MAX_LOCAL, DEFAULT_THREADS, SMALL_PLAN_PARTIALS,
+                   BlockPlan, small_mesh_blocks)
 
 
 class Operator:
@@ -132,20 +134,31 @@ class Operator:
         return self._cache["inc"]
 
     def plan(self, block_elems: int | None = None, max_local_nodes: int | None = None,
-             threads: int | None = None):
-        """Element-block plan of the fused kernels (cached per tuning)."""
-        from . import autotune
-        from .plan import BlockPlan, DEFAULT_MAX_LOCAL, DEFAULT_THREADS
-
+             threads: int | None = None, *, box_kernels: bool = True):
+        """Element-block plan of the fused kernels (cached per tuning).  ``box_kernels``:
+        the energy has kernels for 512-element blocks of boxes (linear elasticity)."""
         if block_elems is None and max_local_nodes is None and threads is None:
             cfg = autotune.lookup(self)
-            if cfg == (None, None, None) and self.element.tg_id == _lib.TG_HEX8:
-                # Hex8: 512-element blocks suit the parallelepiped kernels; meshes whose
-                # blocks are mostly general (per-QP path) run faster with 1024 / 128
-                p512 = self.plan(512, DEFAULT_MAX_LOCAL, DEFAULT_THREADS[_lib.TG_HEX8])
-                if 2 * p512.sizes["n_affine_blocks"] >= p512.sizes["n_blocks"]:
-                    return p512
-                return self.plan(1024, DEFAULT_MAX_LOCAL, 128)
+            if cfg == (None, None, None):
+                key = "default_plan_boxes" if box_kernels else "default_plan"
+                if key not in self._cache:
+                    tg_id = self.element.tg_id
+                    cfg = (DEFAULT_BLOCK_ELEMS[tg_id], DEFAULT_MAX_LOCAL, DEFAULT_THREADS[tg_id])
+                    small = small_mesh_blocks(tg_id, self.n_elements)
+                    p = None
+                    if small and not (tg_id == _lib.TG_HEX8 and box_kernels):
+                        p = self._small_plan(small)
+                    if p is None and tg_id == _lib.TG_HEX8:
+                        # Hex8: 512-element blocks suit the parallelepiped kernels; meshes
+                        # whose blocks are mostly general (per-QP path) run faster with
+                        # 1024 / 128 once they have blocks enough
+                        p512 = self.plan(*cfg)
+                        boxes = 2 * p512.sizes["n_affine_blocks"] >= p512.sizes["n_blocks"]
+                        if not boxes:
+                            cfg = (1024, DEFAULT_MAX_LOCAL, 128)
+                            p = self._small_plan(small) if small and box_kernels else None
+                    self._cache[key] = p if p is not None else self.plan(*cfg)
+                return self._cache[key]
             block_elems, max_local_nodes, threads = cfg
         threads = threads or DEFAULT_THREADS[self.element.tg_id]
         key = ("plan", block_elems, max_local_nodes or DEFAULT_MAX_LOCAL, threads)
@@ -156,6 +169,11 @@ class Operator:
                                          max_local_nodes=max_local_nodes or DEFAULT_MAX_LOCAL,
                                          threads=threads)
         return self._cache[key]
+
+    def _small_plan(self, small):
+        """The small-mesh plan, or None when its partial sums outgrow the fixed scratch."""
+        p = self.plan(small[0], DEFAULT_MAX_LOCAL, small[1])
+        return p if p.sizes["n_partials"] <= SMALL_PLAN_PARTIALS else None
 
     def unused_nodes(self) -> torch.Tensor:
         """Nodes that no element references (cached); the fused kernels do not write

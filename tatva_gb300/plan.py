@@ -23,6 +23,32 @@ DEFAULT_BLOCK_ELEMS = {_lib.TG_TRI3: 2048, _lib.TG_TET4: 2048, _lib.TG_HEX8: 512
 DEFAULT_THREADS = {_lib.TG_TRI3: 256, _lib.TG_TET4: 128, _lib.TG_HEX8: 128}
 DEFAULT_MAX_LOCAL = 4096
 
+# Blocks a mesh should be cut into before its blocks get larger: about four CTAs for each
+# of the 152 SMs.  A block's elements pass through one CTA a chunk at a time, so a mesh of
+# few default blocks leaves most SMs idle: Kuhn Tet4 24^3 (82,944 elements) Neo-Hookean
+# HVP in 41 blocks of 2048 231 us (FP64) / 28.7 us (FP32), in 648 of 128 108 / 14.0 us;
+# Hex8 44^3 jittered (85,184) FP64 989 us in 84 blocks of 1024, 627 us in 666 of 128; Tri3
+# 64^2 FP64 34.6 us in 4 blocks, 8.8 us in 128.  Below 64 elements a block is mostly shared
+# nodes, and from about 600,000 elements on the default sizes have blocks enough.
+SMALL_MESH_BLOCKS = 600
+SMALL_BLOCK_ELEMS = (64, 512)
+# Small blocks share more nodes.  The fixed scratch of tg_apply_noalloc has to hold the
+# partial sums of every law and precision (3 values, FP64) for a mesh to take them, so that
+# no plan grows out of it.
+SMALL_PLAN_PARTIALS = (8 << 20) // (3 * 8)
+
+
+def small_mesh_blocks(elem_id: int, n_elems: int):
+    """(block_elems, threads) of a mesh with too few default blocks to fill the GPU, or
+    None where the default block size stands."""
+    lo, hi = SMALL_BLOCK_ELEMS
+    be = lo
+    while 2 * be * SMALL_MESH_BLOCKS <= n_elems:
+        be *= 2
+    if be > hi:
+        return None
+    return be, min(be, 128)
+
 
 class BlockPlan:
     def __init__(self, elem_id: int, elements: np.ndarray, coords: np.ndarray, device,
