@@ -167,10 +167,14 @@ __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (
     hex_modes8<T, V>(W);
     hex_scale_gauss<T, V>(W);
   }
+  constexpr bool NH_HVP = MAT == TG_NEO_HOOKEAN && MODE == TG_MODE_HVP;
 #pragma unroll
   for (int m = 0; m < 8; ++m)
 #pragma unroll
-    for (int i = 0; i < V; ++i) Y[m][i] = T(0);
+    for (int i = 0; i < V; ++i) {
+      Y[m][i] = T(0);
+      if constexpr (NH_HVP) U[m][i] += X[m][i];  // modes of the deformed cell
+    }
   // not unrolled: the four pairs differ in two signs, and one pair already holds a
   // Jacobian, a gradient and a flux per point
 #pragma unroll 1
@@ -187,6 +191,13 @@ __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (
     for (int up = 0; up < 2; ++up) {
       T J[3][3], R[3][3];  // 8 J and its inverse
       jx.at(up, J);
+      if constexpr (NH_HVP) {
+        T j[3][3], D[3][3];
+        ju.at(up, j);
+        jw.at(up, D);
+        nh_hvp_axes<T>(law.mu, law.lam, T(1.0 / 512), J, j, D, F[up]);
+        continue;
+      }
       const T wd = inv3(J, R) * T(1.0 / 512);
       auto physical = [&](const HexPair<T, V>& f, T (&H)[V][3]) {
         T D[3][V];
@@ -233,6 +244,92 @@ __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (
   }
   hex_scale_gauss<T, V>(Y);
   hex_modes8_adjoint<T, V>(Y);
+}
+
+// ------------------------------------------------------------------ simplex element
+// Residual or HVP of a Tri3 / Tet4 element through its edge vectors from node 0: with
+// D_k f = f_{k+1} - f_0 the field gradient is R D (R: inverse of the coordinates' D), the
+// nodal result of nodes 1.. is F_k = wd P R_k and node 0 takes minus their sum.
+template <int ET, int MAT, class T, int MODE>
+__device__ __forceinline__ void simplex_element(
+    const Law<MAT, Elem<ET>::D, T>& law, const T (&X)[Elem<ET>::NN][Elem<ET>::D],
+    const T (&U)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
+    const T (&W)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
+    T (&Y)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V]) {
+  using E = Elem<ET>;
+  using L = Law<MAT, E::D, T>;
+  constexpr int D = E::D, V = L::V;
+  T J[D][D], F[D][V];
+#pragma unroll
+  for (int k = 0; k < D; ++k)
+#pragma unroll
+    for (int d = 0; d < D; ++d) J[k][d] = X[k + 1][d] - X[0][d];
+  T fsrc = T(0);
+  if constexpr (MAT == TG_NEO_HOOKEAN && MODE == TG_MODE_HVP) {
+    T j[3][3], dw[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        j[k][i] = J[k][i] + (U[k + 1][i] - U[0][i]);
+        dw[k][i] = W[k + 1][i] - W[0][i];
+      }
+    nh_hvp_axes<T>(law.mu, law.lam, E::template w<T>(0), J, j, dw, F);
+  } else {
+    T R[D][D];
+    const T wd = invD<T, D>(J, R) * E::template w<T>(0);
+    auto gradient = [&](const T (&f)[E::NN][V], T (&H)[V][D]) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        T e[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) e[k] = f[k + 1][i] - f[0][i];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          T s = R[d][0] * e[0];
+#pragma unroll
+          for (int k = 1; k < D; ++k) s = fma(R[d][k], e[k], s);
+          H[i][d] = s;
+        }
+      }
+    };
+    T H[V][D], P[V][D];
+    if constexpr (MODE == TG_MODE_RESIDUAL || !L::LINEAR) gradient(U, H);
+    if constexpr (MODE == TG_MODE_RESIDUAL) {
+      law.flux(H, P);
+    } else {
+      const auto lin = law.linearize(H);
+      T dH[V][D];
+      gradient(W, dH);
+      lin.dflux(dH, P);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) P[i][d] *= wd;
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        T s = P[i][0] * R[0][k];
+#pragma unroll
+        for (int d = 1; d < D; ++d) s = fma(P[i][d], R[d][k], s);
+        F[k][i] = s;
+      }
+    }
+    if constexpr (MODE == TG_MODE_RESIDUAL && MAT == TG_POISSON) fsrc = wd * law.source();
+  }
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    T s = F[0][i];
+#pragma unroll
+    for (int k = 1; k < D; ++k) s += F[k][i];
+    Y[0][i] = -s;
+#pragma unroll
+    for (int k = 0; k < D; ++k) Y[k + 1][i] = F[k][i];
+  }
+  if constexpr (MODE == TG_MODE_RESIDUAL && MAT == TG_POISSON) {
+#pragma unroll
+    for (int a = 0; a < E::NN; ++a) Y[a][0] -= fsrc * E::template N<T>(0, a);
+  }
 }
 
 // ------------------------------------------------------------------ Hex8 affine modal path
@@ -622,6 +719,8 @@ __device__ __forceinline__ void element_apply(
     const Law<MAT, E::D, T> law(p0, p1);
     if constexpr (ET == TG_HEX8 && MODE != TG_MODE_DIAG)
       hex_element_modal<MAT, T, MODE>(law, X, U, W, Y);
+    else if constexpr (E::SIMPLEX && MODE != TG_MODE_DIAG)
+      simplex_element<ET, MAT, T, MODE>(law, X, U, W, Y);
     else
       element_generic<ET, MAT, T, MODE>(law, X, U, W, Y);
   }

@@ -116,13 +116,14 @@ __device__ __forceinline__ T inv2(const T (&J)[2][2], T (&Ji)[2][2]) {
   return det;
 }
 
+// inverse and determinant of J; r: the reciprocal of the determinant
 template <class T>
-__device__ __forceinline__ T inv3(const T (&J)[3][3], T (&Ji)[3][3]) {
+__device__ __forceinline__ T inv3(const T (&J)[3][3], T (&Ji)[3][3], T& r) {
   const T c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
   const T c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
   const T c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
   const T det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
-  const T r = T(1) / det;
+  r = T(1) / det;
   Ji[0][0] = c00 * r;
   Ji[1][0] = c01 * r;
   Ji[2][0] = c02 * r;
@@ -133,6 +134,11 @@ __device__ __forceinline__ T inv3(const T (&J)[3][3], T (&Ji)[3][3]) {
   Ji[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * r;
   Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
   return det;
+}
+template <class T>
+__device__ __forceinline__ T inv3(const T (&J)[3][3], T (&Ji)[3][3]) {
+  T r;
+  return inv3(J, Ji, r);
 }
 
 template <class T, int D>

@@ -181,4 +181,51 @@ struct Law<TG_NEO_HOOKEAN, 3, T> {
   __device__ T source() const { return T(0); }
 };
 
+// Neo-Hookean HVP at one point, in the element's own coordinates: J and j are the
+// Jacobians of the undeformed and the deformed cell, D of the direction (row k: derivative
+// along reference axis k), all with the same scale.  With the inverses R and r of J and j,
+// the spatial gradient of the direction g = dH F^-1 = sum_m D_m (x) r_m and the metric
+// C = R^T R of the undeformed axes,
+//   F_k = wd dP G_k = wd (mu sum_m C_mk D_m + c1 g^T r_k + lambda tr(g) r_k),
+//   c1 = mu - lambda ln(det j / det J),
+// which is Lin::dflux above without forming F, its inverse or the 3 x 3 products with it.
+template <class T>
+__device__ __forceinline__ void nh_hvp_axes(T mu, T lam, T weight, const T (&J)[3][3],
+                                            const T (&j)[3][3], const T (&D)[3][3],
+                                            T (&F)[3][3]) {
+  T R[3][3], r[3][3], rdet;
+  const T det = inv3(J, R, rdet);
+  const T wd = det * weight;
+  const T dj = inv3(j, r);
+  const T c1 = wd * (mu - lam * log(dj * rdet));
+  const T m = wd * mu;
+  T C[3][3], g[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int b = a; b < 3; ++b) {
+      C[a][b] = m * fma(R[2][a], R[2][b], fma(R[1][a], R[1][b], R[0][a] * R[0][b]));
+      C[b][a] = C[a][b];
+    }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int l = 0; l < 3; ++l)
+      g[i][l] = fma(D[2][i], r[l][2], fma(D[1][i], r[l][1], D[0][i] * r[l][0]));
+  const T lt = wd * lam * (g[0][0] + g[1][1] + g[2][2]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) g[a][i] *= c1;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) g[i][i] += lt;  // (c1 g + lt I)^T r_k
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const T e = fma(C[2][k], D[2][i], fma(C[1][k], D[1][i], C[0][k] * D[0][i]));
+      F[k][i] = fma(g[2][i], r[2][k], fma(g[1][i], r[1][k], fma(g[0][i], r[0][k], e)));
+    }
+}
+
 }  // namespace tg
