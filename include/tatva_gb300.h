@@ -322,6 +322,26 @@ TG_API int tg_compressed_hessian(int elem, int prec, const tg_material* mat, con
                           int64_t n_nodes, const int32_t* conn, int64_t n_elems,
                           const void* u, const int32_t* inc_ptr, const int32_t* inc_idx,
                           const int32_t* dof_colors, int n_colors, void* Jc, void* stream);
+/* H straight into the values of a CSR matrix, without Jc: what tg_compressed_hessian
+ * and tg_decompress give for patterns of the form tg_csr_slots accepts -- per node,
+ * n_vals rows with the same ascending columns, those in groups of the n_vals dofs of one
+ * node, every pair of nodes of an element among them, and the colours of a row all
+ * different.  tg_csr_slots checks that (info, 2 ints on the device: [0] = 0 if accepted,
+ * [1] = the most columns of a row, in nodes) and writes slots[pad * j + b], the position
+ * of corner b's node among the columns of incidence entry j's node (16-byte aligned,
+ * n_elems * nodes_per_elem * pad entries; pad 4 for Tri3 / Tet4, 8 for Hex8).
+ * tg_hessian_csr takes max_deg = info[1]; TG_ERR_UNSUPPORTED where a row block does not
+ * fit in shared memory (16-byte aligned slots, deterministic).                        */
+TG_API int tg_csr_slots(int elem, int n_vals, int64_t n_nodes, const int32_t* conn,
+                        int64_t n_elems, const int32_t* inc_ptr, const int32_t* inc_idx,
+                        const int32_t* indptr, const int32_t* indices, int64_t nnz,
+                        const int32_t* colors, int n_colors, uint16_t* slots, int32_t* info,
+                        void* stream);
+TG_API int tg_hessian_csr(int elem, int prec, const tg_material* mat, const void* coords,
+                          int64_t n_nodes, const int32_t* conn, int64_t n_elems,
+                          const void* u, const int32_t* inc_ptr, const int32_t* inc_idx,
+                          const uint16_t* slots, const int32_t* indptr, int max_deg,
+                          void* data, void* stream);
 /* rows[k] = row of nonzero k; col_colors[k] = colors[indices[k]]   base.py:108-136 */
 TG_API int tg_rows_cols(const int32_t* indptr, const int32_t* indices, const int32_t* colors,
                  int64_t n_rows, int64_t nnz, int32_t* rows, int32_t* col_colors,

@@ -18,78 +18,364 @@
 // writes its consecutive nodes' rows as one contiguous, coalesced block of Jc.
 #include "tg_common.cuh"
 #include "tg_dispatch.cuh"
+#include "tg_hex.cuh"
 #include "tg_materials.cuh"
 
 namespace tg {
 
+// One quadrature point's share of the row block of corner a.  For every law here the
+// tangent block of corners (a, b) is
+//   K_ab[i][k] = wd (mu delta_ik G_a.G_b + c1 g_a[k] g_b[i] + lam g_a[i] g_b[k])
+// with the shape gradients G in the undeformed cell and g = G, c1 = mu (linear elastic),
+// or g the gradients in the deformed cell and c1 = mu - lam ln J (Neo-Hookean: the two
+// F^-T of each term of d2psi/dF2 take G to g); Poisson has the first term alone.  s: the
+// first term, ca = wd c1 g_a, la = wd lam g_a.
+template <int V, int COLS, class T>
+__device__ __forceinline__ void add_tangent_block(T (&rb)[V][COLS], int b, T s, const T (&ca)[V],
+                                                  const T (&la)[V], const T (&gb)[V]) {
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      T v = rb[i][b * V + k];
+      if constexpr (V > 1) v = fma(gb[k], la[i], fma(gb[i], ca[k], v));
+      if (i == k) v += s;
+      rb[i][b * V + k] = v;
+    }
+}
+
 // Row block K_e[(a, i), (b, k)] (i, k < V, b < NN) of element e's tangent at u,
-// acc[i][b V + k]; nid: the element's nodes
+// rb[i][b V + k]; nid: the element's nodes
 template <int ET, int MAT, class T>
 __device__ __forceinline__ void element_row_block(
     const T* __restrict__ coords, const int32_t* __restrict__ conn, const T* __restrict__ u,
     T p0, T p1, const T* __restrict__ eparam, int64_t e, int a,
-    T (&acc)[Law<MAT, Elem<ET>::D, T>::V][Elem<ET>::NN * Law<MAT, Elem<ET>::D, T>::V],
+    T (&rb)[LawDims<MAT, Elem<ET>::D>::V][Elem<ET>::NN * LawDims<MAT, Elem<ET>::D>::V],
     int (&nid)[Elem<ET>::NN]) {
   using E = Elem<ET>;
-  using L = Law<MAT, E::D, T>;
-  constexpr int NN = E::NN, D = E::D, V = L::V;
-  T X[NN][D], U[NN][V];
+  constexpr int NN = E::NN, D = E::D, V = LawDims<MAT, D>::V;
+  constexpr bool NH = MAT == TG_NEO_HOOKEAN;
+  T X[NN][D], U[NN][NH ? 3 : 1];
 #pragma unroll
-  for (int b = 0; b < NN; ++b) {
-    nid[b] = __ldg(conn + e * NN + b);
+  for (int b = 0; b < NN; ++b) nid[b] = __ldg(conn + e * NN + b);
 #pragma unroll
-    for (int d = 0; d < D; ++d) X[b][d] = coords[(int64_t)nid[b] * D + d];
+  for (int b = 0; b < NN; ++b)
 #pragma unroll
-    for (int i = 0; i < V; ++i) U[b][i] = L::LINEAR ? T(0) : u[(int64_t)nid[b] * V + i];
-  }
-  const L law(eparam ? eparam[e] : p0, p1);
+    for (int d = 0; d < D; ++d) {
+      X[b][d] = coords[(int64_t)nid[b] * D + d];
+      if constexpr (NH) U[b][d] = u[(int64_t)nid[b] * 3 + d];
+    }
+  const T mu = eparam ? eparam[e] : p0, lam = MAT == TG_POISSON ? T(0) : p1;
 #pragma unroll
   for (int i = 0; i < V; ++i)
 #pragma unroll
-    for (int c = 0; c < NN * V; ++c) acc[i][c] = T(0);
+    for (int c = 0; c < NN * V; ++c) rb[i][c] = T(0);
+  if constexpr (E::SIMPLEX) {
+    T J[D][D], R[D][D], G[NN][D], g[NN][D];
 #pragma unroll
-  for (int q = 0; q < E::Q; ++q) {
-    T G[NN][D];
-    const T wd = qp_geometry<ET, T>(q, X, G) * E::template w<T>(q);
-    T H[V][D];
+    for (int k = 0; k < D; ++k)
 #pragma unroll
-    for (int i = 0; i < V; ++i)
+      for (int d = 0; d < D; ++d) J[k][d] = X[k + 1][d] - X[0][d];
+    auto nodes_of = [&](const T (&Ri)[D][D], T (&out)[NN][D]) {
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        T s = T(0);
-        if constexpr (!L::LINEAR) {
+        T s0 = T(0);
 #pragma unroll
-          for (int b = 0; b < NN; ++b) s += G[b][d] * U[b][i];
+        for (int k = 0; k < D; ++k) {
+          out[k + 1][d] = Ri[d][k];
+          s0 -= Ri[d][k];
         }
-        H[i][d] = s;
+        out[0][d] = s0;
       }
-    const auto lin = law.linearize(H);
-    T ga[D];
+    };
+    T wd, c1;
+    if constexpr (NH) {
+      T j[3][3], r[3][3], rdet;
+      wd = inv3(J, R, rdet) * E::template w<T>(0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) j[k][d] = J[k][d] + (U[k + 1][d] - U[0][d]);
+      const T dj = inv3(j, r);
+      c1 = wd * (mu - lam * log(dj * rdet));
+      nodes_of(r, g);
+    } else {
+      wd = invD<T, D>(J, R) * E::template w<T>(0);
+      c1 = wd * mu;
+    }
+    nodes_of(R, G);
+    T Ga[D], ca[V], la[V];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      ga[d] = G[0][d];
+      Ga[d] = G[0][d];
+      T ga = NH ? g[0][d] : T(0);
 #pragma unroll
       for (int b = 1; b < NN; ++b)
-        if (b == a) ga[d] = G[b][d];
+        if (b == a) {
+          Ga[d] = G[b][d];
+          if constexpr (NH) ga = g[b][d];
+        }
+      if (!NH) ga = Ga[d];
+      if constexpr (V > 1) {
+        ca[d] = c1 * ga;
+        la[d] = wd * lam * ga;
+      }
+      Ga[d] *= wd * mu;
     }
 #pragma unroll
-    for (int b = 0; b < NN; ++b)
+    for (int b = 0; b < NN; ++b) {
+      T s = Ga[0] * G[b][0];
 #pragma unroll
-      for (int k = 0; k < V; ++k) {
-        T dH[V][D], dP[V][D];
+      for (int d = 1; d < D; ++d) s = fma(Ga[d], G[b][d], s);
+      T gb[V];
 #pragma unroll
-        for (int kk = 0; kk < V; ++kk)
+      for (int i = 0; i < V; ++i) gb[i] = NH ? g[b][i] : G[b][i];
+      add_tangent_block<V, NN * V, T>(rb, b, s, ca, la, gb);
+    }
+  } else {
+    // Hex8, modal form (tg_hex.cuh).  8 dN_b/dxi at a point are products of two of the
+    // factors 1 +- x_l; the metric C = R^T R gives G_a.G_b without forming the G.
+    hex_modes8<T, 3>(X);
+    hex_scale_gauss<T, 3>(X);
+    if constexpr (NH) {
+      hex_modes8<T, 3>(U);
+      hex_scale_gauss<T, 3>(U);
 #pragma unroll
-          for (int d = 0; d < D; ++d) dH[kk][d] = (kk == k) ? G[b][d] : T(0);
-        lin.dflux(dH, dP);
+      for (int m = 0; m < 8; ++m)
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          T s = T(0);
+        for (int d = 0; d < 3; ++d) U[m][d] += X[m][d];  // modes of the deformed cell
+    }
+    const T sa[3] = {T(E::s(a, 0)), T(E::s(a, 1)), T(E::s(a, 2))};
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+      T sx, sy;
+      hex_pair_sides<T>(q & 3, sx, sy);
+      const int up = q >> 2;
+      const T sz = up ? T(1) : T(-1), gp = T(HEX_GAUSS);
+      T J[3][3], R[3][3], r[3][3], rdet;
+      HexPair<T, 3> pr;
+      pr.set(X, sx, sy);
+      pr.at(up, J);
+      const T wd = inv3(J, R, rdet) * T(1.0 / 512);
+      T c1 = wd * mu;
+      if constexpr (NH) {
+        pr.set(U, sx, sy);
+        pr.at(up, J);
+        const T dj = inv3(J, r);
+        c1 = wd * (mu - lam * log(dj * rdet));
+      }
+      // f[l][side]: 1 + s x_l of the corners on that side along axis l
+      const T f[3][2] = {{T(1) - sx * gp, T(1) + sx * gp},
+                         {T(1) - sy * gp, T(1) + sy * gp},
+                         {T(1) - sz * gp, T(1) + sz * gp}};
+      T pa[3];  // 8 dN_a/dxi, corner a at run time
+      {
+        const T fa[3] = {fma(sa[0], sx * gp, T(1)), fma(sa[1], sy * gp, T(1)),
+                         fma(sa[2], sz * gp, T(1))};
+        pa[0] = sa[0] * fa[1] * fa[2];
+        pa[1] = sa[1] * fa[0] * fa[2];
+        pa[2] = sa[2] * fa[0] * fa[1];
+      }
+      T Ca[3], ca[V], la[V];  // wd mu C pa; c1 g_a, lam g_a
+      {
+        T Ga[3];
 #pragma unroll
-          for (int d = 0; d < D; ++d) s += dP[i][d] * ga[d];
-          acc[i][b * V + k] += wd * s;
+        for (int d = 0; d < 3; ++d)
+          Ga[d] = fma(R[d][2], pa[2], fma(R[d][1], pa[1], R[d][0] * pa[0]));
+        const T m = wd * mu;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          Ca[k] = m * fma(R[2][k], Ga[2], fma(R[1][k], Ga[1], R[0][k] * Ga[0]));
+        if constexpr (V > 1) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const T ga = NH ? fma(r[d][2], pa[2], fma(r[d][1], pa[1], r[d][0] * pa[0])) : Ga[d];
+            ca[d] = c1 * ga;
+            la[d] = wd * lam * ga;
+          }
         }
       }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const int b0 = E::s(b, 0) > 0, b1 = E::s(b, 1) > 0, b2 = E::s(b, 2) > 0;
+        const T q0 = f[1][b1] * f[2][b2], q1 = f[0][b0] * f[2][b2], q2 = f[0][b0] * f[1][b1];
+        const T pb[3] = {b0 ? q0 : -q0, b1 ? q1 : -q1, b2 ? q2 : -q2};
+        const T s = fma(Ca[2], pb[2], fma(Ca[1], pb[1], Ca[0] * pb[0]));
+        T gb[V];
+        if constexpr (V > 1) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            if constexpr (NH)
+              gb[d] = fma(r[d][2], pb[2], fma(r[d][1], pb[1], r[d][0] * pb[0]));
+            else
+              gb[d] = fma(R[d][2], pb[2], fma(R[d][1], pb[1], R[d][0] * pb[0]));
+          }
+        } else {
+          gb[0] = T(0);
+        }
+        add_tangent_block<V, NN * V, T>(rb, b, s, ca, la, gb);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ straight into CSR
+// The CSR values without the compressed matrix: thread = node, a warp's 32 nodes = one
+// contiguous run of `data`.  The node's row block (V rows of V deg values, the order of
+// the CSR rows) is accumulated in shared memory with word e of lane l at e 32 + l: every
+// lane stays in its own bank whatever word it adds to, so the scattered adds never
+// conflict.  slots[NP j + b]: position of corner b's node among the columns of incidence
+// entry j's node (tg_csr_slots).  Sums run in incidence order (ascending element).
+// What bounds it is on chip: about 250 arithmetic instructions and 36 shared-memory adds
+// per (Tet4 element, corner) and the gathers of the element's nodes; the data is written
+// once and neither column indices nor colours are read.  Kuhn 56^3 jittered, Neo-Hookean
+// FP32 (1.05 M tets, 24 M values): 201 us; compressed Hessian and decompression, which it
+// replaces on the mesh's own pattern, 717 + 125 us.
+template <int ET>
+constexpr int slot_pad() { return Elem<ET>::NN <= 4 ? 4 : 8; }
+constexpr int CSR_WARPS = 2;   // warps per CTA
+constexpr int CSR_SLAB = 16;   // row words a lane hands over at a time when writing
+
+template <int ET, int MAT, class T>
+__global__ void __launch_bounds__(32 * CSR_WARPS)
+    hessian_csr_kernel(const T* __restrict__ coords, const int32_t* __restrict__ conn,
+                       const T* __restrict__ u, T p0, T p1, const T* __restrict__ eparam,
+                       int64_t n_nodes, const int32_t* __restrict__ inc_ptr,
+                       const int32_t* __restrict__ inc_idx, const uint16_t* __restrict__ slots,
+                       const int32_t* __restrict__ indptr, int row_words, T* __restrict__ data) {
+  using E = Elem<ET>;
+  constexpr int NN = E::NN, V = LawDims<MAT, E::D>::V, NP = slot_pad<ET>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T* acc = reinterpret_cast<T*>(smem_raw) + (size_t)warp * row_words * 32;
+  const int64_t n = ((int64_t)blockIdx.x * CSR_WARPS + warp) * 32 + lane;
+  const bool live = n < n_nodes;
+  const int base = live ? __ldg(indptr + V * n) : 0;
+  const int len = live ? __ldg(indptr + V * n + V) - base : 0;
+  const int L = len / V;  // the length of each of the node's rows
+  for (int k = 0; k < len; ++k) acc[k * 32 + lane] = T(0);
+  const int j1 = live ? __ldg(inc_ptr + n + 1) : 0;
+  for (int j = live ? __ldg(inc_ptr + n) : 0; j < j1; ++j) {
+    const int ea = __ldg(inc_idx + j);
+    const int64_t e = ea / NN;
+    const int a = ea - (int)(e * NN);
+    int sl[NP];
+    load_lconn<NP>(slots + (int64_t)j * NP, sl);
+    T rb[V][NN * V];
+    int nid[NN];
+    element_row_block<ET, MAT, T>(coords, conn, u, p0, p1, eparam, e, a, rb, nid);
+#pragma unroll
+    for (int b = 0; b < NN; ++b) {
+      T* w = acc + (V * sl[b]) * 32 + lane;
+      T t[V][V];
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+#pragma unroll
+        for (int k = 0; k < V; ++k) t[i][k] = w[(i * L + k) * 32];
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+#pragma unroll
+        for (int k = 0; k < V; ++k) w[(i * L + k) * 32] = t[i][k] + rb[i][b * V + k];
+    }
+  }
+  // write-out in slabs of CSR_SLAB words per node: each lane moves its slab from its own
+  // bank to row l of a 32 x CSR_SLAB tile in the same place (columns XORed so that neither
+  // side conflicts), then half a warp writes one node's slab
+  int longest = len;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  const int half = lane >> 4, q = lane & 15;
+  for (int s0 = 0; s0 < longest; s0 += CSR_SLAB) {
+    T* tile = acc + s0 * 32;
+    T v[CSR_SLAB];
+#pragma unroll
+    for (int k = 0; k < CSR_SLAB; ++k) v[k] = tile[k * 32 + lane];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < CSR_SLAB; ++k) tile[lane * CSR_SLAB + (k ^ (lane >> 1))] = v[k];
+    __syncwarp();
+#pragma unroll 4
+    for (int t = 0; t < 16; ++t) {
+      const int m = 2 * t + half;
+      const int bm = __shfl_sync(0xffffffffu, base, m), lm = __shfl_sync(0xffffffffu, len, m);
+      if (s0 + q < lm) data[(int64_t)bm + s0 + q] = tile[m * CSR_SLAB + (q ^ (m >> 1))];
+    }
+  }
+}
+
+// Checks that a CSR pattern has the form hessian_csr_kernel writes and that a colouring
+// separates its columns: per node, V rows of the same ascending columns in groups of V
+// dofs of one node, all of different colours (then Jc[i, colour(j)] is H[i, j] alone).
+// info[0] |= 1 where it does not; info[1]: the most columns (nodes) of a row.  A warp per
+// node; the colours seen so far as bits in shared memory.
+constexpr int SLOT_MAX_COLORS = 1024;
+template <int V>
+__global__ void __launch_bounds__(128)
+    csr_pattern_check_kernel(int64_t n_nodes, int64_t nnz, const int32_t* __restrict__ indptr,
+                             const int32_t* __restrict__ indices,
+                             const int32_t* __restrict__ colors, int n_colors,
+                             int32_t* __restrict__ info) {
+  __shared__ unsigned seen[4][SLOT_MAX_COLORS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = (int64_t)blockIdx.x * 4 + warp;
+  if (n >= n_nodes) return;
+  for (int k = lane; k < SLOT_MAX_COLORS / 32; k += 32) seen[warp][k] = 0u;
+  __syncwarp();
+  const int64_t N = n_nodes * V;
+  const int64_t r0 = __ldg(indptr + V * n);
+  const int64_t L = __ldg(indptr + V * n + 1) - r0;
+  bool good = r0 >= 0 && L >= 0 && L % V == 0 && r0 + V * L <= nnz && (n > 0 || r0 == 0);
+  for (int i = 0; i < V; ++i)
+    good = good && (__ldg(indptr + V * n + i + 1) - __ldg(indptr + V * n + i) == L);
+  if (n == n_nodes - 1) good = good && r0 + V * L == nnz;
+  if (good) {
+    for (int64_t p = lane; p < L; p += 32) {
+      const int64_t c = __ldg(indices + r0 + p);
+      bool ok = c >= 0 && c < N;
+      for (int i = 1; i < V; ++i) ok = ok && __ldg(indices + r0 + i * L + p) == c;
+      if (p % V == 0) ok = ok && c % V == 0 && (p == 0 || __ldg(indices + r0 + p - 1) < c);
+      else ok = ok && __ldg(indices + r0 + p - 1) == c - 1;
+      if (ok) {
+        const int col = __ldg(colors + c);
+        ok = col >= 0 && col < n_colors;
+        if (ok) ok = !(atomicOr(&seen[warp][col >> 5], 1u << (col & 31)) >> (col & 31) & 1u);
+      }
+      good = good && ok;
+    }
+  }
+  if (!good) atomicOr(info, 1);
+  if (lane == 0 && good) atomicMax(info + 1, (int)(L / V));
+}
+
+// slots of the incidence entries (a thread per node); info[0] |= 2 where a node of an
+// element is not among the columns.  Runs after the check, on rows it found ascending.
+template <int ET, int V>
+__global__ void csr_slots_kernel(int64_t n_nodes, const int32_t* __restrict__ conn,
+                                 const int32_t* __restrict__ inc_ptr,
+                                 const int32_t* __restrict__ inc_idx,
+                                 const int32_t* __restrict__ indptr,
+                                 const int32_t* __restrict__ indices,
+                                 uint16_t* __restrict__ slots, int32_t* __restrict__ info) {
+  constexpr int NN = Elem<ET>::NN, NP = slot_pad<ET>();
+  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= n_nodes || (*(volatile int32_t*)info & 1)) return;
+  const int64_t r0 = __ldg(indptr + V * n);
+  const int deg = (int)((__ldg(indptr + V * n + 1) - r0) / V);
+  for (int j = __ldg(inc_ptr + n); j < __ldg(inc_ptr + n + 1); ++j) {
+    const int64_t e = __ldg(inc_idx + j) / NN;
+    for (int b = 0; b < NN; ++b) {
+      const int64_t want = (int64_t)V * __ldg(conn + e * NN + b);
+      int lo = 0, hi = deg;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(indices + r0 + (int64_t)V * mid) < want) lo = mid + 1;
+        else hi = mid;
+      }
+      const bool found = lo < deg && lo < 65536 && __ldg(indices + r0 + (int64_t)V * lo) == want;
+      if (!found) atomicOr(info, 2);
+      slots[(int64_t)j * NP + b] = (uint16_t)(found ? lo : 0);
+    }
+    for (int b = NN; b < NP; ++b) slots[(int64_t)j * NP + b] = 0;
   }
 }
 
@@ -279,6 +565,113 @@ extern "C" int tg_compressed_hessian(int elem, int prec, const tg_material* mat,
                 (T*)Jc);
           }
           return launch_check("tg_compressed_hessian");
+        });
+      }
+    });
+  });
+}
+
+// dofs per node of a law on an element (0: not available)
+static int law_values(int elem, int kind) {
+  if (kind == TG_POISSON) return 1;
+  if (kind == TG_LINEAR_ELASTIC) return elem == TG_TRI3 ? 2 : 3;
+  return (kind == TG_NEO_HOOKEAN && elem != TG_TRI3) ? 3 : 0;
+}
+
+extern "C" int tg_csr_slots(int elem, int n_vals, int64_t n_nodes, const int32_t* conn,
+                            int64_t n_elems, const int32_t* inc_ptr, const int32_t* inc_idx,
+                            const int32_t* indptr, const int32_t* indices, int64_t nnz,
+                            const int32_t* colors, int n_colors, uint16_t* slots, int32_t* info,
+                            void* stream) {
+  TG_TRY(check_sizes(n_elems, n_nodes, n_vals));
+  if (nnz < 0) return set_error(TG_ERR_VALUE, "negative size");
+  if (n_vals > 3 || n_colors < 1 || n_colors > SLOT_MAX_COLORS)
+    return set_error(TG_ERR_UNSUPPORTED, "tg_csr_slots: at most 3 values per node and %d colours",
+                     SLOT_MAX_COLORS);
+  if (n_nodes == 0 || n_elems == 0) return set_error(TG_ERR_UNSUPPORTED, "tg_csr_slots: empty mesh");
+  TG_TRY(check_ptr(conn, "conn"));
+  TG_TRY(check_ptr(inc_ptr, "inc_ptr"));
+  TG_TRY(check_ptr(inc_idx, "inc_idx"));
+  TG_TRY(check_ptr(indptr, "indptr"));
+  TG_TRY(check_ptr(indices, "indices"));
+  TG_TRY(check_ptr(colors, "colors"));
+  TG_TRY(check_ptr(slots, "slots"));
+  TG_TRY(check_ptr(info, "info"));
+  if (reinterpret_cast<uintptr_t>(slots) % 16 != 0)
+    return set_error(TG_ERR_VALUE, "tg_csr_slots: slots must be 16-byte aligned");
+  cudaStream_t st = as_stream(stream);
+  TG_TRY(cuda_check(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st), "tg_csr_slots: info"));
+  return dispatch_elem(elem, [&](auto et) -> int {
+    constexpr int ET = decltype(et)::value;
+    auto go = [&](auto vc) -> int {
+      constexpr int V = decltype(vc)::value;
+      csr_pattern_check_kernel<V><<<grid_for(n_nodes, 4), 128, 0, st>>>(
+          n_nodes, nnz, indptr, indices, colors, n_colors, info);
+      csr_slots_kernel<ET, V><<<grid_for(n_nodes, 128), 128, 0, st>>>(
+          n_nodes, conn, inc_ptr, inc_idx, indptr, indices, slots, info);
+      return launch_check("tg_csr_slots");
+    };
+    if (n_vals == 1) return go(IntC<1>{});
+    if (n_vals == 2) return go(IntC<2>{});
+    return go(IntC<3>{});
+  });
+}
+
+// shared-memory words per lane of a row block of max_deg columns
+static int csr_row_words(int V, int max_deg) {
+  return (V * V * max_deg + CSR_SLAB - 1) / CSR_SLAB * CSR_SLAB;
+}
+
+extern "C" int tg_hessian_csr(int elem, int prec, const tg_material* mat, const void* coords,
+                              int64_t n_nodes, const int32_t* conn, int64_t n_elems,
+                              const void* u, const int32_t* inc_ptr, const int32_t* inc_idx,
+                              const uint16_t* slots, const int32_t* indptr, int max_deg,
+                              void* data, void* stream) {
+  TG_TRY(check_ptr(mat, "mat"));
+  TG_TRY(check_sizes(n_elems, n_nodes, 1));
+  if (n_nodes == 0) return TG_OK;
+  const int values = law_values(elem, mat->kind);
+  if (values == 0) return set_error(TG_ERR_UNSUPPORTED, "Neo-Hookean needs a 3D element");
+  TG_TRY(check_ptr(coords, "coords"));
+  TG_TRY(check_ptr(conn, "conn"));
+  TG_TRY(check_ptr(inc_ptr, "inc_ptr"));
+  TG_TRY(check_ptr(inc_idx, "inc_idx"));
+  TG_TRY(check_ptr(slots, "slots"));
+  TG_TRY(check_ptr(indptr, "indptr"));
+  TG_TRY(check_ptr(data, "data"));
+  if (reinterpret_cast<uintptr_t>(slots) % 16 != 0)
+    return set_error(TG_ERR_VALUE, "tg_hessian_csr: slots must be 16-byte aligned");
+  int dev = 0, cta_bytes = 0;
+  TG_TRY(cuda_check(cudaGetDevice(&dev), "tg_hessian_csr: device"));
+  TG_TRY(cuda_check(cudaDeviceGetAttribute(&cta_bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
+                    "tg_hessian_csr: shared memory per CTA"));
+  const size_t word = prec == TG_F32 ? 4 : 8;
+  if (max_deg < 1 || max_deg > 65536 ||
+      (size_t)csr_row_words(values, max_deg) * 32 * CSR_WARPS * word > (size_t)cta_bytes)
+    return set_error(TG_ERR_UNSUPPORTED, "tg_hessian_csr: rows of %d columns do not fit", max_deg);
+  cudaStream_t st = as_stream(stream);
+  return dispatch_elem(elem, [&](auto et) -> int {
+    constexpr int ET = decltype(et)::value;
+    return dispatch_mat2(mat->kind, [&](auto mk) -> int {
+      constexpr int MAT = decltype(mk)::value;
+      if constexpr (MAT == TG_NEO_HOOKEAN && Elem<ET>::D != 3) {
+        return set_error(TG_ERR_UNSUPPORTED, "Neo-Hookean needs a 3D element");
+      } else {
+        return dispatch_prec(prec, [&](auto t) -> int {
+          using T = decltype(t);
+          constexpr int V = LawDims<MAT, Elem<ET>::D>::V;
+          if (!Law<MAT, Elem<ET>::D, T>::LINEAR) TG_TRY(check_ptr(u, "u"));
+          const int words = csr_row_words(V, max_deg);
+          const size_t smem = (size_t)words * 32 * CSR_WARPS * sizeof(T);
+          auto kern = hessian_csr_kernel<ET, MAT, T>;
+          TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem),
+                            "tg_hessian_csr: shared memory"));
+          kern<<<grid_for(n_nodes, 32 * CSR_WARPS), 32 * CSR_WARPS, smem, st>>>(
+              (const T*)coords, conn, (const T*)u, (T)mat->p0, (T)mat->p1,
+              (const T*)mat->elem_param, n_nodes, inc_ptr, inc_idx, slots, indptr, words,
+              (T*)data);
+          return launch_check("tg_hessian_csr");
         });
       }
     });

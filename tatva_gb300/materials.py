@@ -210,6 +210,48 @@ class Energy:
                   ptr(Jc), stream())
         return Jc
 
+    def csr_slots(self, colored_matrix, n_colors: int):
+        """(slots, max_deg) for ``tangent_csr`` on the pattern and colouring of
+        ``colored_matrix``, or None where it takes the compressed Hessian: patterns that are
+        not node blocks or miss a coupling of the mesh, colourings that do not separate a
+        row's columns, rows too long for shared memory."""
+        cm, op, V = colored_matrix, self.op, self.n_values
+        index = (cm.indptr, cm.indices, cm.colors)
+        if (op.n_elements == 0 or not 1 <= n_colors <= 1024
+                or tuple(cm.shape) != (self.n_dofs, self.n_dofs)
+                or not all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous()
+                           for t in index)
+                or cm.indptr.numel() != self.n_dofs + 1 or cm.colors.numel() != self.n_dofs):
+            return None
+        ip, ii = op.incidence()
+        npe = op.element.n_nodes
+        pad = 4 if npe <= 4 else 8
+        slots = torch.empty(op.n_elements * npe * pad, dtype=torch.int16, device=op.device)
+        info = torch.empty(2, dtype=torch.int32, device=op.device)
+        _lib.call("tg_csr_slots", op.element.tg_id, V, op.n_nodes, ptr(op.mesh.elements),
+                  op.n_elements, ptr(ip), ptr(ii), ptr(cm.indptr), ptr(cm.indices), cm.nnz,
+                  ptr(cm.colors), n_colors, ptr(slots), ptr(info), stream())
+        refused, max_deg = info.tolist()
+        # the kernel's FP64 row blocks of 64 nodes: 227 KB of shared memory
+        if refused or max_deg < 1 or -(-V * V * max_deg // 16) * 16 * 64 * 8 > 227 * 1024:
+            return None
+        return slots, max_deg
+
+    def tangent_csr(self, u: torch.Tensor, colored_matrix, slots) -> torch.Tensor:
+        """CSR values of d2E/du2(u) on the pattern of ``colored_matrix`` (``slots`` from
+        ``csr_slots``), in the dtype of ``u``."""
+        uf = self._flat(u)
+        dtype = uf.dtype
+        op, cm = self.op, colored_matrix
+        ip, ii = op.incidence()
+        data = torch.empty(cm.nnz, dtype=dtype, device=uf.device)
+        m = self.material(dtype)
+        _lib.call("tg_hessian_csr", op.element.tg_id, prec_of(dtype), ctypes.byref(m),
+                  ptr(op.coords_as(dtype)), op.n_nodes, ptr(op.mesh.elements), op.n_elements,
+                  ptr(uf), ptr(ip), ptr(ii), ptr(slots[0]), ptr(cm.indptr), slots[1], ptr(data),
+                  stream())
+        return data
+
     def operator_desc(self, u, fixed=None, dtype=torch.float64):
         """tg_operator_desc for the device solvers (keeps referenced tensors alive)."""
         d = _lib.OperatorDesc()

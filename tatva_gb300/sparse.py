@@ -11,8 +11,10 @@ Drop-in for ``tatva.sparse`` (tatva/sparse/__init__.py):
   in for jax.experimental.sparse).
 * ``compute_rows_cols`` (base.py:108-136) -> ``tg_rows_cols``.
 * ``jacfwd(fn, cm, color_batch_size=None)`` and ``linearized_jacfwd`` (base.py:139-227):
-  - ``fn`` a fused energy residual (``energy.residual`` or the ``Energy`` itself):
-    the compressed Jacobian comes from element tangents (``tg_compressed_hessian``);
+  - ``fn`` a fused energy residual (``energy.residual`` or the ``Energy`` itself): the
+    values come from element tangents, on the energy's own mesh pattern straight into CSR
+    (``tg_hessian_csr``), otherwise through the compressed Jacobian
+    (``tg_compressed_hessian``);
   - any other differentiable torch function: one JVP per colour with the seeds of
     ``colored_jacobian_batch`` (base.py:230-270), JVPs through torch autograd's
     double-backward (``torch.autograd.functional.jvp``).
@@ -170,12 +172,22 @@ def colored_jacobian(fn: Callable, u: torch.Tensor, colors: torch.Tensor, n_colo
 
 def jacfwd(fn: Callable, colored_matrix: ColoredMatrix, *, color_batch_size: int | None = None):
     """Sparse Jacobian of ``fn`` on the pattern of ``colored_matrix`` (base.py:139-176)."""
+    from .materials import Energy
+
     nb_colors = colored_matrix.n_colors
-    rows, col_colors = compute_rows_cols(colored_matrix)
+    require_cuda(colored_matrix.indptr)
+    energy = _fused_energy(fn)
+    # a fused energy on a pattern of its mesh: the values straight from the element tangents
+    slots = (energy.csr_slots(colored_matrix, nb_colors) if isinstance(energy, Energy)
+             else None)
+    row_colors = compute_rows_cols(colored_matrix) if slots is None else None
 
     def _wrapped_jacfwd(u: torch.Tensor, *args, **kwargs) -> ColoredMatrix:
+        if slots is not None and not args and not kwargs:
+            return replace(colored_matrix, data=energy.tangent_csr(u, colored_matrix, slots))
         Jc = colored_jacobian(fn, u, colored_matrix.colors, nb_colors, color_batch_size, *args,
                               **kwargs)
+        rows, col_colors = row_colors or compute_rows_cols(colored_matrix)
         return replace(colored_matrix, data=decompress(Jc, rows, col_colors))
 
     return _wrapped_jacfwd
