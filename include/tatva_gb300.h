@@ -123,6 +123,14 @@ TG_API int tg_grad_transpose(int elem, int prec, const void* flux, const void* c
 TG_API int tg_eval_transpose(int elem, int prec, const void* quad, int64_t n_nodes, int n_vals,
                       const int32_t* conn, int64_t n_elems, const int32_t* inc_ptr,
                       const int32_t* inc_idx, void* out, void* stream);
+/* The same with a workspace (tg_eval_transpose_workspace_bytes, 0 for Tri3 / Tet4): each
+ * Hex8 element's points are summed to its corners once, then per node in the order of the
+ * incidence.                                                                            */
+TG_API size_t tg_eval_transpose_workspace_bytes(int elem, int prec, int64_t n_elems, int n_vals);
+TG_API int tg_eval_transpose_ws(int elem, int prec, const void* quad, int64_t n_nodes, int n_vals,
+                                const int32_t* conn, int64_t n_elems, const int32_t* inc_ptr,
+                                const int32_t* inc_idx, void* out, void* workspace,
+                                size_t workspace_bytes, void* stream);
 
 /* ============================================================================
  * Fused element assembly (K4 residual, K5 HVP, Jacobi diagonal) over a

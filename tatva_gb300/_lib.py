@@ -187,6 +187,8 @@ SIGNATURES = {
     "tg_grad_transpose_workspace_bytes": (S, [I, I, L, I]),
     "tg_grad_transpose": (I, [I, I, P, P, L, I, P, L, P, P, P, P, S, P]),
     "tg_eval_transpose": (I, [I, I, P, L, I, P, L, P, P, P, P]),
+    "tg_eval_transpose_workspace_bytes": (S, [I, I, L, I]),
+    "tg_eval_transpose_ws": (I, [I, I, P, L, I, P, L, P, P, P, P, S, P]),
     "tg_plan_build": (I, [I, P, L, L, P, I, I, I, POINTER(c_void_p)]),
     "tg_plan_sizes": (I, [P, P]),
     "tg_plan_export": (I, [P] + [P] * 12),

@@ -235,9 +235,14 @@ class Operator:
         V = int(math.prod(vshape)) if vshape else 1
         out = torch.empty((self.n_nodes,) + tuple(vshape), dtype=q.dtype, device=q.device)
         ip, ii = self.incidence()
-        _lib.call("tg_eval_transpose", self.element.tg_id, prec_of(q.dtype), ptr(q),
+        nb, ws = 0, None
+        if self.element.tg_id == _lib.TG_HEX8:  # the one-point elements need none
+            nb = _lib.lib().tg_eval_transpose_workspace_bytes(
+                self.element.tg_id, prec_of(q.dtype), self.n_elements, V)
+            ws = workspace(nb, q.device)
+        _lib.call("tg_eval_transpose_ws", self.element.tg_id, prec_of(q.dtype), ptr(q),
                   self.n_nodes, V, ptr(self.mesh.elements), self.n_elements, ptr(ip), ptr(ii),
-                  ptr(out), stream())
+                  ptr(out), ptr(ws), nb, stream())
         return out
 
     def _weights_raw(self, dtype) -> torch.Tensor:
