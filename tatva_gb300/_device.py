@@ -44,7 +44,9 @@ def aligned16(t: torch.Tensor) -> torch.Tensor:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, as an integer handle.  (A call of every
+    entry point: torch.cuda.current_stream() builds a Stream object, 2.9 us against 0.2.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:

@@ -38,6 +38,7 @@ from typing import Callable, Sequence
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib, autotune
 from ._device import prec_of, ptr, require_cuda, stream, workspace
@@ -190,8 +191,7 @@ class Operator:
             raise ValueError(
                 f"nodal values must have leading dimension n_nodes={self.n_nodes}, "
                 f"got shape {tuple(u.shape)}")
-        vshape = tuple(u.shape[1:])
-        return vshape, int(math.prod(vshape)) if vshape else 1
+        return u.shape[1:], u.numel() // u.shape[0]
 
     # ------------------------------------------------------------------ raw kernels
     def _eval_raw(self, u: torch.Tensor) -> torch.Tensor:
@@ -449,6 +449,14 @@ def _needs_grad(t) -> bool:
     return isinstance(t, torch.Tensor) and t.requires_grad and torch.is_grad_enabled()
 
 
+def _plain() -> bool:
+    """Whether a backward pass runs without any further differentiation or transform: no
+    graph of the backward (create_graph), no forward-mode level, no torch.func transform.
+    Its transposes then need no autograd node of their own (about 10 us each)."""
+    return (not torch.is_grad_enabled() and forward_ad._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
+
+
 def _sum_rows_raw(per: torch.Tensor) -> torch.Tensor:
     require_cuda(per)
     per = per.contiguous()
@@ -470,6 +478,8 @@ class _Eval(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if _plain():
+            return ctx.op._eval_t_raw(g, ctx.vshape), None
         return _EvalT.apply(g, ctx.op, ctx.vshape), None
 
 
@@ -492,6 +502,8 @@ class _Grad(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if _plain():
+            return ctx.op._grad_t_raw(g, ctx.vshape), None
         return _GradT.apply(g, ctx.op, ctx.vshape), None
 
 
@@ -514,6 +526,8 @@ class _IntQ(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if _plain():
+            return ctx.op._intq_t_raw(g), None
         return _IntQT.apply(g, ctx.op), None
 
 
@@ -547,6 +561,8 @@ class _Gather(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if _plain():
+            return ctx.op._scatter_raw(g, ctx.vshape), None
         return _Scatter.apply(g, ctx.op, ctx.vshape), None
 
 
