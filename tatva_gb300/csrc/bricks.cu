@@ -25,6 +25,7 @@
 // decomposition, fixed-order dot reductions, no atomics on values -- so a solve
 // gives the same bits alone and in any mix.
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -43,7 +44,7 @@ struct BrickSlot {
   GridCoef<float> c32;
   GridCoef<double> c64;
   int64_t n_nodes, n_dofs;
-  int grid_ctas, chunks;
+  int chunks;
   const double* b;
   double* x;
   const uint8_t* fixed;  // one byte per dof (or NULL)
@@ -127,12 +128,16 @@ __device__ __forceinline__ void reslot(const Launch& L, int& e, int& s, BrickSlo
   count = L.off[e + 1] - L.off[e];
 }
 
+// the slot's stencil into shared memory: the face stencils only for the face CTAs (b: this
+// CTA's index in the brick's launch)
 template <class T>
-__device__ __forceinline__ void copy_words(T* dst, const T* src) {
-  static_assert(sizeof(T) % 4 == 0, "word copy");
+__device__ __forceinline__ void copy_coefficients(GridCoef<T>* dst, const GridCoef<T>* src, int b) {
+  constexpr int HEAD = offsetof(GridCoef<T>, fx) / 4, ALL = sizeof(GridCoef<T>) / 4;
+  static_assert(offsetof(GridCoef<T>, fx) % 4 == 0 && sizeof(GridCoef<T>) % 4 == 0, "word copy");
   const unsigned* s = reinterpret_cast<const unsigned*>(src);
   unsigned* d = reinterpret_cast<unsigned*>(dst);
-  for (int i = threadIdx.x; i < (int)(sizeof(T) / 4); i += blockDim.x) d[i] = s[i];
+  const int n = grid_is_interior(*src, b) ? HEAD : ALL;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
 }
 
 __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
@@ -200,32 +205,22 @@ __global__ void __launch_bounds__(256) brick_xupdate_kernel(const __grid_constan
 
 // r64 = b - A64 x (FP64 grid stencil, Dirichlet rows identity) and |r64|; the slot's
 // last CTA decides: DONE, FAILED, or a restart of the inner solve at scale |r64|
-__global__ void __launch_bounds__(GR_THREADS, 2)
+__global__ void __launch_bounds__(grid_threads<double>(), 2)
     brick_resid_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
                        tg_brick_state* __restrict__ st) {
+  constexpr int GR_THREADS = grid_threads<double>();
   __shared__ GridCoef<double> P;
-  __shared__ double4 sm[2 * GR_PLANE];
+  __shared__ GridShared<double> sh;
   int e = find_entry(L, blockIdx.x);
   int s = L.slot[e];
   if (st[s].phase != PH_REFINE) return;
   BrickSlot* S = slots + s;
   int b = blockIdx.x - L.off[e], count = L.off[e + 1] - L.off[e];
-  copy_words(&P, &S->c64);
+  copy_coefficients(&P, &S->c64, b);
   __syncthreads();
   GridDotAcc<double> dot;
-  {
-    const double* x = S->x;
-    if (b < P.n_boundary_ctas)
-      grid_boundary<double, TG_MODE_HVP, MASK_NODE, true, EPI_RESID>(
-          P, (int64_t)b * GR_BNODES, x, x, S->nmask, S->r64, reinterpret_cast<double*>(sm), dot,
-          S->b);
-    else if (b < P.n_boundary_ctas + P.n_xface_ctas)
-      grid_xface<double, TG_MODE_HVP, MASK_NODE, true, EPI_RESID>(
-          P, b - P.n_boundary_ctas, x, x, S->nmask, S->r64, sm, dot, S->b);
-    else
-      grid_interior<double, TG_MODE_HVP, MASK_NODE, true, EPI_RESID>(
-          P, b - P.n_boundary_ctas - P.n_xface_ctas, x, x, S->nmask, S->r64, sm, dot, S->b);
-  }
+  grid_cta<double, TG_MODE_HVP, MASK_NODE, true, EPI_RESID>(P, b, S->x, S->x, S->nmask, S->r64,
+                                                            sh, dot, S->b);
   double v[1] = {dot.value()};
   reslot(L, e, s, S, b, count, slots);
   block_reduce_store<1, GR_THREADS>(v, S->part + b);
@@ -300,32 +295,21 @@ __global__ void __launch_bounds__(DOT_THREADS)
 
 // ------------------------------------------------------------------ one CG step
 // q = A32 p (grid stencil, Dirichlet rows identity) with p.q; last CTA: alpha
-__global__ void __launch_bounds__(GR_THREADS, TG_GRID_MINB)
+__global__ void __launch_bounds__(grid_threads<float>(), grid_ctas_per_sm<float>())
     brick_hvp_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
                      tg_brick_state* __restrict__ st) {
+  constexpr int GR_THREADS = grid_threads<float>();
   __shared__ GridCoef<float> P;
-  __shared__ float4 sm[2 * GR_PLANE];
+  __shared__ GridShared<float> sh;
   int e = find_entry(L, blockIdx.x);
   int s = L.slot[e];
   if (st[s].phase != PH_RUN) return;
   BrickSlot* S = slots + s;
   int b = blockIdx.x - L.off[e], count = L.off[e + 1] - L.off[e];
-  copy_words(&P, &S->c32);
+  copy_coefficients(&P, &S->c32, b);
   __syncthreads();
   GridDotAcc<float> dot;
-  {
-    const float* p = S->p;
-    if (b < P.n_boundary_ctas)
-      grid_boundary<float, TG_MODE_HVP, MASK_NODE_OUT, true>(P, (int64_t)b * GR_BNODES, p, p,
-                                                             S->nmask, S->q,
-                                                             reinterpret_cast<float*>(sm), dot);
-    else if (b < P.n_boundary_ctas + P.n_xface_ctas)
-      grid_xface<float, TG_MODE_HVP, MASK_NODE_OUT, true>(P, b - P.n_boundary_ctas, p, p,
-                                                          S->nmask, S->q, sm, dot);
-    else
-      grid_interior<float, TG_MODE_HVP, MASK_NODE_OUT, true>(
-          P, b - P.n_boundary_ctas - P.n_xface_ctas, p, p, S->nmask, S->q, sm, dot);
-  }
+  grid_cta<float, TG_MODE_HVP, MASK_NODE_OUT, true>(P, b, S->p, S->p, S->nmask, S->q, sh, dot);
   double v[1] = {dot.value()};
   reslot(L, e, s, S, b, count, slots);  // recomputed: not held in registers across the sweep
   block_reduce_store<1, GR_THREADS>(v, S->part + b);
@@ -443,15 +427,17 @@ int brick_chunks(int64_t n_dofs) {
   return (int)(c < 1 ? 1 : (c > DOT_CHUNKS ? DOT_CHUNKS : c));
 }
 
+template <class T>
 int64_t brick_grid_ctas(const int32_t nodes[3]) {
-  GridCoef<float> P;
+  GridCoef<T> P;
   const double h[3] = {1.0, 1.0, 1.0};
-  return grid_setup_dims<float>(nodes, h, 1.0, 1.0, P, true);
+  return grid_setup_dims<T>(nodes, h, 1.0, 1.0, P, true);
 }
 
 size_t brick_part_doubles(const int32_t nodes[3]) {
   const int64_t n = 3 * (int64_t)nodes[0] * nodes[1] * nodes[2];
-  const int64_t g = brick_grid_ctas(nodes), c = 2 * (int64_t)brick_chunks(n);
+  const int64_t g32 = brick_grid_ctas<float>(nodes), g64 = brick_grid_ctas<double>(nodes);
+  const int64_t g = g32 > g64 ? g32 : g64, c = 2 * (int64_t)brick_chunks(n);
   return (size_t)(g > c ? g : c);
 }
 
@@ -468,7 +454,8 @@ struct tg_brick_batch {
   tg_brick_state* d_state = nullptr;
   tg_brick_state* h_state = nullptr;  // pinned
   bool used[TG_BRICK_MAX_SLOTS] = {};
-  int grid_ctas[TG_BRICK_MAX_SLOTS] = {};
+  int grid32_ctas[TG_BRICK_MAX_SLOTS] = {};
+  int grid64_ctas[TG_BRICK_MAX_SLOTS] = {};
   int chunks[TG_BRICK_MAX_SLOTS] = {};
   std::vector<int> admitted;
   // the last step's launches as a CUDA graph, replayed while the slots in use and the
@@ -557,11 +544,10 @@ extern "C" int tg_brick_admit(tg_brick_batch* bt, const tg_brick_request* req, v
   std::memset(&h, 0, sizeof(h));
   const int64_t g32 = grid_setup_dims<float>(nd, req->h, req->mu, req->lam, h.c32, true);
   const int64_t g64 = grid_setup_dims<double>(nd, req->h, req->mu, req->lam, h.c64, true);
-  if (g32 <= 0 || g64 != g32 || g32 > 0x3fffffff)
+  if (g32 <= 0 || g64 <= 0 || g32 > 0x3fffffff || g64 > 0x3fffffff)
     return set_error(TG_ERR_VALUE, "tg_brick_admit: brick too large");
   h.n_nodes = (int64_t)nd[0] * nd[1] * nd[2];
   h.n_dofs = 3 * h.n_nodes;
-  h.grid_ctas = (int)g32;
   h.chunks = brick_chunks(h.n_dofs);
   h.b = req->b;
   h.x = req->x;
@@ -596,7 +582,8 @@ extern "C" int tg_brick_admit(tg_brick_batch* bt, const tg_brick_request* req, v
   TG_TRY(cuda_check(cudaMemcpyAsync(bt->d_state + s, &q, sizeof(q), cudaMemcpyHostToDevice, st),
                     "brick admit: state"));
   bt->used[s] = true;
-  bt->grid_ctas[s] = h.grid_ctas;
+  bt->grid32_ctas[s] = (int)g32;
+  bt->grid64_ctas[s] = (int)g64;
   bt->chunks[s] = h.chunks;
   bt->admitted.push_back(s);
   bt->exec_stale = true;
@@ -630,10 +617,12 @@ extern "C" int tg_brick_step(tg_brick_batch* bt, int iterations, void* stream) {
     if (bt->used[i]) active.push_back(i);
   if (active.empty()) return TG_OK;
   cudaStream_t st = as_stream(stream);
-  int64_t ng = 0, nc = 0, na = 0;
-  const Launch Lg = make_launch(active, bt->grid_ctas, &ng);
+  int64_t n32 = 0, n64 = 0, nc = 0, na = 0;
+  const Launch L32 = make_launch(active, bt->grid32_ctas, &n32);
+  const Launch L64 = make_launch(active, bt->grid64_ctas, &n64);
   const Launch Lc = make_launch(active, bt->chunks, &nc);
-  if (ng > 0x7fffffff) return set_error(TG_ERR_VALUE, "tg_brick_step: too many CTAs");
+  if (n32 > 0x7fffffff || n64 > 0x7fffffff)
+    return set_error(TG_ERR_VALUE, "tg_brick_step: too many CTAs");
   if (!bt->admitted.empty()) {
     const Launch La = make_launch(bt->admitted, bt->chunks, &na);
     brick_admit_kernel<<<(unsigned)na, 256, 0, st>>>(La, bt->d_slots);
@@ -642,10 +631,12 @@ extern "C" int tg_brick_step(tg_brick_batch* bt, int iterations, void* stream) {
   }
   auto enqueue = [&]() {
     brick_xupdate_kernel<<<(unsigned)nc, 256, 0, st>>>(Lc, bt->d_slots, bt->d_state);
-    brick_resid_kernel<<<(unsigned)ng, GR_THREADS, 0, st>>>(Lg, bt->d_slots, bt->d_state);
+    brick_resid_kernel<<<(unsigned)n64, grid_threads<double>(), 0, st>>>(L64, bt->d_slots,
+                                                                         bt->d_state);
     brick_restart_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
     for (int it = 0; it < iterations; ++it) {
-      brick_hvp_kernel<<<(unsigned)ng, GR_THREADS, 0, st>>>(Lg, bt->d_slots, bt->d_state);
+      brick_hvp_kernel<<<(unsigned)n32, grid_threads<float>(), 0, st>>>(L32, bt->d_slots,
+                                                                        bt->d_state);
       brick_update_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
       brick_p_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
     }

@@ -48,27 +48,17 @@ struct GridDot {
 // partials added by the CTA that arrives last in index order -- and stores
 // alpha = rz / (p.q) for the CG update (breakdown flag when p.q <= 0 or not finite).
 template <class T, int MODE, int MK, bool DOT>
-__global__ void __launch_bounds__(GR_THREADS, sizeof(T) == 4 ? TG_GRID_MINB : 2)
+__global__ void __launch_bounds__(grid_threads<T>(), grid_ctas_per_sm<T>())
     grid_le_kernel(const __grid_constant__ GridCoef<T> P, const T* __restrict__ in,
                    const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                    T* __restrict__ y, const GridDot D) {
-  using V4 = typename Vec4<T>::type;
-  __shared__ V4 sm[2 * GR_PLANE];
+  constexpr int GR_THREADS = grid_threads<T>();
+  __shared__ GridShared<T> sh;
   if constexpr (DOT) {
     if (D.scal[SCAL_DONE] != 0.0) return;  // the CG converged earlier in this block
   }
   GridDotAcc<T> dot;
-  // boundary CTAs first: they start with the first wave and overlap the interior tiles
-  const int b = blockIdx.x;
-  if (b < P.n_boundary_ctas) {
-    grid_boundary<T, MODE, MK, DOT>(P, (int64_t)b * GR_BNODES, in, vin, fixed, y,
-                                      reinterpret_cast<T*>(sm), dot);
-  } else if (b < P.n_boundary_ctas + P.n_xface_ctas) {
-    grid_xface<T, MODE, MK, DOT>(P, b - P.n_boundary_ctas, in, vin, fixed, y, sm, dot);
-  } else {
-    grid_interior<T, MODE, MK, DOT>(P, b - P.n_boundary_ctas - P.n_xface_ctas, in, vin, fixed,
-                                    y, sm, dot);
-  }
+  grid_cta<T, MODE, MK, DOT>(P, blockIdx.x, in, vin, fixed, y, sh, dot);
   if constexpr (DOT) {
     double v[1] = {dot.value()};
     block_reduce_store<1, GR_THREADS>(v, D.part + blockIdx.x);
@@ -103,26 +93,28 @@ static int launch_grid_le_t(const tg_block_plan* plan, int mode, const T* u, con
   const T* in = (mode == TG_MODE_HVP) ? v : u;
   const unsigned grid = (unsigned)n;
   const GridDot D{nullptr, nullptr, nullptr};
+  constexpr int NT = grid_threads<T>();
   if (mode == TG_MODE_HVP) {
     if (fixed)
-      grid_le_kernel<T, TG_MODE_HVP, MASK_DOF, false><<<grid, GR_THREADS, 0, st>>>(P, in, v, fixed,
-                                                                                  y, D);
+      grid_le_kernel<T, TG_MODE_HVP, MASK_DOF, false><<<grid, NT, 0, st>>>(P, in, v, fixed, y, D);
     else
-      grid_le_kernel<T, TG_MODE_HVP, MASK_NONE, false><<<grid, GR_THREADS, 0, st>>>(P, in, v,
-                                                                                   fixed, y, D);
+      grid_le_kernel<T, TG_MODE_HVP, MASK_NONE, false><<<grid, NT, 0, st>>>(P, in, v, fixed, y, D);
   } else if (fixed) {
-    grid_le_kernel<T, TG_MODE_RESIDUAL, MASK_DOF, false><<<grid, GR_THREADS, 0, st>>>(
-        P, in, v, fixed, y, D);
+    grid_le_kernel<T, TG_MODE_RESIDUAL, MASK_DOF, false><<<grid, NT, 0, st>>>(P, in, v, fixed, y,
+                                                                             D);
   } else {
-    grid_le_kernel<T, TG_MODE_RESIDUAL, MASK_NONE, false><<<grid, GR_THREADS, 0, st>>>(
-        P, in, v, fixed, y, D);
+    grid_le_kernel<T, TG_MODE_RESIDUAL, MASK_NONE, false><<<grid, NT, 0, st>>>(P, in, v, fixed, y,
+                                                                              D);
   }
   return launch_check("grid linear-elastic kernel");
 }
 
 int64_t grid_cg_ctas(const tg_block_plan* plan) {
-  GridCoef<float> P;
-  return grid_setup<float>(plan, 1.0, 1.0, P);
+  GridCoef<float> P32;
+  GridCoef<double> P64;
+  const int64_t a = grid_setup<float>(plan, 1.0, 1.0, P32);
+  const int64_t b = grid_setup<double>(plan, 1.0, 1.0, P64);
+  return (a < 0 || b < 0) ? -1 : (a > b ? a : b);
 }
 
 // The grid CG's handling of fixed dofs: x = b there (the identity rows of the masked
@@ -170,11 +162,12 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
     if (n <= 0) return set_error(TG_ERR_VALUE, "grid CG: empty or too large grid");
     const GridDot D{scal, part, ticket};
     const T* in = (const T*)p;
+    constexpr int NT = grid_threads<T>();
     if (node_mask)  // p is zero on the fixed dofs (grid_cg_fixed): only the rows are masked
-      grid_le_kernel<T, TG_MODE_HVP, MASK_NODE_OUT, true><<<(unsigned)n, GR_THREADS, 0, st>>>(
+      grid_le_kernel<T, TG_MODE_HVP, MASK_NODE_OUT, true><<<(unsigned)n, NT, 0, st>>>(
           P, in, in, node_mask, (T*)q, D);
     else
-      grid_le_kernel<T, TG_MODE_HVP, MASK_NONE, true><<<(unsigned)n, GR_THREADS, 0, st>>>(
+      grid_le_kernel<T, TG_MODE_HVP, MASK_NONE, true><<<(unsigned)n, NT, 0, st>>>(
           P, in, in, node_mask, (T*)q, D);
     return launch_check("grid HVP with p.q");
   };
