@@ -128,16 +128,20 @@ __device__ __forceinline__ void reslot(const Launch& L, int& e, int& s, BrickSlo
   count = L.off[e + 1] - L.off[e];
 }
 
-// the slot's stencil into shared memory: the face stencils only for the face CTAs (b: this
-// CTA's index in the brick's launch)
+// the slot's stencil into shared memory: the head, and what CTA b of the brick's launch reads
+// besides
 template <class T>
 __device__ __forceinline__ void copy_coefficients(GridCoef<T>* dst, const GridCoef<T>* src, int b) {
-  constexpr int HEAD = offsetof(GridCoef<T>, fx) / 4, ALL = sizeof(GridCoef<T>) / 4;
+  constexpr int FX = offsetof(GridCoef<T>, fx) / 4, FY = offsetof(GridCoef<T>, fy) / 4,
+                KE = offsetof(GridCoef<T>, ke) / 4, ALL = sizeof(GridCoef<T>) / 4;
   static_assert(offsetof(GridCoef<T>, fx) % 4 == 0 && sizeof(GridCoef<T>) % 4 == 0, "word copy");
   const unsigned* s = reinterpret_cast<const unsigned*>(src);
   unsigned* d = reinterpret_cast<unsigned*>(dst);
-  const int n = grid_is_interior(*src, b) ? HEAD : ALL;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) d[i] = s[i];
+  for (int i = threadIdx.x; i < FX; i += blockDim.x) d[i] = s[i];
+  const GridPart part = grid_part(*src, b);
+  const int lo = part == GRID_XFACE ? FX : (part == GRID_YFACE ? FY : KE);
+  const int hi = part == GRID_INTERIOR ? 0 : (part == GRID_XFACE ? FY : (part == GRID_YFACE ? KE : ALL));
+  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) d[i] = s[i];
 }
 
 __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(grid_threads<T>(), grid_ctas_per_sm<T>())
     grid_le_kernel(const __grid_constant__ GridCoef<T> P, const T* __restrict__ in,
                    const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                    T* __restrict__ y, const GridDot D) {
-  constexpr int GR_THREADS = grid_threads<T>();
+  constexpr int NT = grid_threads<T>();
   __shared__ GridShared<T> sh;
   if constexpr (DOT) {
     if (D.scal[SCAL_DONE] != 0.0) return;  // the CG converged earlier in this block
@@ -61,12 +61,12 @@ __global__ void __launch_bounds__(grid_threads<T>(), grid_ctas_per_sm<T>())
   grid_cta<T, MODE, MK, DOT>(P, blockIdx.x, in, vin, fixed, y, sh, dot);
   if constexpr (DOT) {
     double v[1] = {dot.value()};
-    block_reduce_store<1, GR_THREADS>(v, D.part + blockIdx.x);
+    block_reduce_store<1, NT>(v, D.part + blockIdx.x);
     if (!last_cta(D.ticket)) return;
     double w[1] = {0.0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += GR_THREADS) w[0] += __ldcg(D.part + i);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += NT) w[0] += __ldcg(D.part + i);
     __shared__ double out[1];
-    block_reduce_store<1, GR_THREADS>(w, out);
+    block_reduce_store<1, NT>(w, out);
     if (threadIdx.x == 0) {
       const double pq = out[0];
       D.scal[SCAL_PQ] = pq;
@@ -170,6 +170,343 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
       grid_le_kernel<T, TG_MODE_HVP, MASK_NONE, true><<<(unsigned)n, NT, 0, st>>>(
           P, in, in, node_mask, (T*)q, D);
     return launch_check("grid HVP with p.q");
+  };
+  return prec == TG_F32 ? go(0.f) : go(0.0);
+}
+
+// ------------------------------------------------------------------ persistent CG
+// `iters` Jacobi-CG iterations in one cooperative launch.  Per iteration
+//   A: q = A p (the grid's tiles and faces) with p.q           | grid barrier
+//   B: alpha; r -= alpha q with r.z and r.r                     | grid barrier
+//   C: beta, stopping test; x += alpha p, p = r dinv + beta p   | grid barrier
+// One CTA per SM holds the groups that would be separate CTAs, so that a barrier joins 152
+// arrivals and a dot 152 partials.  Every CTA adds the partials itself, in the same fixed
+// order, so all of them hold the same scalars and take the same decisions, and none waits
+// for one that sums up.  Tiles and vector entries are taken by a fixed stride: the result
+// depends on the number of CTAs alone.
+// Three launches a step spent most of a small or mid-size brick's iteration between kernels
+// and in the arrival counters and last-CTA sums of their dots.  CG in FP32, us an iteration,
+// three launches -> one: 16^3 20.8 -> 12.7, 32^3 20.7 -> 13.9, 64^3 28.4 -> 21.3, 96^3 41.9 ->
+// 37.6.  At 64^3 the tiles take 12,000 clocks, the two vector passes 5,500 each and a barrier
+// 2,500 to 4,500.
+// The barrier's wait ends after GRID_SPIN polls (a second or more); the kernel then reports
+// SCAL_FLAG = 2 and returns.
+constexpr unsigned GRID_SPIN = 1u << 22;
+constexpr int CG_MAX_CTAS = DOT_CHUNKS / 2;  // partials: CTAs of A, then two per CTA of B
+template <class T>
+constexpr int cg_groups() { return grid_ctas_per_sm<T>(); }
+template <class T>
+constexpr int cg_threads() { return cg_groups<T>() * grid_threads<T>(); }
+
+template <class T>
+struct GridCg {
+  T *x, *r, *p, *q;
+  const T* dinv;
+  const uint8_t* nmask;
+  int64_t n;
+  double *scal, *part;
+  unsigned* count;  // zero before the launch
+  int iters, n_items;
+};
+
+// The scalars of the recursion.  FP32 vectors: unevaluated float pairs throughout (two-sums,
+// 48 bits, as the threads' accumulators): an FP64 addition takes about 100 clocks here and an
+// FP64 division in every warp 3,000, several times a whole brick's vector pass.  FP64 vectors:
+// FP64, the divisions in one thread.
+template <class T>
+struct Scalar;
+template <>
+struct Scalar<float> {
+  float hi, lo;
+  __device__ static Scalar of(double v) {
+    const float h = (float)v;
+    return {h, (float)(v - (double)h)};
+  }
+  __device__ double value() const { return (double)hi + (double)lo; }
+  __device__ void add(const Scalar& o) {
+    const float s = hi + o.hi, b = s - hi;
+    lo += o.lo + ((hi - (s - b)) + (o.hi - b));
+    hi = s;
+  }
+  __device__ Scalar down(int o) const {
+    return {__shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o)};
+  }
+  __device__ bool finite() const { return isfinite(hi) && isfinite(lo); }
+  __device__ bool positive() const { return hi + lo > 0.f; }
+  __device__ bool at_most(const Scalar& o) const { return (hi - o.hi) + (lo - o.lo) <= 0.f; }
+  // this / o, rounded to FP32 (the quotient's residual taken into account)
+  __device__ float over(const Scalar& o) const {
+    const float q = hi / o.hi;
+    if (!isfinite(q)) return q;
+    const float r = fmaf(-q, o.hi, hi) + fmaf(-q, o.lo, lo);
+    return q + r / o.hi;
+  }
+};
+template <>
+struct Scalar<double> {
+  double v;
+  __device__ static Scalar of(double a) { return {a}; }
+  __device__ double value() const { return v; }
+  __device__ void add(const Scalar& o) { v += o.v; }
+  __device__ Scalar down(int o) const { return {__shfl_down_sync(0xffffffffu, v, o)}; }
+  __device__ bool finite() const { return isfinite(v); }
+  __device__ bool positive() const { return v > 0.0; }
+  __device__ bool at_most(const Scalar& o) const { return v <= o.v; }
+  __device__ double over(const Scalar& o) const { return v / o.v; }
+};
+__device__ __forceinline__ Scalar<float> scalar_of(const GridDotAcc<float>& a) { return {a.hi, a.lo}; }
+__device__ __forceinline__ Scalar<float> scalar_of(const DotAcc<float>& a) { return {a.hi, a.lo}; }
+__device__ __forceinline__ Scalar<double> scalar_of(const GridDotAcc<double>& a) { return {a.v}; }
+__device__ __forceinline__ Scalar<double> scalar_of(const DotAcc<double>& a) { return {a.v}; }
+
+// sum over the warp's lanes (lane 0)
+template <class T>
+__device__ __forceinline__ Scalar<T> warp_total(Scalar<T> a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a.add(a.down(o));
+  return a;
+}
+
+__device__ __forceinline__ bool grid_arrive_wait(unsigned* count, unsigned target) {
+  __threadfence();
+  atomicAdd(count, 1u);
+  unsigned seen, polls = 0;
+  do {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
+  } while (seen < target && ++polls < GRID_SPIN);
+  __threadfence();
+  return seen >= target;
+}
+
+// The CTA's K sums (v: the thread's) stored as its partials, a grid barrier, and the sums of
+// all CTAs' partials, the same in every thread of every CTA.  False where the wait ran out.
+// den: what v[0]'s total is divided by (quot = total / den) or, with INV, what divides it.
+template <class T, int K, int NT, bool INV>
+__device__ __forceinline__ bool grid_sum(const Scalar<T> (&v)[K], Scalar<T>* part, unsigned* count,
+                                         unsigned target, const Scalar<T>& den, Scalar<T> (&out)[K],
+                                         T& quot) {
+  constexpr int NW = NT / 32;
+  static_assert(NW <= 16, "one warp adds the warps' sums");
+  __shared__ Scalar<T> warps[K][NW], total[K];
+  __shared__ T ratio;
+  __shared__ bool ok;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Scalar<T> a[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) a[k] = warp_total<T>(v[k]);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < K; ++k) warps[k][warp] = a[k];
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      a[k] = lane < NW ? warps[k][lane] : Scalar<T>::of(0.0);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) a[k].add(a[k].down(o));
+      if (lane == 0) part[K * blockIdx.x + k] = a[k];
+    }
+    bool here = true;
+    if (lane == 0) here = grid_arrive_wait(count, target);
+    here = __shfl_sync(0xffffffffu, (int)here, 0) != 0;
+    Scalar<T> w[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) w[k] = Scalar<T>::of(0.0);
+#pragma unroll 8
+    for (int i = lane; i < (int)gridDim.x; i += 32)
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const double raw = __ldcg(reinterpret_cast<const double*>(part) + K * i + k);
+        w[k].add(*reinterpret_cast<const Scalar<T>*>(&raw));
+      }
+#pragma unroll
+    for (int k = 0; k < K; ++k) w[k] = warp_total<T>(w[k]);
+    if (lane == 0) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) total[k] = w[k];
+      ratio = INV ? den.over(w[0]) : w[0].over(den);
+      ok = here;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = total[k];
+  quot = ratio;
+  return ok;
+}
+
+// grid barrier alone
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) ok = grid_arrive_wait(count, target);
+  __syncthreads();
+  return ok;
+}
+
+// four entries of a vector from i on (zero beyond n), and back
+template <class T>
+__device__ __forceinline__ void ld4n(const T* p, int64_t i, int64_t n, T (&v)[4]) {
+  if (i + 3 < n) {
+    ldv(p + i, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k < n ? p[i + k] : T(0);
+  }
+}
+template <class T>
+__device__ __forceinline__ void st4n(T* p, int64_t i, int64_t n, const T (&v)[4]) {
+  if (i + 3 < n) {
+    stv(p + i, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k < n) p[i + k] = v[k];
+  }
+}
+
+template <class T, int MK>
+__global__ void __launch_bounds__(cg_threads<T>(), 1)
+    grid_cg_kernel(const __grid_constant__ GridCoef<T> P, const GridCg<T> G) {
+  constexpr int NT = cg_threads<T>(), NG = cg_groups<T>();
+  extern __shared__ __align__(16) unsigned char cg_smem[];
+  GridShared<T>* sh = reinterpret_cast<GridShared<T>*>(cg_smem);  // one per group
+  using S = Scalar<T>;
+  static_assert(sizeof(S) == sizeof(double), "a partial is one 8-byte slot");
+  const int group = threadIdx.x / grid_threads<T>();
+  S* part_a = reinterpret_cast<S*>(G.part);
+  S* part_b = part_a + CG_MAX_CTAS;
+  unsigned target = 0;
+  S rz = S::of(G.scal[SCAL_RZ]), rr = S::of(G.scal[SCAL_RR]), pq = S::of(0.0), rz_old = rz;
+  const S tol2 = S::of(G.scal[SCAL_TOL2]);
+  T alpha = T(0), beta = T(0);
+  double flag = G.scal[SCAL_FLAG];
+  bool done = G.scal[SCAL_DONE] != 0.0;
+  int it = 0;
+  const int64_t i0 = 4 * ((int64_t)blockIdx.x * NT + threadIdx.x), stride = 4 * (int64_t)gridDim.x * NT;
+  while (it < G.iters && !done && flag == 0.0) {
+    GridDotAcc<T> dot;
+    for (int item = group * gridDim.x + blockIdx.x; item < G.n_items; item += NG * gridDim.x) {
+      grid_cta<T, TG_MODE_HVP, MK, true, EPI_PLAIN, true>(P, item, G.p, G.p, G.nmask, G.q,
+                                                          sh[group], dot);
+      group_sync<T, true>();  // the next item restages the group's shared memory
+    }
+    {
+      const S v[1] = {scalar_of(dot)};
+      S s[1];
+      if (!grid_sum<T, 1, NT, true>(v, part_a, G.count, target += gridDim.x, rz, s, alpha)) {
+        flag = 2.0;
+        break;
+      }
+      pq = s[0];
+    }
+    ++it;
+    if (!pq.positive() || !pq.finite()) {
+      flag = 1.0;
+      alpha = T(0);
+      break;
+    }
+    DotAcc<T> a0, a1;
+#pragma unroll 2
+    for (int64_t i = i0; i < G.n; i += stride) {
+      T rv[4], qv[4], dv[4];
+      ld4n(G.r, i, G.n, rv);
+      ld4n(G.q, i, G.n, qv);
+      ld4n(G.dinv, i, G.n, dv);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        rv[k] = rv[k] - alpha * qv[k];
+        a0.add(rv[k], rv[k] * dv[k]);
+        a1.add(rv[k], rv[k]);
+      }
+      st4n(G.r, i, G.n, rv);
+    }
+    const S v[2] = {scalar_of(a0), scalar_of(a1)};
+    S s[2];
+    if (!grid_sum<T, 2, NT, false>(v, part_b, G.count, target += gridDim.x, rz, s, beta)) {
+      flag = 2.0;
+      break;
+    }
+    rr = s[1];
+    if (!s[0].finite()) {
+      flag = 1.0;
+      beta = T(0);
+    } else {
+      rz_old = rz;
+      rz = s[0];
+    }
+    done = rr.at_most(tol2);
+    const bool stop = done || flag != 0.0;  // the direction stays as it is
+#pragma unroll 2
+    for (int64_t i = i0; i < G.n; i += stride) {
+      T xv[4], pv[4], rv[4], dv[4];
+      ld4n(G.x, i, G.n, xv);
+      ld4n(G.p, i, G.n, pv);
+      ld4n(G.r, i, G.n, rv);
+      ld4n(G.dinv, i, G.n, dv);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        xv[k] += alpha * pv[k];
+        pv[k] = rv[k] * dv[k] + beta * pv[k];
+      }
+      st4n(G.x, i, G.n, xv);
+      if (!stop) st4n(G.p, i, G.n, pv);
+    }
+    if (stop || it == G.iters) break;
+    if (!grid_barrier(G.count, target += gridDim.x)) {
+      flag = 2.0;
+      break;
+    }
+  }
+  if (it > 0 && blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read the scalars
+    const double z1 = rz.value(), z0 = rz_old.value();
+    G.scal[SCAL_PQ] = pq.value();
+    G.scal[SCAL_ALPHA] = (double)alpha;
+    G.scal[SCAL_BETA] = flag == 0.0 ? z1 / z0 : 0.0;
+    G.scal[SCAL_RZ] = z1;
+    G.scal[SCAL_RR] = rr.value();
+    G.scal[SCAL_DONE] = done ? 1.0 : 0.0;
+    G.scal[SCAL_ITERS] += (double)it;
+  }
+  // any CTA whose wait ran out reports it (the others' waits then run out too)
+  if (threadIdx.x == 0 && flag != 0.0) G.scal[SCAL_FLAG] = flag;
+}
+
+bool grid_cg_persistent(const tg_block_plan* plan) {
+  const int64_t n = 3 * (int64_t)plan->grid_nodes[0] * plan->grid_nodes[1] * plan->grid_nodes[2];
+  return n <= GRID_CG_MAX_DOFS;
+}
+
+int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,
+                   const uint8_t* node_mask, void* x, void* r, void* p, void* q, const void* dinv,
+                   double* scal, double* part, unsigned* count, int iters, cudaStream_t st) {
+  auto go = [&](auto t) -> int {
+    using T = decltype(t);
+    constexpr int NT = cg_threads<T>();
+    GridCoef<T> P;
+    const int64_t sms = grid_sm_count();
+    const int64_t items = grid_setup<T>(plan, mu, lam, P, cg_groups<T>() * sms);
+    if (items <= 0) return set_error(TG_ERR_VALUE, "grid CG: empty or too large grid");
+    GridCg<T> G{(T*)x, (T*)r, (T*)p, (T*)q, (const T*)dinv, node_mask,
+                3 * (int64_t)P.nx * P.ny * P.nz, scal, part, count, iters, (int)items};
+    const void* kern = node_mask ? (const void*)grid_cg_kernel<T, MASK_NODE_OUT>
+                                 : (const void*)grid_cg_kernel<T, MASK_NONE>;
+    constexpr int smem = cg_groups<T>() * (int)sizeof(GridShared<T>);
+    TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                      "grid CG: shared memory"));
+    // one CTA per SM (all resident), none without work
+    const int64_t vec = (G.n + 4 * NT - 1) / (4 * NT), want = items > vec ? items : vec;
+    int64_t ctas = sms < want ? sms : want;
+    ctas = ctas < CG_MAX_CTAS ? ctas : CG_MAX_CTAS;
+    TG_TRY(cuda_check(cudaMemsetAsync(count, 0, sizeof(unsigned), st), "grid CG: barrier"));
+    void* args[] = {&P, &G};
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(kern, dim3((unsigned)ctas), dim3(NT), args, smem, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      cudaGetLastError();  // fewer SMs than the device reports: the caller's other path runs
+      return TG_ERR_UNSUPPORTED;
+    }
+    return cuda_check(e, "grid CG: launch");
   };
   return prec == TG_F32 ? go(0.f) : go(0.0);
 }

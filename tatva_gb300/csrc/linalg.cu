@@ -43,24 +43,6 @@ __device__ __forceinline__ void chunk_range(int64_t n, int64_t& i0, int64_t& i1)
   i1 = min(n, i0 + chunk);
 }
 
-// 16-byte vector access of 4 consecutive values (4-aligned index, 16-byte aligned base)
-__device__ __forceinline__ void ldv(const float* p, float (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-}
-__device__ __forceinline__ void ldv(const double* p, double (&v)[4]) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0];
-  const double2 b = reinterpret_cast<const double2*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void stv(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void stv(double* p, const double (&v)[4]) {
-  reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
-  reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
-}
-
 template <class T>
 __global__ void __launch_bounds__(DOT_THREADS)
     dot_partial_kernel(const T* __restrict__ x, const T* __restrict__ y, int64_t n,
@@ -694,6 +676,7 @@ namespace tg {
 struct CgBuffers {
   void *r, *p, *q, *dinv, *apply_ws;
   bool grid;  // structured-brick linear elasticity: the HVP launch also forms p.q
+  bool persistent;  // ... and blocks of iterations run as one launch
   uint8_t* nmask;  // grid: the Dirichlet mask packed to one byte per node (or NULL)
   double *part, *scal;
   unsigned* ticket;  // [2] last-CTA arrival counters of the p.q and update kernels
@@ -718,7 +701,8 @@ struct CgGraphGuard {
 };
 
 // The operator is linear elasticity on a structured brick whose plan carries the grid:
-// the CG's HVP runs as the grid stencil and forms p.q and alpha in the same launch.
+// the CG's HVP runs as the grid stencil and forms p.q and alpha in the same launch, or, up
+// to GRID_CG_MAX_DOFS, a block of iterations runs as one cooperative launch.
 static bool grid_op(const tg_operator_desc* op) {
   return !op->csr_data && op->plan && op->elem == TG_HEX8 && op->mat.kind == TG_LINEAR_ELASTIC &&
          op->mat.elem_param == nullptr && op->plan->grid_nodes[0] > 0 &&
@@ -747,6 +731,7 @@ static CgBuffers cg_carve(const tg_operator_desc* op, void* ws) {
   CgBuffers b;
   const size_t vb = (size_t)n * prec_size(op->prec);
   b.grid = grid_op(op);
+  b.persistent = b.grid && grid_cg_persistent(op->plan);
   b.r = c.take(vb);
   b.p = c.take(vb);
   b.dinv = c.take(vb);
@@ -843,7 +828,16 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
   while (*iters < max_iter) {
     const int k = (max_iter - *iters) < check_every ? (max_iter - *iters) : check_every;
     const int before = *iters;
-    if (can_capture && k == check_every) {
+    if (B.persistent) {
+      rc = launch_grid_cg(op->plan, op->prec, op->mat.p0, op->mat.p1, B.nmask, x, B.r, B.p, B.q,
+                          B.dinv, B.scal, B.part, B.ticket, k, st);
+      if (rc == TG_ERR_UNSUPPORTED) {
+        B.persistent = false;
+        rc = TG_OK;
+        continue;
+      }
+      if (rc != TG_OK) break;
+    } else if (can_capture && k == check_every) {
       if (!exec || graph_len != k) {
         cudaGraph_t graph;
         rc = cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cg: capture");
@@ -869,6 +863,10 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
     rc = read_scalars(B.scal, h, st);
     if (rc != TG_OK) break;
     *iters = (int)h[SCAL_ITERS];  // iterations that ran (a converged block stops early)
+    if (h[SCAL_FLAG] == 2.0) {
+      rc = set_error(TG_ERR_CUDA, "cg: a grid barrier ran out of time after %d iterations", *iters);
+      break;
+    }
     if (h[SCAL_FLAG] != 0.0 || !std::isfinite(h[SCAL_RR])) {
       rc = set_error(TG_ERR_BREAKDOWN, "cg: breakdown (p.Ap <= 0 or non-finite) after %d iterations", *iters);
       break;

@@ -1,6 +1,6 @@
 // CG building blocks shared by the vector kernels (linalg.cu) and the fused grid
 // iteration (grid.cu): device-scalar slots, compensated FP32 dot accumulation, the
-// fixed-order CTA reduction and the last-arriving-CTA pattern.
+// fixed-order CTA reduction, 16-byte access and the last-arriving-CTA pattern.
 #pragma once
 
 #include "tg_common.cuh"
@@ -15,6 +15,24 @@ constexpr int DOT_THREADS = 256;
 // it); SCAL_ITERS: iterations performed.  Slots 5 and 7: true-residual norms.
 constexpr int SCAL_RZ = 0, SCAL_PQ = 1, SCAL_ALPHA = 2, SCAL_BETA = 3, SCAL_RR = 4,
               SCAL_FLAG = 6, SCAL_TOL2 = 8, SCAL_DONE = 9, SCAL_ITERS = 10, SCAL_N = 12;
+
+// 16-byte vector access of 4 consecutive values (4-aligned index, 16-byte aligned base)
+__device__ __forceinline__ void ldv(const float* p, float (&v)[4]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void ldv(const double* p, double (&v)[4]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0];
+  const double2 b = reinterpret_cast<const double2*>(p)[1];
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void stv(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void stv(double* p, const double (&v)[4]) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
+  reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+}
 
 // ------------------------------------------------------------------ dot accumulators
 // FP32 vectors: each thread accumulates x_i y_i as an unevaluated pair (hi, lo) of

@@ -42,8 +42,8 @@
 //     cells around it merged, in constants): y faces a node per thread, consecutive along
 //     x; x faces in 16 x 8 patches (FP64 16 x 16) whose two node columns next to the face
 //     are staged in shared memory first (consecutive nodes are a grid row apart).
-//   * edge CTAs: nodes on two or three faces, one per thread, as the sum over the cells
-//     that exist around the node of the element matrix times the cell's input values.
+//   * edge CTAs: nodes on two or three faces, as the sum over the cells that exist around
+//     the node of the element matrix times the cell's input values.
 // Every output is written once by the thread that owns it, in a fixed order: the
 // result is deterministic and needs no atomics, partial slots or second pass.
 #pragma once
@@ -62,6 +62,10 @@ namespace tg {
 // brick).  FP32: 128 threads, each two node columns four rows apart (grid_interior_pair);
 // FP64: 256 threads, a column each (grid_interior), its kernels being FP64-pipe bound.
 constexpr int GR_DEEP_TZ = 11, GR_MAX_TZ = 15;
+// Unknowns up to which CG iterations run as one cooperative launch (grid_cg_kernel): at 96^3
+// (2.7 M) 37.6 against 41.9 us an iteration in three launches, at 128^3 (6.4 M), where the
+// vector passes want more loads in flight than one CTA per SM keeps, 90.1 against 81.5.
+constexpr int64_t GRID_CG_MAX_DOFS = 3500000;
 constexpr int GR_TX = 32, GR_TY = 8;
 constexpr int GR_PX = GR_TX + 2, GR_PY = GR_TY + 2, GR_PLANE = GR_PX * GR_PY;  // 340
 template <class T>
@@ -111,7 +115,7 @@ struct GridCoef {
   T kxz[2], kyz[2];  // (lambda - mu)/4 M_y, M_x: the z faces' own-plane coupling
   int nx, ny, nz;    // nodes per axis
   int tiles_x, tiles_y, tiles_z, tz;  // tiling of the interior columns: tz planes per tile
-  int n_edge_ctas;       // nodes on two or three faces, one per thread
+  int n_edge_ctas, edge_lanes;  // nodes on two or three faces, edge_lanes lanes each
   int n_yface_ctas;      // y face nodes, one per thread
   int xt_y, xt_z;        // x-face patches per face along y and z
   int n_xface_ctas;      // 2 xt_y xt_z
@@ -188,6 +192,39 @@ struct GridDotAcc<float> {
 // output), or the residual y = b - A x of a right-hand side b (EPI_RESID; with DOT,
 // y.y).
 constexpr int EPI_PLAIN = 0, EPI_RESID = 1;
+
+// A group of grid_threads<T>() threads works on one tile or face.  It is the CTA, or (COH:
+// the persistent CG, whose CTA holds several groups) a part of it with its own barrier.
+template <class T, bool COH>
+__device__ __forceinline__ int group_tid() {
+  return COH ? threadIdx.x & (grid_threads<T>() - 1) : threadIdx.x;
+}
+template <class T, bool COH>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (COH)
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / grid_threads<T>()),
+                 "n"(grid_threads<T>())
+                 : "memory");
+  else
+    __syncthreads();
+}
+
+// Loads of a launch's input vector.  COH: the vector is written between the sweeps of one
+// launch (the persistent CG), so a load must not be moved or served as read-only data; it
+// sees the other CTAs' stores after a grid barrier (whose fence also empties the SM's L1).
+template <bool COH, class T>
+__device__ __forceinline__ T ld_in(const T* p) {
+  if constexpr (!COH) {
+    return __ldg(p);
+  } else {
+    T v;
+    if constexpr (sizeof(T) == 4)
+      asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    else
+      asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+  }
+}
 
 // bit d of the mask of node g (0: free)
 template <int MK>
@@ -275,13 +312,13 @@ __device__ __forceinline__ void stencil_plane(const GridCoef<T>& P,
 
 // Tile of interior columns: thread (lx, ly) owns node column (x0 + lx, y0 + ly), planes
 // [zs, ze) of output (the z faces among them), from the input planes ps .. pe.
-template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN>
+template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN, bool COH = false>
 __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restrict__ in,
                               const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                               T* __restrict__ y, typename Vec4<T>::type* sm, GridDotAcc<T>& dot,
                               const T* __restrict__ bres = nullptr) {
   using V4 = typename Vec4<T>::type;
-  const int tid = threadIdx.x;
+  const int tid = group_tid<T, COH>();
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const int tx = item % P.tiles_x;
   const int rest = item / P.tiles_x;
@@ -320,7 +357,7 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
         const int64_t g = soff[k] + plane_nodes * p;
         if (masks_input<MODE, MK>()) m[k] = mask_bits<MK>(fixed, g);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) r[k][d] = __ldg(in + 3 * g + d);
+        for (int d = 0; d < 3; ++d) r[k][d] = ld_in<COH>(in + 3 * g + d);
       }
     }
   };
@@ -360,7 +397,7 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
     for (int d = 0; d < 3; ++d) {
       T val = acc[d], pv = pc[d];
       if (m >> d & 1) {
-        val = (MODE == TG_MODE_HVP) ? __ldg(vin + base + d) : T(0);
+        val = (MODE == TG_MODE_HVP) ? ld_in<COH>(vin + base + d) : T(0);
         pv = val;
       }
       if constexpr (EPI == EPI_RESID) {
@@ -392,7 +429,7 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
   load_plane(ps + 1, rB, mB);
   load_plane(ps + 2, rA, mA);
   int m_out = out_mask(ps - 1);  // mask of the node emitted after the next plane
-  __syncthreads();
+  group_sync<T, COH>();
   // planes p = ps .. pe, two per trip: buf0 holds p, buf1 gets p + 1
   ctr[0] = ctr[1] = ctr[2] = T(0);
   for (int p = ps; p <= pe; p += 2) {
@@ -404,7 +441,7 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
     shift();
     store_plane(buf1, rB, mB);
     load_plane(p + 3, rB, mB);
-    __syncthreads();
+    group_sync<T, COH>();
     if (p + 1 > pe) break;
 #pragma unroll
     for (int a = 0; a < 3; ++a) pc[a] = ctr[a];
@@ -415,7 +452,7 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
     shift();
     store_plane(buf0, rA, mA);
     load_plane(p + 4, rA, mA);
-    __syncthreads();
+    group_sync<T, COH>();
   }
   if (ze == nz) emit(nz - 1, accM, ctr, m_out);  // the high z face: no plane above it
 }
@@ -561,14 +598,14 @@ struct RawMask {
   }
 };
 
-template <int MODE, int MK, bool DOT>
+template <int MODE, int MK, bool DOT, bool COH = false>
 __device__ void grid_interior_pair(const GridCoef<float>& P, int item,
                                    const float* __restrict__ in, const float* __restrict__ vin,
                                    const uint8_t* __restrict__ fixed, float* __restrict__ y,
                                    GridPairStage* stage, GridDotAcc<float>& dot) {
   constexpr bool MASK_IN = masks_input<MODE, MK>();
   constexpr int NT = grid_threads<float>();
-  const int tid = threadIdx.x;
+  const int tid = group_tid<float, COH>();
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const int tx = item % P.tiles_x;
   const int rest = item / P.tiles_x;
@@ -683,7 +720,7 @@ __device__ void grid_interior_pair(const GridCoef<float>& P, int item,
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         if (m >> d & 1) {
-          val[d] = (MODE == TG_MODE_HVP) ? __ldg(vin + 3 * n + d) : 0.f;
+          val[d] = (MODE == TG_MODE_HVP) ? ld_in<COH>(vin + 3 * n + d) : 0.f;
           pv[d] = val[d];
         }
     }
@@ -710,7 +747,7 @@ __device__ void grid_interior_pair(const GridCoef<float>& P, int item,
   for (int p = ps; p <= pe; ++p) {
     asm volatile("cp.async.wait_group %0;" ::"n"(GP_STAGES - 2) : "memory");
     apply_masks(p, st);
-    __syncthreads();  // plane p complete; every thread is done with the stage refilled below
+    group_sync<float, COH>();  // plane p complete; every thread is done with the stage refilled below
     issue(p + GP_STAGES - 1, (st + GP_STAGES - 1) % GP_STAGES);
     if constexpr (MASK_IN) load_masks(p + 1);
     const GridPairStage& S = stage[st];
@@ -761,7 +798,7 @@ __host__ __device__ inline int edge_nodes(int nx, int ny, int nz) {
 }
 
 // Output of a face node: the Dirichlet rows, the residual epilogue and the dot.
-template <class T, int MODE, int MK, bool DOT, int EPI>
+template <class T, int MODE, int MK, bool DOT, int EPI, bool COH>
 __device__ __forceinline__ void grid_emit_node(int x, int yy, int z, int nx, int ny,
                                                const T (&acc)[3], const T* __restrict__ in,
                                                const T* __restrict__ vin,
@@ -775,9 +812,9 @@ __device__ __forceinline__ void grid_emit_node(int x, int yy, int z, int nx, int
   for (int d = 0; d < 3; ++d) {
     T val = acc[d];
     T pv = T(0);
-    if constexpr (DOT && EPI == EPI_PLAIN) pv = __ldg(in + base + d);
+    if constexpr (DOT && EPI == EPI_PLAIN) pv = ld_in<COH>(in + base + d);
     if (mn >> d & 1) {
-      val = (MODE == TG_MODE_HVP) ? __ldg(vin + base + d) : T(0);
+      val = (MODE == TG_MODE_HVP) ? ld_in<COH>(vin + base + d) : T(0);
       pv = val;
     }
     if constexpr (EPI == EPI_RESID) {
@@ -791,22 +828,26 @@ __device__ __forceinline__ void grid_emit_node(int x, int yy, int z, int nx, int
   if constexpr (DOT) dot.add3(pvs, vals);
 }
 
-// Edge nodes, one per thread: the sum over the cells that exist around the node of the
-// element matrix times the cell's input values.
-template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN>
-__device__ void grid_edges(const GridCoef<T>& P, int t0, const T* __restrict__ in,
+// Edge nodes: the sum over the cells that exist around the node of the element matrix times
+// the cell's input values.  P.edge_lanes lanes per node share its cells (added in a fixed
+// tree): eight where one brick's latency counts (a thread walking the cells one after the
+// other took 8,800 clocks, the longest path of a small brick's HVP), one in launches shared by
+// many bricks, whose CTA count costs more (64 bricks in flight: 333 against 347 ms).
+template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN, bool COH = false>
+__device__ void grid_edges(const GridCoef<T>& P, int b, const T* __restrict__ in,
                            const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                            T* __restrict__ y, T* ke, GridDotAcc<T>& dot,
                            const T* __restrict__ bres = nullptr) {
-  for (int i = threadIdx.x; i < 8 * 8 * 9; i += blockDim.x) ke[i] = (&P.ke[0][0][0][0])[i];
-  __syncthreads();
-  const int nx = P.nx, ny = P.ny, nz = P.nz;
-  const int t = t0 + threadIdx.x;
-  if (t >= edge_nodes(nx, ny, nz)) return;
+  for (int i = group_tid<T, COH>(); i < 8 * 8 * 9; i += grid_threads<T>())
+    ke[i] = (&P.ke[0][0][0][0])[i];
+  group_sync<T, COH>();
+  const int nx = P.nx, ny = P.ny, nz = P.nz, lanes = P.edge_lanes;
+  const int t = (b * grid_threads<T>() + group_tid<T, COH>()) / lanes, n = edge_nodes(nx, ny, nz);
   int x, yy, z;
-  edge_node(t, nx, ny, nz, x, yy, z);
+  edge_node(t < n ? t : n - 1, nx, ny, nz, x, yy, z);
+  const int lane = group_tid<T, COH>() & (lanes - 1);
   T acc[3] = {T(0), T(0), T(0)};
-  for (int o = 0; o < 8; ++o) {  // cell whose corner o is this node
+  for (int o = lane; o < 8; o += lanes) {  // cell whose corner o is this node
     const int cx = x - (o & 1), cy = yy - ((o >> 1) & 1), cz = z - (o >> 2);
     if (cx < 0 || cy < 0 || cz < 0 || cx >= nx - 1 || cy >= ny - 1 || cz >= nz - 1) continue;
     const T* kr = ke + o * 72;  // rows of corner o: [cm][a][b]
@@ -815,27 +856,32 @@ __device__ void grid_edges(const GridCoef<T>& P, int t0, const T* __restrict__ i
       const int64_t g = (cx + (cm & 1)) + (int64_t)nx * ((cy + ((cm >> 1) & 1)) +
                                                          (int64_t)ny * (cz + (cm >> 2)));
       const int m = masks_input<MODE, MK>() ? mask_bits<MK>(fixed, g) : 0;
-      const T v0 = (m & 1) ? T(0) : __ldg(in + 3 * g);
-      const T v1 = (m & 2) ? T(0) : __ldg(in + 3 * g + 1);
-      const T v2 = (m & 4) ? T(0) : __ldg(in + 3 * g + 2);
+      const T v0 = (m & 1) ? T(0) : ld_in<COH>(in + 3 * g);
+      const T v1 = (m & 2) ? T(0) : ld_in<COH>(in + 3 * g + 1);
+      const T v2 = (m & 4) ? T(0) : ld_in<COH>(in + 3 * g + 2);
       const T* k9 = kr + cm * 9;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) acc[a] = fma(k9[3 * a + 2], v2, fma(k9[3 * a + 1], v1, fma(k9[3 * a], v0, acc[a])));
+      for (int a = 0; a < 3; ++a)
+        acc[a] = fma(k9[3 * a + 2], v2, fma(k9[3 * a + 1], v1, fma(k9[3 * a], v0, acc[a])));
     }
   }
-  grid_emit_node<T, MODE, MK, DOT, EPI>(x, yy, z, nx, ny, acc, in, vin, fixed, y, dot, bres);
+  for (int s = lanes >> 1; s > 0; s >>= 1)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) acc[a] += __shfl_down_sync(0xffffffffu, acc[a], s, lanes);
+  if (lane == 0 && t < n)
+    grid_emit_node<T, MODE, MK, DOT, EPI, COH>(x, yy, z, nx, ny, acc, in, vin, fixed, y, dot, bres);
 }
 
 // Nodes of the y faces (1 <= x <= nx - 2, 1 <= z <= nz - 2), one per thread, consecutive
 // threads consecutive along x: the corner loads coalesce.
-template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN>
+template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN, bool COH = false>
 __device__ void grid_yface(const GridCoef<T>& P, int64_t t0, const T* __restrict__ in,
                            const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                            T* __restrict__ y, GridDotAcc<T>& dot,
                            const T* __restrict__ bres = nullptr) {
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const int64_t per = (int64_t)(nx - 2) * (nz - 2);
-  int64_t t = t0 + threadIdx.x;
+  int64_t t = t0 + group_tid<T, COH>();
   if (t >= 2 * per) return;
   const int high = t >= per;
   if (high) t -= per;
@@ -850,9 +896,9 @@ __device__ void grid_yface(const GridCoef<T>& P, int64_t t0, const T* __restrict
       for (int j = 0; j < 9; ++j) {
         const int64_t g = (x + j % 3 - 1) + (int64_t)nx * ((yb + row) + (int64_t)ny * (z + j / 3 - 1));
         const int m = masks_input<MODE, MK>() ? mask_bits<MK>(fixed, g) : 0;
-        const T v0 = (m & 1) ? T(0) : __ldg(in + 3 * g);
-        const T v1 = (m & 2) ? T(0) : __ldg(in + 3 * g + 1);
-        const T v2 = (m & 4) ? T(0) : __ldg(in + 3 * g + 2);
+        const T v0 = (m & 1) ? T(0) : ld_in<COH>(in + 3 * g);
+        const T v1 = (m & 2) ? T(0) : ld_in<COH>(in + 3 * g + 1);
+        const T v2 = (m & 4) ? T(0) : ld_in<COH>(in + 3 * g + 2);
 #pragma unroll
         for (int a = 0; a < 3; ++a)
           acc[a] = fma(P.fy[S][row][j][a][2], v2, fma(P.fy[S][row][j][a][1], v1, fma(P.fy[S][row][j][a][0], v0, acc[a])));
@@ -860,7 +906,7 @@ __device__ void grid_yface(const GridCoef<T>& P, int64_t t0, const T* __restrict
   };
   if (high) stencil(std::integral_constant<int, 1>{});
   else stencil(std::integral_constant<int, 0>{});
-  grid_emit_node<T, MODE, MK, DOT, EPI>(x, high ? ny - 1 : 0, z, nx, ny, acc, in, vin, fixed, y,
+  grid_emit_node<T, MODE, MK, DOT, EPI, COH>(x, high ? ny - 1 : 0, z, nx, ny, acc, in, vin, fixed, y,
                                         dot, bres);
 }
 
@@ -869,7 +915,7 @@ __device__ void grid_yface(const GridCoef<T>& P, int64_t t0, const T* __restrict
 // row apart, so per-thread corner loads would touch one cache line per thread; the CTA
 // instead stages the two node columns next to the face (x = 0, 1 or nx - 2, nx - 1)
 // of its patch and halo, row by row (contiguous 24-byte runs), masked on the way.
-template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN>
+template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN, bool COH = false>
 __device__ void grid_xface(const GridCoef<T>& P, int item, const T* __restrict__ in,
                            const T* __restrict__ vin, const uint8_t* __restrict__ fixed,
                            T* __restrict__ y, typename Vec4<T>::type* sm, GridDotAcc<T>& dot,
@@ -882,21 +928,21 @@ __device__ void grid_xface(const GridCoef<T>& P, int item, const T* __restrict__
   const int xb = face ? nx - 2 : 0;  // first of the two staged columns
   const int y0 = 1 + ty * GR_XT, z0 = 1 + tz * grid_xt_z<T>();
   // slot s = 2 (rz GR_XS + ry) + col: node (xb + col, y0 - 1 + ry, z0 - 1 + rz)
-  for (int s = threadIdx.x; s < 2 * GR_XS * (grid_xt_z<T>() + 2); s += blockDim.x) {
+  for (int s = group_tid<T, COH>(); s < 2 * GR_XS * (grid_xt_z<T>() + 2); s += grid_threads<T>()) {
     const int col = s & 1, r = s >> 1;
     const int gy = y0 - 1 + r % GR_XS, gz = z0 - 1 + r / GR_XS;
     T v0 = T(0), v1 = T(0), v2 = T(0);
     if (gy < ny && gz < nz) {
       const int64_t g = (xb + col) + (int64_t)nx * (gy + (int64_t)ny * gz);
       const int m = masks_input<MODE, MK>() ? mask_bits<MK>(fixed, g) : 0;
-      v0 = (m & 1) ? T(0) : __ldg(in + 3 * g);
-      v1 = (m & 2) ? T(0) : __ldg(in + 3 * g + 1);
-      v2 = (m & 4) ? T(0) : __ldg(in + 3 * g + 2);
+      v0 = (m & 1) ? T(0) : ld_in<COH>(in + 3 * g);
+      v1 = (m & 2) ? T(0) : ld_in<COH>(in + 3 * g + 1);
+      v2 = (m & 4) ? T(0) : ld_in<COH>(in + 3 * g + 2);
     }
     sm[s] = make4<T>(v0, v1, v2);
   }
-  __syncthreads();
-  const int ly = threadIdx.x % GR_XT, lz = threadIdx.x / GR_XT;
+  group_sync<T, COH>();
+  const int ly = group_tid<T, COH>() % GR_XT, lz = group_tid<T, COH>() / GR_XT;
   const int yy = y0 + ly, z = z0 + lz;
   if (yy > ny - 2 || z > nz - 2) return;
   T acc[3] = {T(0), T(0), T(0)};
@@ -914,45 +960,51 @@ __device__ void grid_xface(const GridCoef<T>& P, int item, const T* __restrict__
   };
   if (face) stencil(std::integral_constant<int, 1>{});
   else stencil(std::integral_constant<int, 0>{});
-  grid_emit_node<T, MODE, MK, DOT, EPI>(face ? nx - 1 : 0, yy, z, nx, ny, acc, in, vin, fixed, y,
+  grid_emit_node<T, MODE, MK, DOT, EPI, COH>(face ? nx - 1 : 0, yy, z, nx, ny, acc, in, vin, fixed, y,
                                         dot, bres);
 }
 
+// What CTA b of a brick's launch works on (grid_cta's order): the coefficients it reads are
+// GridCoef's head and, on faces and edges, one of its arrays.
+enum GridPart { GRID_INTERIOR, GRID_XFACE, GRID_YFACE, GRID_EDGE };
 template <class T>
-__device__ __forceinline__ bool grid_is_interior(const GridCoef<T>& P, int b) {
-  return b < P.tiles_x * P.tiles_y * P.tiles_z;
+__device__ __forceinline__ GridPart grid_part(const GridCoef<T>& P, int b) {
+  b -= P.tiles_x * P.tiles_y * P.tiles_z;
+  if (b < 0) return GRID_INTERIOR;
+  if (b < P.n_xface_ctas) return GRID_XFACE;
+  return b - P.n_xface_ctas < P.n_yface_ctas ? GRID_YFACE : GRID_EDGE;
 }
 
-// CTA b of a launch over the brick: edge and face CTAs first (they start with the first wave
-// and overlap the interior tiles)
-template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN>
+// CTA b of a launch over the brick: interior tiles first, then the shorter face and edge CTAs,
+// which fill the launch's tail (faces first measured 24.3 instead of 23.3 us at 128^3)
+template <class T, int MODE, int MK, bool DOT, int EPI = EPI_PLAIN, bool COH = false>
 __device__ __forceinline__ void grid_cta(const GridCoef<T>& P, int b, const T* __restrict__ in,
                                          const T* __restrict__ vin,
                                          const uint8_t* __restrict__ fixed, T* __restrict__ y,
                                          GridShared<T>& sh, GridDotAcc<T>& dot,
                                          const T* __restrict__ bres = nullptr) {
-  if (grid_is_interior(P, b)) {
+  if (grid_part(P, b) == GRID_INTERIOR) {
     if constexpr (std::is_same<T, float>::value) {
       static_assert(EPI == EPI_PLAIN, "the FP32 launches apply the operator only");
-      grid_interior_pair<MODE, MK, DOT>(P, b, in, vin, fixed, y, sh.stage, dot);
+      grid_interior_pair<MODE, MK, DOT, COH>(P, b, in, vin, fixed, y, sh.stage, dot);
     } else {
-      grid_interior<T, MODE, MK, DOT, EPI>(P, b, in, vin, fixed, y, sh.sm, dot, bres);
+      grid_interior<T, MODE, MK, DOT, EPI, COH>(P, b, in, vin, fixed, y, sh.sm, dot, bres);
     }
     return;
   }
   b -= P.tiles_x * P.tiles_y * P.tiles_z;
   if (b < P.n_xface_ctas) {
-    grid_xface<T, MODE, MK, DOT, EPI>(P, b, in, vin, fixed, y, sh.sm, dot, bres);
+    grid_xface<T, MODE, MK, DOT, EPI, COH>(P, b, in, vin, fixed, y, sh.sm, dot, bres);
     return;
   }
   b -= P.n_xface_ctas;
   if (b < P.n_yface_ctas) {
-    grid_yface<T, MODE, MK, DOT, EPI>(P, (int64_t)b * grid_threads<T>(), in, vin, fixed, y, dot,
+    grid_yface<T, MODE, MK, DOT, EPI, COH>(P, (int64_t)b * grid_threads<T>(), in, vin, fixed, y, dot,
                                       bres);
     return;
   }
   b -= P.n_yface_ctas;
-  grid_edges<T, MODE, MK, DOT, EPI>(P, b * grid_threads<T>(), in, vin, fixed, y, sh.ke, dot, bres);
+  grid_edges<T, MODE, MK, DOT, EPI, COH>(P, b, in, vin, fixed, y, sh.ke, dot, bres);
 }
 
 // ------------------------------------------------------------------------- host
@@ -1069,9 +1121,11 @@ static int grid_sm_count() {
 // tiles), or -1 when it does not fit an int.
 // deep: always GR_DEEP_TZ planes per tile (launches shared by many bricks need no spreading
 // of one brick over the SMs, and deeper tiles reload fewer halo planes).
+// groups > 0: the tiles and faces are shared out among that many groups at once (the
+// persistent CG): the fewest planes that leave each at most one, or the rule above.
 template <class T>
 static int64_t grid_setup_dims(const int32_t nodes[3], const double h[3], double mu, double lam,
-                               GridCoef<T>& P, bool deep = false) {
+                               GridCoef<T>& P, bool deep = false, int64_t groups = 0) {
   const int nx = nodes[0], ny = nodes[1], nz = nodes[2];
   grid_coefficients<T>(h, mu, lam, P);
   P.nx = nx;
@@ -1082,6 +1136,15 @@ static int64_t grid_setup_dims(const int32_t nodes[3], const double h[3], double
   P.tiles_y = iy > 0 ? (iy + GR_TY - 1) / GR_TY : 0;
   const int64_t columns = (int64_t)P.tiles_x * P.tiles_y, sms = grid_sm_count();
   auto tiles_of = [&](int64_t tz) { return (nz + tz - 1) / tz; };
+  const int64_t nt = grid_threads<T>();
+  P.edge_lanes = deep ? 1 : 8;
+  const int64_t per_edge = nt / P.edge_lanes;
+  const int64_t n_edge = (edge_nodes(nx, ny, nz) + per_edge - 1) / per_edge;
+  const int64_t n_y = (2 * (int64_t)ix * iz + nt - 1) / nt;
+  P.xt_y = iy > 0 ? (iy + GR_XT - 1) / GR_XT : 0;
+  P.xt_z = iz > 0 ? (iz + grid_xt_z<T>() - 1) / grid_xt_z<T>() : 0;
+  const int64_t n_x = 2 * (int64_t)P.xt_y * P.xt_z;
+  const int64_t faces = n_edge + n_y + n_x;
   // Planes per tile: a tile sweeps its planes one after the other, at a few CTAs per SM
   // mostly waiting on itself, and reloads two halo planes.
   int64_t tz = GR_DEEP_TZ;
@@ -1093,38 +1156,43 @@ static int64_t grid_setup_dims(const int32_t nodes[3], const double h[3], double
       tz = (2 * columns * nz + 5 * sms - 1) / (5 * sms);
       tz = tz < 2 ? 2 : (tz > GR_MAX_TZ ? GR_MAX_TZ : tz);
     } else {
-      // one CTA fills an SM's FP64 pipe: the fewest planes for the SM with the most tiles
-      int64_t best = -1;
-      for (int64_t c = 2; c <= 64; ++c) {
-        const int64_t rounds = (columns * tiles_of(c) + sms - 1) / sms, cost = rounds * (c + 2);
-        if (best < 0 || cost < best) {
+      // Two CTAs share an SM's FP64 pipe: the fewest planes for the busiest SM (with one tile
+      // per SM some still hold two of the launch's CTAs).  HVP at 64^3: 4 planes 86 us, 6
+      // planes 112; 96^3: 13 planes 217 us, 25 planes 339; 128^3: 19 planes 448 us, 13
+      // planes 497.
+      double best = -1.0;
+      for (int64_t c = 2; c <= 24; ++c) {
+        const int64_t r = (columns * tiles_of(c) + sms - 1) / sms;
+        const double cost = (r <= 1 ? 1.6 : (double)r) * (double)(c + 2);
+        if (best < 0.0 || cost < best) {
           best = cost;
           tz = c;
         }
       }
     }
     tz = (nz + tiles_of(tz) - 1) / tiles_of(tz);  // the same tiles, of even depth
+    if (groups > 0)
+      for (int64_t c = 2; c <= GR_MAX_TZ; ++c)
+        if (columns * tiles_of(c) + faces <= groups) {
+          tz = c;
+          break;
+        }
   }
   P.tz = (int)tz;
   P.tiles_z = (int)tiles_of(tz);
   const int64_t n_int = columns * P.tiles_z;
-  const int64_t nt = grid_threads<T>();
-  const int64_t n_edge = (edge_nodes(nx, ny, nz) + nt - 1) / nt;
-  const int64_t n_y = (2 * (int64_t)ix * iz + nt - 1) / nt;
-  P.xt_y = iy > 0 ? (iy + GR_XT - 1) / GR_XT : 0;
-  P.xt_z = iz > 0 ? (iz + grid_xt_z<T>() - 1) / grid_xt_z<T>() : 0;
-  const int64_t n_x = 2 * (int64_t)P.xt_y * P.xt_z;
-  if (n_int + n_edge + n_y + n_x > 0x7fffffff) return -1;
+  if (n_int + faces > 0x7fffffff) return -1;
   P.n_edge_ctas = (int)n_edge;
   P.n_yface_ctas = (int)n_y;
   P.n_xface_ctas = (int)n_x;
-  return n_int + n_edge + n_y + n_x;
+  return n_int + faces;
 }
 
 // The same for a structured-brick plan (tg_grid_detect's nodes and spacings).
 template <class T>
-static int64_t grid_setup(const tg_block_plan* plan, double mu, double lam, GridCoef<T>& P) {
-  return grid_setup_dims<T>(plan->grid_nodes, plan->grid_h, mu, lam, P);
+static int64_t grid_setup(const tg_block_plan* plan, double mu, double lam, GridCoef<T>& P,
+                          int64_t groups = 0) {
+  return grid_setup_dims<T>(plan->grid_nodes, plan->grid_h, mu, lam, P, false, groups);
 }
 
 }  // namespace tg

@@ -30,6 +30,17 @@ int64_t grid_cg_ctas(const tg_block_plan* plan);
 int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double lam,
                         const void* p, const uint8_t* node_mask, void* q, double* scal,
                         double* part, unsigned* ticket, cudaStream_t st);
+// Whether blocks of CG iterations on the plan's grid run as one launch (launch_grid_cg).
+bool grid_cg_persistent(const tg_block_plan* plan);
+// `iters` CG iterations (fewer when they converge or break down) from the residual r, the
+// direction p and the scalars scal (SCAL_*) on a structured brick, as one cooperative
+// launch; part: 2 DOT_CHUNKS doubles, count: one counter.  node_mask: NULL, or one byte per
+// node, bit d set when dof 3 n + d is fixed (pack_node_mask from the C ABI's per-dof mask);
+// p and dinv are zero on fixed dofs (grid_cg_fixed).  TG_ERR_UNSUPPORTED (nothing launched)
+// where the CTAs cannot all be resident.
+int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,
+                   const uint8_t* node_mask, void* x, void* r, void* p, void* q, const void* dinv,
+                   double* scal, double* part, unsigned* count, int iters, cudaStream_t st);
 int pack_node_mask(const uint8_t* fixed, int64_t n_nodes, uint8_t* out, cudaStream_t st);
 // x = b and dinv = 0 on the fixed dofs of a packed node mask (the grid CG)
 int grid_cg_fixed(int prec, int64_t n_nodes, const uint8_t* nmask, const void* b, void* x,
