@@ -286,7 +286,7 @@ typedef struct tg_batch_desc {
   const int64_t* row_ofs;     /* (n_systems + 1) */
   const int64_t* ell_ofs;     /* (n_systems) */
   const int32_t* ell_width;   /* (n_systems) */
-  const int32_t* order;       /* (n_systems) order in which CTAs take systems */
+  const int32_t* order;       /* (n_systems) order in which systems are taken */
   const uint16_t* ell_col;
   const float* ell_val32;
   const double* ell_val64;
@@ -301,8 +301,9 @@ TG_API int tg_batch_ell_from_csr(const tg_batch_desc* desc, int64_t n_rows, cons
 TG_API size_t tg_batch_workspace_bytes(int64_t n_rows);
 /* Solve A_s x_s = b_s for every system (x overwritten, starting from 0): FP32
  * Jacobi-CG inner solves on r64/|r64| to inner_rtol, FP64 refinement on the true
- * residual until |b - A64 x| <= rtol |b|.  One CTA of `threads` (128, 256, 512)
- * threads per system at a time, at most ctas_per_sm CTAs per SM (0: as many as fit).
+ * residual until |b - A64 x| <= rtol |b|.  CTAs of `threads` (128, 256, 512) threads,
+ * one per system at a time (a cluster of four for a large system), at most ctas_per_sm
+ * CTAs per SM (0: as many as fit).
  * Per system (device arrays): total inner iterations, refinements, final relative
  * residual, status (TG_OK, TG_ERR_NOT_CONVERGED, TG_ERR_BREAKDOWN, TG_ERR_VALUE).
  * The result of a system does not depend on the other systems in the batch.    */

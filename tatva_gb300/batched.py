@@ -5,10 +5,10 @@ The reference solves one mesh at a time: a user assembles ``tatva.sparse.jacfwd`
 ``jax.scipy.sparse.linalg.cg`` per mesh.  Here a batch of meshes becomes one
 disconnected mesh, its Hessian is assembled once by the colored compressed-Hessian
 kernels, Dirichlet rows/columns are reduced on the device, and every mesh's diagonal
-block is solved by ``tg_batch_solve``: one CTA per mesh at a time, FP32 CG inner
-solves with FP64 iterative refinement on the true residual, until
-``|b - A x| <= rtol |b|`` per mesh.  The solve can be captured once in a CUDA graph
-(``BatchedSystems.capture``) and replayed.
+block is solved by ``tg_batch_solve``: one CTA per mesh at a time (a cluster of four
+for a large mesh), FP32 CG inner solves with FP64 iterative refinement on the true
+residual, until ``|b - A x| <= rtol |b|`` per mesh.  The solve can be captured once in a
+CUDA graph (``BatchedSystems.capture``) and replayed.
 
 ``poisson_batch`` builds the batched Poisson problem
 ``psi = 1/2 kappa_e |grad u|^2 - f u`` with per-element conductivity (an

@@ -7,28 +7,54 @@
 // column-major (entry k of local row i at k * n_rows + i) with 16-bit local column
 // ids, so that one thread per row reads coalesced.
 //
-// One CTA solves one system at a time, start to finish, and then takes the next one
-// from a device counter (systems ordered largest first).  The search direction p
-// lives in shared memory, so the SpMV gathers hit shared memory; the other vectors
-// stay in global memory (the working set of the systems in flight fits in L2).
+// Systems are taken from device counters (in the caller's order, largest first).  A system
+// whose matrix fits beside the others' in half an SM's shared memory is solved by one CTA,
+// a larger one by a cluster of four, each CTA with a quarter of the rows.  On chip for the
+// whole solve: the FP32 matrix and the window of p that the CTA's rows touch in shared
+// memory, the CG vectors of a thread's rows in its registers.  What does not fit (wide
+// rows, systems of more than 10,000 rows) stays in global memory: the last entries of each
+// row, then the vectors.  After the first dot of an iteration the CTAs of a cluster need
+// only the rows that others' windows hold: z = D^-1 r of those rows travels with the
+// second dot, and every CTA updates its copies of p itself -- two cluster barriers an
+// iteration.
+//
+// Bound: the latency of an iteration (two sums over the CTA or cluster, the SpMV's
+// dependent loads), 2.0 us for 289 rows, 3.2 us for 9,409 rows on a cluster; at full
+// load the shared-memory loads (2.5 per entry).  768 unit squares of 8..96 cells a side:
+// 28.5 -> 5.6 ms; 4,096 of them 59.7 -> 30.7; 4,096 of 6..24: 13.9 -> 1.6.  Before, one CTA
+// streamed a system's matrix from the L2 and DRAM: 27 us an iteration for the largest, which
+// the whole batch waited for, and FP64 sums in every warp, 7 us for the smallest.  Clusters
+// of two: 10 ms, of eight: 14 (768 squares).
+//
 // Each system runs FP32 Jacobi-preconditioned CG on the residual direction
 // r64 / |r64| and FP64 iterative refinement on the true residual b - A64 x, until
-// |b - A64 x| <= rtol |b|.  Dots accumulate as exact-product float pairs per thread
-// and are reduced in FP64 in a fixed order, so each system's result depends only on
-// its own data and the block size -- not on which CTA took it, nor on what else ran.
-// Every loop is bounded by max_outer / max_inner; no CTA waits on another.
+// |b - A64 x| <= rtol |b|.  Dots accumulate as exact-product float pairs (about 48 bits)
+// through the whole sum, in a fixed order, so each system's result depends only on its own
+// data and the block size -- not on which CTA took it, nor on what else ran.  Every loop is
+// bounded by max_outer / max_inner; CTAs wait for others of their cluster only, at cluster
+// barriers that all of it reach (every decision is taken on sums that are the same bits
+// in each).
 #include <cmath>
 #include <map>
 #include <mutex>
 
-#include "tg_common.cuh"
+#include "tg_cg.cuh"
 #include "tg_dispatch.cuh"
 
 namespace tg {
 namespace {
 
-constexpr int BATCH_MAX_ROWS = 49152;  // shared-memory p: 192 KB
-constexpr int RU = 4;                  // rows per thread in flight in the CG passes
+constexpr int BATCH_MAX_ROWS = 49152;  // p of one system in shared memory: 192 KB
+constexpr int TEAM = 4;  // CTAs of a cluster
+// shared memory of a CTA when `per_sm` of them share an SM (228 KB, of which Crew::Shared
+// and 1 KB for the system are the CTA's own)
+constexpr int batch_smem(int nt, int per_sm) { return 228 * 1024 / per_sm - 2048 - 16 * nt; }
+// What one CTA solves alone: its FP32 matrix and p within half an SM's shared memory, its
+// vectors within its registers (10 rows a thread at 256 threads).  768 squares of 8..96: 5.6
+// ms with this limit, 5.9 with 80 KB, 7 with 54 KB (more work at cluster barriers).
+constexpr int64_t SOLO_BYTES = 103 * 1024;
+constexpr int SOLO_ROWS = 2560;
+using Pair = Scalar<float>;
 
 struct BatchArgs {
   tg_batch_desc d;
@@ -39,7 +65,8 @@ struct BatchArgs {
   float* dv;
   float* idiag;
   double* r64;
-  int* counter;
+  unsigned* counter;  // [0] systems of a whole cluster, [1] systems of one CTA
+  int smem_floats;
   double rtol, inner_rtol;
   int max_outer, max_inner;
   int32_t* iters;
@@ -48,70 +75,526 @@ struct BatchArgs {
   int32_t* status;
 };
 
-struct Acc2 {  // float pair with exact products (two-sum + FMA split)
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float a, float b) {
-    const float pr = a * b;
-    const float pe = fmaf(a, b, -pr);
-    const float s = hi + pr;
-    const float bp = s - hi;
-    const float err = (hi - (s - bp)) + (pr - bp);
-    hi = s;
-    lo += err + pe;
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// address of this CTA's shared-memory object in the CTA of rank `cta`
+__device__ __forceinline__ unsigned remote(const void* p, int cta) {
+  const unsigned l = (unsigned)__cvta_generic_to_shared(p);
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(l), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ void put(unsigned addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void put(unsigned addr, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void put(unsigned addr, Pair v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.hi), "f"(v.lo) : "memory");
+}
+__device__ __forceinline__ void put(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ Pair shfl_down(const Pair& v, int o) { return v.down(o); }
+__device__ __forceinline__ double shfl_down(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ Pair lane0(const Pair& v) {
+  return {__shfl_sync(0xffffffffu, v.hi, 0), __shfl_sync(0xffffffffu, v.lo, 0)};
+}
+__device__ __forceinline__ double lane0(double v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void acc(Pair& a, const Pair& b) { a.add(b); }
+__device__ __forceinline__ void acc(double& a, double b) { a += b; }
+
+// The CTAs that solve one system: the whole cluster (size TEAM) or this CTA alone.
+template <int NT>
+struct Crew {
+  static constexpr int NW = NT / 32;
+  struct Shared {
+    Pair part[2][NT];          // the threads' partial sums
+    Pair total[2][2][TEAM];    // the CTAs' sums; two halves, used in turn
+    double dtotal[2][TEAM];
+    double scal[4];
+    int lo[TEAM], hi[TEAM];  // window of every CTA
+    int next;
+  };
+  Shared& S;
+  int size, rank, flip;
+
+  __device__ void sync() const {
+    if (size > 1) cluster_sync(); else __syncthreads();
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ Pair* part(Pair*, int k) const { return S.part[k]; }
+  __device__ double* part(double*, int k) const { return reinterpret_cast<double*>(S.part[k]); }
+  __device__ Pair* total(Pair*, int k) const { return S.total[flip][k]; }
+  __device__ double* total(double*, int) const { return S.dtotal[flip]; }
+
+  // Sum of K per-thread values over the crew in a fixed order; every thread gets it.
+  // Warp k adds value k for the whole CTA: a tree in every warp was more instructions
+  // than the rows of a mid-size system.  A CTA may be one sum ahead of the others (its
+  // total goes to the other half), not two (the sync).
+  // between(): work of the threads after warp K - 1 while those add.
+  template <class V, int K>
+  __device__ __forceinline__ void sum(V (&v)[K]) {
+    sum(v, [] {});
+  }
+  template <class V, int K, class F>
+  __device__ __forceinline__ void sum(V (&v)[K], F&& between) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) part((V*)nullptr, k)[threadIdx.x] = v[k];
+    __syncthreads();
+    if (w < K) {
+      const V* in = part((V*)nullptr, w);
+      V t = in[lane];
+#pragma unroll
+      for (int j = 1; j < NW; ++j) acc(t, in[lane + 32 * j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc(t, shfl_down(t, o));
+      V* out = total((V*)nullptr, w) + rank;
+      if (size > 1) {
+        t = lane0(t);
+        if (lane < TEAM) put(remote(out, lane), t);
+      } else if (lane == 0) {
+        *out = t;
+      }
+    } else {
+      between();
+    }
+    sync();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const V* in = total((V*)nullptr, k);
+      v[k] = in[0];
+      if (size > 1)
+#pragma unroll
+        for (int t = 1; t < TEAM; ++t) acc(v[k], in[t]);
+    }
+    flip ^= 1;
+  }
 };
 
-// Sum of K per-thread values over the block in a fixed order; every thread gets the
-// result.  `buf` alternates between two halves so that one barrier per reduction
-// suffices (a half is rewritten only after the next reduction's barrier).
-template <int NT, int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double* buf, int& flip) {
-  constexpr int NW = NT / 32;
-  double* h = buf + flip * (NW * 4);
-  flip ^= 1;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double t = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    v[k] = t;
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) h[w * 4 + k] = v[k];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double s = 0.0;
-#pragma unroll
-    for (int j = 0; j < NW; ++j) s += h[j * 4 + k];
-    v[k] = s;
+// Systems larger than this go to a whole cluster.  Own size only: which other systems
+// are in the batch changes nothing in a system's arithmetic.
+__device__ __forceinline__ bool for_cluster(const tg_batch_desc& d, int sys) {
+  const int64_t n = d.row_ofs[sys + 1] - d.row_ofs[sys];
+  const int W = d.ell_width[sys];
+  return n > 0 && n <= d.max_rows && W >= 0 && 
+         (n > SOLO_ROWS || n * (6 * (int64_t)W + 4) > SOLO_BYTES);
+}
+
+// The next system (in `order`) of the wanted kind, n_systems when none is left; called
+// by one whole warp.  Claims go through the counter; a warp that claims one of the other
+// kind looks ahead and moves the counter past the stretch it has seen to hold no match.
+__device__ int take(const tg_batch_desc& d, unsigned* counter, bool cluster) {
+  const int lane = threadIdx.x & 31, N = d.n_systems;
+  for (;;) {
+    int k = 0;
+    if (lane == 0) k = (int)min(atomicAdd(counter, 1u), (unsigned)N);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= N || for_cluster(d, d.order[k]) == cluster) return k;
+    int at = k + 1;
+    unsigned hit = 0;
+    for (; at < N; at += 32) {
+      const bool m = at + lane < N && for_cluster(d, d.order[at + lane]) == cluster;
+      hit = __ballot_sync(0xffffffffu, m);
+      if (hit) break;
+    }
+    if (lane == 0) atomicMax(counter, (unsigned)(hit ? at + __ffs(hit) - 1 : N));
   }
 }
 
-template <int NT>
-__device__ void solve_system(const BatchArgs& a, int sys, float* p, double* red, int& flip) {
-  const int tid = threadIdx.x;
-  const int64_t r0 = a.d.row_ofs[sys];
-  const int n = (int)(a.d.row_ofs[sys + 1] - r0);
-  const int W = a.d.ell_width[sys];
-  const int64_t e0 = a.d.ell_ofs[sys];
-  const uint16_t* __restrict__ col = a.d.ell_col + e0;
-  const float* __restrict__ v32 = a.d.ell_val32 + e0;
-  const double* __restrict__ v64 = a.d.ell_val64 + e0;
-  const double* __restrict__ b = a.b + r0;
-  double* __restrict__ x = a.x + r0;
-  float* __restrict__ q = a.q + r0;
-  float* __restrict__ r = a.r + r0;
-  float* __restrict__ dv = a.dv + r0;
-  float* __restrict__ idg = a.idiag + r0;
-  double* __restrict__ r64 = a.r64 + r0;
+// y = A p for the P row pairs (l, l + half), l = tid + j NT, of this thread: entries k < Ks
+// of the rows from shared memory, the others (what did not fit) from global memory.
+template <int NT, int P, int NR>
+__device__ __forceinline__ void spmv(float (&y)[NR], const float* __restrict__ p,
+                                     const float* __restrict__ sval,
+                                     const uint32_t* __restrict__ scol, int m, int half, int Ks,
+                                     int W, int n, int wlo, const float* __restrict__ v32,
+                                     const uint16_t* __restrict__ col) {
+  int l[P], t0 = threadIdx.x;
+  asm volatile("" : "+r"(t0));
+#pragma unroll
+  for (int j = 0; j < P; ++j) {
+    l[j] = min(t0 + j * NT, half - 1);
+    y[2 * j] = y[2 * j + 1] = 0.f;
+  }
+#pragma unroll(P == 1 ? 2 : 1)
+  for (int k = 0; k < Ks; ++k) {
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      const uint32_t c = scol[l[j]];
+      y[2 * j] = fmaf(sval[l[j]], p[c & 0xffffu], y[2 * j]);
+      y[2 * j + 1] = fmaf(sval[l[j] + half], p[c >> 16], y[2 * j + 1]);
+    }
+    sval += m;
+    scol += half;
+  }
+  for (int k = Ks; k < W; ++k) {
+    const int64_t e = (int64_t)k * n;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      const int h = min(l[j] + half, m - 1);
+      y[2 * j] = fmaf(v32[e + l[j]], p[col[e + l[j]] - wlo], y[2 * j]);
+      y[2 * j + 1] = fmaf(v32[e + h], p[col[e + h] - wlo], y[2 * j + 1]);
+    }
+  }
+}
+template <int NT, int P, int NR>
+__device__ __forceinline__ void spmv_pairs(int np, float (&y)[NR], const float* p, const float* sval,
+                                           const uint32_t* scol, int m, int half, int Ks, int W,
+                                           int n, int wlo, const float* v32, const uint16_t* col) {
+  if constexpr (P > 0) {
+    if (np == P) return spmv<NT, P>(y, p, sval, scol, m, half, Ks, W, n, wlo, v32, col);
+    if constexpr (P > 1)
+      return spmv_pairs<NT, P - 1>(np, y, p, sval, scol, m, half, Ks, W, n, wlo, v32, col);
+  }
+}
 
-  if (n < 0 || n > a.d.max_rows || W < 0) {  // inconsistent description: skip the system
+// PP > 0: the CG vectors of this thread's rows live in registers (at most PP row pairs a
+// thread); PP = 0: in shared memory if they fit there, else in the workspace.
+template <int NT, int PP>
+__device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& crew) {
+  const int tid = threadIdx.x;
+  const int n = (int)(a.d.row_ofs[sys + 1] - a.d.row_ofs[sys]);
+  const int W = a.d.ell_width[sys];
+  // this CTA's rows [f0, f0 + m); thread t has rows l and l + half, l = t, t + NT, ...
+  const int chunk = (n + crew.size - 1) / crew.size;
+  const int f0 = min(n, crew.rank * chunk), m = min(n, f0 + chunk) - f0, half = (m + 1) >> 1;
+  const int np = max(0, (half - (tid & ~31) + NT - 1) / NT);  // of this warp
+  // offsets, not pointers, and made opaque where they are used: kept as addresses they
+  // drove the CG vectors out of the registers
+  const int64_t g0 = a.d.row_ofs[sys] + f0, e0 = a.d.ell_ofs[sys] + f0;
+  auto at_row = [&](auto* base) {
+    int64_t o = g0;
+    asm volatile("" : "+l"(o));
+    return base + o;
+  };
+  auto at_entry = [&](auto* base) {
+    int64_t o = e0;
+    asm volatile("" : "+l"(o));
+    return base + o;
+  };
+  // the columns that its rows touch: the window of p kept here
+  int wlo = 0, whi = n - 1;
+  if (crew.size > 1) {
     if (tid == 0) {
+      crew.S.lo[crew.rank] = m ? f0 : n;  // no rows: an empty window above all
+      crew.S.hi[crew.rank] = m ? f0 + m - 1 : n - 1;
+    }
+    __syncthreads();
+    int lo = n, hi = -1;
+    const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
+    for (int i = tid; i < m; i += NT)
+      for (int k = 0; k < W; ++k) {
+        const int c = col[(int64_t)k * n + i];
+        lo = min(lo, c);
+        hi = max(hi, c);
+      }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((tid & 31) == 0 && hi >= 0) {
+      atomicMin(&crew.S.lo[crew.rank], lo);
+      atomicMax(&crew.S.hi[crew.rank], hi);
+    }
+    __syncthreads();
+    wlo = crew.S.lo[crew.rank];
+    whi = crew.S.hi[crew.rank];
+    if (tid < TEAM && tid != crew.rank) {
+      put(remote(&crew.S.lo[crew.rank], tid), wlo);
+      put(remote(&crew.S.hi[crew.rank], tid), whi);
+    }
+  }
+  // shared memory: the window of p, the CG vectors (PP = 0), then as many of the W
+  // entries of every row as fit
+  float* p = smem;
+  float* pown = p + (f0 - wlo);
+  const int nw = whi - wlo + 1;
+  float* hz = p + nw;  // PP > 0: the direction's update z of the window's other rows
+  int at = PP > 0 ? nw + (nw - m) : nw;
+  const bool vs = PP == 0 && at + 4 * m <= a.smem_floats;
+  float* mem[4];  // r, d, 1 / diagonal, q
+  {
+    float* const ws[4] = {at_row(a.r), at_row(a.dv), at_row(a.idiag), at_row(a.q)};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) mem[v] = vs ? smem + at + v * m : ws[v];
+    if (vs) at += 4 * m;
+  }
+  const int Ks = m ? min(W, (a.smem_floats - at) / (m + half)) : 0;
+  float* sval = smem + at;
+  uint32_t* scol = reinterpret_cast<uint32_t*>(sval + Ks * m);
+  // the thread's values (PP > 0); a row that does not exist holds zeros throughout
+  constexpr int NR = PP ? 2 * PP : 4;
+  float vr[NR] = {}, vd[NR] = {}, vg[NR] = {}, vq[NR] = {}, vp[NR] = {};
+  auto R = [&](int j, int i) -> float& { if constexpr (PP > 0) return vr[j]; else return mem[0][i]; };
+  auto D = [&](int j, int i) -> float& { if constexpr (PP > 0) return vd[j]; else return mem[1][i]; };
+  auto G = [&](int j, int i) -> float& { if constexpr (PP > 0) return vg[j]; else return mem[2][i]; };
+  auto Q = [&](int j, int i) -> float& { if constexpr (PP > 0) return vq[j]; else return mem[3][i]; };
+  auto Pv = [&](int j, int i) -> float& { if constexpr (PP > 0) return vp[j]; else return pown[i]; };
+  // f(j, i, exists) for the thread's rows i; with PP > 0 also for its places j without a row
+  auto each = [&](auto&& f) {
+    if constexpr (PP > 0) {
+      int t0 = tid;
+      // indices and conditions made anew in each pass: kept, they drove the vectors out of
+      // the registers
+      asm volatile("" : "+r"(t0));
+#pragma unroll
+      for (int j = 0; j < PP; ++j) {
+        if (j >= np) break;
+        const int l = t0 + j * NT;
+        f(2 * j, l, l < half);
+        f(2 * j + 1, l + half, l + half < m && l < half);
+      }
+    } else {
+#pragma unroll 2
+      for (int i = tid; i < m; i += NT) f(0, i, true);
+    }
+  };
+
+  // set-up: inverse diagonal, x = 0, r64 = b, |b|^2; the matrix
+  double s2[1] = {0.0};
+  bool bad = false;
+  {
+    const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
+    const float* __restrict__ v32 = at_entry(a.d.ell_val32);
+    const double* __restrict__ b = at_row(a.b);
+    double* __restrict__ x = at_row(a.x);
+    double* __restrict__ r64 = at_row(a.r64);
+    for (int l = tid; l < half; l += NT) {
+      const int h = min(l + half, m - 1);
+#pragma unroll 4
+      for (int k = 0; k < Ks; ++k) {
+        const int64_t e = (int64_t)k * n;
+        sval[k * m + l] = v32[e + l];
+        sval[k * m + h] = v32[e + h];
+        scol[k * half + l] = (uint32_t)(col[e + l] - wlo) | ((uint32_t)(col[e + h] - wlo) << 16);
+      }
+    }
+    each([&](int j, int i, bool ok) {
+      float dg = 0.f;
+      if (ok) {
+#pragma unroll 1
+        for (int k = 0; k < W; ++k) {
+          const int64_t e = (int64_t)k * n + i;
+          if (col[e] == f0 + i) dg += v32[e];
+        }
+        bad |= !(dg > 0.f);
+        G(j, i) = 1.f / dg;
+      }
+    });
+    for (int i = tid; i < m; i += NT) {
+      x[i] = 0.0;
+      const double bi = b[i];
+      r64[i] = bi;
+      s2[0] += bi * bi;
+    }
+  }
+  crew.sum(s2);  // also publishes the windows
+  Pair nbad[1] = {{bad ? 1.f : 0.f, 0.f}};
+  crew.sum(nbad);
+  // scal: |b|, |r|, |r| / |b|, 1 / |r|
+  double* const scal = crew.S.scal;
+  if (tid == 0) scal[0] = scal[1] = sqrt(s2[0]);
+  __syncthreads();
+  // What `pown` holds, to the CTAs whose windows have these rows: p into the window, or
+  // z into hz (the window without that CTA's own rows).  By the warps from 2 on, after a
+  // barrier on pown; warp w serves CTA w mod TEAM.
+  constexpr int PW = (Crew<NT>::NW - 2) / TEAM ? (Crew<NT>::NW - 2) / TEAM : 1;
+  auto publish = [&](bool z) {
+    const int w = (tid >> 5) - 2;
+    if (w < 0) return;
+    for (int v = w; v < TEAM * PW; v += Crew<NT>::NW - 2) {
+      const int t = v % TEAM;
+      if (t == crew.rank) continue;
+      const int lo = crew.S.lo[t], hi = crew.S.hi[t];
+      const int skip = z ? hi - lo + 1 - (t < crew.rank ? chunk : 0) : 0;
+      const unsigned dst = remote(p, t) + 4u * (unsigned)(f0 - lo + skip);
+      const int last = min(m - 1, hi - f0);
+      for (int i = max(0, lo - f0) + (v / TEAM) * 32 + (tid & 31); i <= last; i += 32 * PW)
+        put(dst + 4u * (unsigned)i, pown[i]);
+    }
+  };
+  int status = TG_OK, it_total = 0, n_outer = 0;
+  if (nbad[0].hi > 0.f) {
+    status = TG_ERR_BREAKDOWN;  // a non-positive diagonal entry: not SPD
+    if (tid == 0) scal[2] = 1.0;
+  } else if (!(scal[0] > 0.0)) {
+    if (tid == 0) scal[2] = 0.0;
+  } else {
+    for (;;) {
+      if (tid == 0) {
+        scal[2] = scal[1] / scal[0];
+        scal[3] = 1.0 / scal[1];
+      }
+      __syncthreads();
+      if (scal[2] <= a.rtol) break;
+      if (n_outer >= a.max_outer) { status = TG_ERR_NOT_CONVERGED; break; }
+      ++n_outer;
+      // inner FP32 CG on A d = r64 / |r64|
+      const double inv_rn = scal[3];
+      DotAcc<float> rz_acc, rr_acc;
+      const double* __restrict__ r64 = at_row(a.r64);
+      each([&](int j, int i, bool ok) {
+        const float ri = ok ? (float)(r64[i] * inv_rn) : 0.f;
+        const float zi = ok ? ri * G(j, i) : 0.f;
+        R(j, i) = ri;
+        D(j, i) = 0.f;
+        Pv(j, i) = zi;
+        if (PP > 0 && ok) pown[i] = zi;
+        rz_acc.add(ri, zi);
+        rr_acc.add(ri, ri);
+      });
+      if (crew.size > 1) {
+        __syncthreads();
+        publish(false);
+      }
+      Pair t2[2] = {{rz_acc.hi, rz_acc.lo}, {rr_acc.hi, rr_acc.lo}};
+      crew.sum(t2);  // also publishes p
+      Pair rz = t2[0];
+      const Pair stop = Pair::of(a.inner_rtol * a.inner_rtol * t2[1].value());
+      bool broke = false;
+      for (int it = 0; it < a.max_inner; ++it) {
+        DotAcc<float> pq_acc;
+        if constexpr (PP > 0) {
+          spmv_pairs<NT, PP>(np, vq, p, sval, scol, m, half, Ks, W, n, wlo, at_entry(a.d.ell_val32),
+                             at_entry(a.d.ell_col));
+          each([&](int j, int i, bool ok) {
+            if (!ok) vq[j] = 0.f;
+            pq_acc.add(vp[j], vq[j]);
+          });
+        } else {
+          const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
+          const float* __restrict__ v32 = at_entry(a.d.ell_val32);
+          for (int l0 = tid; l0 < half; l0 += 2 * NT) {
+            const int l1 = min(l0 + NT, half - 1);
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
+            const float* v = sval;
+            const uint32_t* c = scol;
+#pragma unroll 4
+            for (int k = 0; k < Ks; ++k) {
+              const uint32_t c0 = c[l0], c1 = c[l1];
+              s[0] = fmaf(v[l0], p[c0 & 0xffffu], s[0]);
+              s[1] = fmaf(v[l0 + half], p[c0 >> 16], s[1]);
+              s[2] = fmaf(v[l1], p[c1 & 0xffffu], s[2]);
+              s[3] = fmaf(v[l1 + half], p[c1 >> 16], s[3]);
+              v += m;
+              c += half;
+            }
+            const int h0 = min(l0 + half, m - 1), h1 = min(l1 + half, m - 1);
+#pragma unroll 2
+            for (int k = Ks; k < W; ++k) {
+              const int64_t e = (int64_t)k * n;
+              s[0] = fmaf(v32[e + l0], p[col[e + l0] - wlo], s[0]);
+              s[1] = fmaf(v32[e + h0], p[col[e + h0] - wlo], s[1]);
+              s[2] = fmaf(v32[e + l1], p[col[e + l1] - wlo], s[2]);
+              s[3] = fmaf(v32[e + h1], p[col[e + h1] - wlo], s[3]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int i = (u < 2 ? l0 : l1) + (u & 1) * half;
+              if (i < m && (u < 2 || l0 + NT < half)) {
+                Q(u, i) = s[u];
+                pq_acc.add(pown[i], s[u]);
+              }
+            }
+          }
+        }
+        Pair t1[1] = {{pq_acc.hi, pq_acc.lo}};
+        crew.sum(t1);
+        ++it_total;
+        if (!t1[0].positive() || !t1[0].finite()) { broke = true; break; }
+        const float alpha = rz.over(t1[0]);
+        DotAcc<float> rz2, rr2;
+        each([&](int j, int i, bool ok) {
+          D(j, i) = fmaf(alpha, Pv(j, i), D(j, i));
+          const float ri = fmaf(-alpha, Q(j, i), R(j, i));
+          R(j, i) = ri;
+          const float zi = ri * G(j, i);
+          if constexpr (PP > 0) vq[j] = zi;  // A p is not needed any more
+          rz2.add(ri, zi);
+          rr2.add(ri, ri);
+          if (PP > 0 && crew.size > 1 && ok) pown[i] = zi;  // p itself is in registers
+        });
+        Pair t3[2] = {{rz2.hi, rz2.lo}, {rr2.hi, rr2.lo}};
+        crew.sum(t3, [&] {
+          if (PP > 0 && crew.size > 1) publish(true);
+        });
+        if (!t3[1].finite()) { broke = true; break; }
+        if (t3[1].at_most(stop)) break;
+        const float beta = t3[0].over(rz);
+        rz = t3[0];
+        each([&](int j, int i, bool ok) {
+          const float pi = fmaf(beta, Pv(j, i), PP > 0 ? Q(j, i) : R(j, i) * G(j, i));
+          Pv(j, i) = pi;
+          if (PP > 0 && ok) pown[i] = pi;
+        });
+        if constexpr (PP > 0) {
+          // the window's other rows: their p is updated here as in their own CTA
+          if (crew.size > 1) {
+            const int below = f0 - wlo;
+            for (int i = tid; i < nw - m; i += NT) {
+              float& pi = p[i < below ? i : i + m];
+              pi = fmaf(beta, pi, hz[i]);
+            }
+          }
+          __syncthreads();
+        } else {
+          __syncthreads();
+          if (crew.size > 1) {
+            publish(false);
+            cluster_sync();
+          }
+        }
+      }
+      if (broke) { status = TG_ERR_BREAKDOWN; break; }
+      // refinement: x += |r64| d, r64 = b - A64 x (FP64)
+      double* x = at_row(a.x);
+      each([&](int j, int i, bool ok) {
+        if (ok) x[i] += scal[1] * (double)D(j, i);
+      });
+      if (crew.size > 1) __threadfence();
+      crew.sync();
+      double u2[1] = {0.0};
+      const double* xs = x - f0;
+      const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
+      const double* __restrict__ v64 = at_entry(a.d.ell_val64);
+      const double* __restrict__ b = at_row(a.b);
+      double* __restrict__ rs = at_row(a.r64);
+      for (int i = tid; i < m; i += NT) {
+        double s = b[i];
+#pragma unroll 4
+        for (int k = 0; k < W; ++k) {
+          const int64_t e = (int64_t)k * n + i;
+          s -= v64[e] * __ldcg(xs + col[e]);
+        }
+        rs[i] = s;
+        u2[0] += s * s;
+      }
+      crew.sum(u2);
+      if (tid == 0) scal[1] = sqrt(u2[0]);
+      __syncthreads();
+      if (!isfinite(scal[1])) { status = TG_ERR_BREAKDOWN; break; }
+    }
+  }
+  if (tid == 0 && crew.rank == 0) {
+    a.iters[sys] = it_total;
+    a.outer[sys] = n_outer;
+    a.rel_res[sys] = scal[2];
+    a.status[sys] = status;
+  }
+  crew.sync();  // shared memory is reused by the next system
+}
+
+template <int NT, int PP, bool ALL>
+__device__ void solve_system(const BatchArgs& a, int sys, float* smem, Crew<NT>& crew) {
+  const int n = (int)(a.d.row_ofs[sys + 1] - a.d.row_ofs[sys]);
+  if (n < 0 || n > a.d.max_rows || a.d.ell_width[sys] < 0) {  // inconsistent: skip the system
+    if (threadIdx.x == 0) {
       a.iters[sys] = 0;
       a.outer[sys] = 0;
       a.rel_res[sys] = 1.0;
@@ -120,164 +603,41 @@ __device__ void solve_system(const BatchArgs& a, int sys, float* p, double* red,
     __syncthreads();
     return;
   }
-  // set-up: inverse diagonal, x = 0, r64 = b, |b|^2
-  double s2[2] = {0.0, 0.0};
-  for (int i = tid; i < n; i += NT) {
-    float dg = 0.f;
-    for (int k = 0; k < W; ++k)
-      if (col[(int64_t)k * n + i] == i) dg += v32[(int64_t)k * n + i];
-    if (!(dg > 0.f)) s2[1] += 1.0;
-    idg[i] = 1.f / dg;
-    x[i] = 0.0;
-    const double bi = b[i];
-    r64[i] = bi;
-    s2[0] += bi * bi;
+  if constexpr (ALL) {
+    if ((n + crew.size - 1) / crew.size > 2 * NT * PP) return solve_rows<NT, 0>(a, sys, smem, crew);
   }
-  block_sum<NT, 2>(s2, red, flip);
-  const double nb = sqrt(s2[0]);
-  int status = TG_OK, it_total = 0, n_outer = 0;
-  double rel = 0.0;
-  if (s2[1] > 0.0) {
-    status = TG_ERR_BREAKDOWN;  // a non-positive diagonal entry: not SPD
-    rel = 1.0;
-  } else if (nb > 0.0) {
-    double rn = nb;
-    for (;;) {
-      rel = rn / nb;
-      if (rel <= a.rtol) break;
-      if (n_outer >= a.max_outer) { status = TG_ERR_NOT_CONVERGED; break; }
-      ++n_outer;
-      // inner FP32 CG on A d = r64 / |r64|
-      const double inv_rn = 1.0 / rn;
-      Acc2 rz_acc, rr_acc;
-      for (int i = tid; i < n; i += NT) {
-        const float ri = (float)(r64[i] * inv_rn);
-        const float zi = ri * idg[i];
-        r[i] = ri;
-        dv[i] = 0.f;
-        p[i] = zi;
-        rz_acc.add(ri, zi);
-        rr_acc.add(ri, ri);
-      }
-      double t2[2] = {rz_acc.value(), rr_acc.value()};
-      block_sum<NT, 2>(t2, red, flip);  // also publishes p
-      double rz = t2[0];
-      const double rr0 = t2[1];
-      const double stop = a.inner_rtol * a.inner_rtol * rr0;
-      bool broke = false;
-      for (int it = 0; it < a.max_inner; ++it) {
-        // rows i0, i0 + NT, ..., i0 + (RU-1) NT together: their loads are independent,
-        // so RU rows' worth of L2 requests are in flight at once.  Accumulation order
-        // (rows in increasing i per thread, entries in increasing k) is unchanged.
-        Acc2 pq_acc;
-        for (int i0 = tid; i0 < n; i0 += RU * NT) {
-          float sv[RU];
-#pragma unroll
-          for (int u = 0; u < RU; ++u) sv[u] = 0.f;
-          for (int k = 0; k < W; ++k) {
-            float av[RU];
-            uint16_t cv[RU];
-#pragma unroll
-            for (int u = 0; u < RU; ++u) {
-              const int i = i0 + u * NT;
-              const int64_t e = (int64_t)k * n + (i < n ? i : 0);
-              av[u] = v32[e];
-              cv[u] = col[e];
-            }
-#pragma unroll
-            for (int u = 0; u < RU; ++u)
-              if (i0 + u * NT < n) sv[u] = fmaf(av[u], p[cv[u]], sv[u]);
-          }
-#pragma unroll
-          for (int u = 0; u < RU; ++u) {
-            const int i = i0 + u * NT;
-            if (i < n) {
-              q[i] = sv[u];
-              pq_acc.add(p[i], sv[u]);
-            }
-          }
-        }
-        double t1[1] = {pq_acc.value()};
-        block_sum<NT, 1>(t1, red, flip);
-        const double pq = t1[0];
-        ++it_total;
-        if (!(pq > 0.0) || !isfinite(pq)) { broke = true; break; }
-        const float alpha = (float)(rz / pq);
-        Acc2 rz2, rr2;
-        for (int i0 = tid; i0 < n; i0 += RU * NT) {
-          float dvv[RU], qv[RU], rv[RU], gv[RU];
-#pragma unroll
-          for (int u = 0; u < RU; ++u) {
-            const int i = i0 + u * NT < n ? i0 + u * NT : i0;
-            dvv[u] = dv[i];
-            qv[u] = q[i];
-            rv[u] = r[i];
-            gv[u] = idg[i];
-          }
-#pragma unroll
-          for (int u = 0; u < RU; ++u) {
-            const int i = i0 + u * NT;
-            if (i < n) {
-              dv[i] = fmaf(alpha, p[i], dvv[u]);
-              const float ri = fmaf(-alpha, qv[u], rv[u]);
-              r[i] = ri;
-              const float zi = ri * gv[u];
-              rz2.add(ri, zi);
-              rr2.add(ri, ri);
-            }
-          }
-        }
-        double t3[2] = {rz2.value(), rr2.value()};
-        block_sum<NT, 2>(t3, red, flip);
-        if (!isfinite(t3[1])) { broke = true; break; }
-        if (t3[1] <= stop) break;
-        const float beta = (float)(t3[0] / rz);
-        rz = t3[0];
-#pragma unroll 4
-        for (int i = tid; i < n; i += NT) p[i] = fmaf(beta, p[i], r[i] * idg[i]);
-        __syncthreads();
-      }
-      if (broke) { status = TG_ERR_BREAKDOWN; break; }
-      // refinement: x += |r64| d, r64 = b - A64 x (FP64)
-      for (int i = tid; i < n; i += NT) x[i] += rn * (double)dv[i];
-      __syncthreads();
-      double u2[1] = {0.0};
-      for (int i = tid; i < n; i += NT) {
-        double s = b[i];
-        for (int k = 0; k < W; ++k) {
-          const int64_t e = (int64_t)k * n + i;
-          s -= v64[e] * x[col[e]];
-        }
-        r64[i] = s;
-        u2[0] += s * s;
-      }
-      block_sum<NT, 1>(u2, red, flip);
-      rn = sqrt(u2[0]);
-      if (!isfinite(rn)) { status = TG_ERR_BREAKDOWN; break; }
-    }
-  }
-  if (tid == 0) {
-    a.iters[sys] = it_total;
-    a.outer[sys] = n_outer;
-    a.rel_res[sys] = rel;
-    a.status[sys] = status;
-  }
-  __syncthreads();  // p, red and the system index are reused by the next system
+  solve_rows<NT, PP>(a, sys, smem, crew);
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT) batch_solve_kernel(BatchArgs a) {
-  extern __shared__ __align__(16) float p[];
-  __shared__ double red[2 * (NT / 32) * 4];
-  __shared__ int s_next;
-  int flip = 0;
+template <int NT, int PP, bool ALL, int PER_SM>
+__global__ void __launch_bounds__(NT, PER_SM) __cluster_dims__(TEAM, 1, 1) batch_solve_kernel(BatchArgs a) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ typename Crew<NT>::Shared S;
+  const int me = (int)cluster_rank();
+  {
+    Crew<NT> crew{S, TEAM, me, 0};
+    for (;;) {
+      if (me == 0 && threadIdx.x < 32) {
+        const int k = take(a.d, a.counter, true);
+        if (threadIdx.x < TEAM) put(remote(&S.next, threadIdx.x), k);
+      }
+      cluster_sync();
+      const int k = S.next;
+      if (k >= a.d.n_systems) break;
+      solve_system<NT, PP, ALL>(a, a.d.order[k], smem, crew);
+    }
+  }
+  __syncthreads();
+  Crew<NT> crew{S, 1, 0, 0};
   for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(a.counter, 1);
+    if (threadIdx.x < 32) {
+      const int k = take(a.d, a.counter + 1, false);
+      if (threadIdx.x == 0) S.next = k;
+    }
     __syncthreads();
-    const int k = s_next;
-    __syncthreads();
+    const int k = S.next;
     if (k >= a.d.n_systems) break;
-    solve_system<NT>(a, a.d.order[k], p, red, flip);
+    solve_system<NT, PP, ALL>(a, a.d.order[k], smem, crew);
   }
 }
 
@@ -400,7 +760,7 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
   a.dv = a.r + n;
   a.idiag = a.dv + n;
   a.r64 = (double*)(w + al(4 * n * sizeof(float)));
-  a.counter = (int*)(w + al(4 * n * sizeof(float)) + al(n * sizeof(double)));
+  a.counter = (unsigned*)(w + al(4 * n * sizeof(float)) + al(n * sizeof(double)));
   a.rtol = rtol;
   a.inner_rtol = inner_rtol;
   a.max_outer = max_outer;
@@ -410,12 +770,15 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
   a.rel_res = rel_res;
   a.status = status;
   cudaStream_t st = as_stream(stream);
-  TG_TRY(cuda_check(cudaMemsetAsync(a.counter, 0, sizeof(int), st), "tg_batch_solve: counter reset"));
-  const size_t smem = (size_t)std::max(desc->max_rows, 1) * sizeof(float);
+  TG_TRY(cuda_check(cudaMemsetAsync(a.counter, 0, 2 * sizeof(unsigned), st), "tg_batch_solve: counter reset"));
   int dev = 0, sms = 0;
   TG_TRY(cuda_check(cudaGetDevice(&dev), "cudaGetDevice"));
   TG_TRY(cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"));
-  auto go = [&](auto kern, int nt) -> int {
+  auto go = [&](auto kern, int nt, int fit) -> int {
+    // p of the largest system has to fit whatever its columns; a larger one takes the SM
+    const size_t smem = std::max((size_t)batch_smem(nt, fit),
+                                 ((size_t)desc->max_rows * sizeof(float) + 15) & ~(size_t)15);
+    a.smem_floats = (int)(smem / sizeof(float));
     {
       // the attribute only grows: graphs captured with larger systems stay launchable
       static std::mutex mu;
@@ -433,14 +796,24 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
                       "tg_batch_solve: occupancy"));
     if (per_sm <= 0) return set_error(TG_ERR_UNSUPPORTED, "tg_batch_solve: kernel does not fit on an SM");
     const int want = ctas_per_sm > 0 ? std::min(ctas_per_sm, per_sm) : per_sm;
-    const int grid = std::max(1, std::min(desc->n_systems, sms * want));
+    const int clusters = std::max(1, std::min(desc->n_systems, sms * want / TEAM));
+    const int grid = clusters * TEAM;
     kern<<<grid, nt, smem, st>>>(a);
     return launch_check("tg_batch_solve");
   };
+  // Many small systems (two or more for every CTA at four to an SM): few registers and
+  // little shared memory, four CTAs of 256 on an SM instead of two.  4,096 squares of 6..24:
+  // 1.6 ms, 2.2 with two to an SM; 700 of 6..31: 0.88 ms, 0.52 with two (the largest systems
+  // then share an SM with fewer others).  The rows of a thread and every sum are the same.
+  const bool many = desc->n_systems >= 8 * sms;
   switch (threads) {
-    case 128: return go(batch_solve_kernel<128>, 128);
-    case 256: return go(batch_solve_kernel<256>, 256);
-    case 512: return go(batch_solve_kernel<512>, 512);
+    case 128:
+      return many && desc->max_rows <= 512 ? go(batch_solve_kernel<128, 2, false, 8>, 128, 8)
+                                           : go(batch_solve_kernel<128, 10, true, 2>, 128, 2);
+    case 256:
+      return many && desc->max_rows <= 1024 ? go(batch_solve_kernel<256, 2, false, 4>, 256, 4)
+                                            : go(batch_solve_kernel<256, 5, true, 2>, 256, 2);
+    case 512: return go(batch_solve_kernel<512, 2, true, 2>, 512, 2);
     default: return set_error(TG_ERR_VALUE, "threads must be 128, 256 or 512");
   }
 }

@@ -213,47 +213,6 @@ struct GridCg {
 // 48 bits, as the threads' accumulators): an FP64 addition takes about 100 clocks here and an
 // FP64 division in every warp 3,000, several times a whole brick's vector pass.  FP64 vectors:
 // FP64, the divisions in one thread.
-template <class T>
-struct Scalar;
-template <>
-struct Scalar<float> {
-  float hi, lo;
-  __device__ static Scalar of(double v) {
-    const float h = (float)v;
-    return {h, (float)(v - (double)h)};
-  }
-  __device__ double value() const { return (double)hi + (double)lo; }
-  __device__ void add(const Scalar& o) {
-    const float s = hi + o.hi, b = s - hi;
-    lo += o.lo + ((hi - (s - b)) + (o.hi - b));
-    hi = s;
-  }
-  __device__ Scalar down(int o) const {
-    return {__shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o)};
-  }
-  __device__ bool finite() const { return isfinite(hi) && isfinite(lo); }
-  __device__ bool positive() const { return hi + lo > 0.f; }
-  __device__ bool at_most(const Scalar& o) const { return (hi - o.hi) + (lo - o.lo) <= 0.f; }
-  // this / o, rounded to FP32 (the quotient's residual taken into account)
-  __device__ float over(const Scalar& o) const {
-    const float q = hi / o.hi;
-    if (!isfinite(q)) return q;
-    const float r = fmaf(-q, o.hi, hi) + fmaf(-q, o.lo, lo);
-    return q + r / o.hi;
-  }
-};
-template <>
-struct Scalar<double> {
-  double v;
-  __device__ static Scalar of(double a) { return {a}; }
-  __device__ double value() const { return v; }
-  __device__ void add(const Scalar& o) { v += o.v; }
-  __device__ Scalar down(int o) const { return {__shfl_down_sync(0xffffffffu, v, o)}; }
-  __device__ bool finite() const { return isfinite(v); }
-  __device__ bool positive() const { return v > 0.0; }
-  __device__ bool at_most(const Scalar& o) const { return v <= o.v; }
-  __device__ double over(const Scalar& o) const { return v / o.v; }
-};
 __device__ __forceinline__ Scalar<float> scalar_of(const GridDotAcc<float>& a) { return {a.hi, a.lo}; }
 __device__ __forceinline__ Scalar<float> scalar_of(const DotAcc<float>& a) { return {a.hi, a.lo}; }
 __device__ __forceinline__ Scalar<double> scalar_of(const GridDotAcc<double>& a) { return {a.v}; }

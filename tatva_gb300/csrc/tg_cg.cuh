@@ -64,6 +64,50 @@ struct DotAcc<double> {
   __device__ __forceinline__ double value() const { return v; }
 };
 
+template <class T>
+struct Scalar;
+template <>
+struct Scalar<float> {
+  float hi, lo;
+  __device__ static Scalar of(double v) {
+    const float h = (float)v;
+    return {h, (float)(v - (double)h)};
+  }
+  __device__ double value() const { return (double)hi + (double)lo; }
+  __device__ void add(const Scalar& o) {
+    const float s = hi + o.hi, b = s - hi;
+    lo += o.lo + ((hi - (s - b)) + (o.hi - b));
+    hi = s;
+  }
+  __device__ Scalar down(int o) const {
+    return {__shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o)};
+  }
+  __device__ bool finite() const { return isfinite(hi) && isfinite(lo); }
+  __device__ bool positive() const { return hi + lo > 0.f; }
+  __device__ bool at_most(const Scalar& o) const { return (hi - o.hi) + (lo - o.lo) <= 0.f; }
+  // this / o, rounded to FP32: an approximate quotient and the quotient of its exact
+  // residual (the division with IEEE rounding costs every warp some hundred clocks)
+  __device__ float over(const Scalar& o) const {
+    if (o.hi < 0x1p-120f || o.hi > 0x1p120f) return (float)(value() / o.value());
+    const float q = __fdividef(hi, o.hi);
+    if (!isfinite(q)) return q;
+    const float r = fmaf(-q, o.hi, hi) + fmaf(-q, o.lo, lo);
+    return q + __fdividef(r, o.hi);
+  }
+};
+template <>
+struct Scalar<double> {
+  double v;
+  __device__ static Scalar of(double a) { return {a}; }
+  __device__ double value() const { return v; }
+  __device__ void add(const Scalar& o) { v += o.v; }
+  __device__ Scalar down(int o) const { return {__shfl_down_sync(0xffffffffu, v, o)}; }
+  __device__ bool finite() const { return isfinite(v); }
+  __device__ bool positive() const { return v > 0.0; }
+  __device__ bool at_most(const Scalar& o) const { return v <= o.v; }
+  __device__ double over(const Scalar& o) const { return v / o.v; }
+};
+
 // ------------------------------------------------------------------ reductions
 // Sum of one value per thread of the CTA into out[k] (thread 0 writes): a fixed tree
 // (shuffles inside each warp, then the warps' sums in warp order), so the result does
