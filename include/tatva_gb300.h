@@ -483,7 +483,7 @@ TG_API int tg_mixed_solve(const tg_operator_desc* op64, const tg_operator_desc* 
 #define TG_BRICK_MAX_SLOTS 64
 /* slot phases */
 #define TG_BRICK_FREE 0
-#define TG_BRICK_REFINE 1 /* FP64 residual / restart pending */
+#define TG_BRICK_REFINE 1 /* FP64 residual pending */
 #define TG_BRICK_RUN 2    /* inner FP32 CG running */
 #define TG_BRICK_DONE 3   /* converged: status TG_OK */
 #define TG_BRICK_FAILED 4 /* status TG_ERR_NOT_CONVERGED or TG_ERR_BREAKDOWN */
@@ -496,7 +496,8 @@ TG_API int tg_mixed_solve(const tg_operator_desc* op64, const tg_operator_desc* 
  * stay owned by the caller and must live until the slot is polled DONE / FAILED;
  * workspace: tg_brick_workspace_bytes(nodes) bytes, 256-byte aligned, likewise.
  * Converges to ||b - A x|| <= rtol ||b||; each inner solve stops at relative
- * residual inner_rtol or max_inner iterations; at most max_outer inner solves.   */
+ * residual inner_rtol or max_inner iterations (the FP64 residual replaces the FP32
+ * one several times on the way); at most max_outer inner solves.                 */
 typedef struct tg_brick_request {
   int32_t nodes[3];
   int32_t reserved;

@@ -11,15 +11,25 @@
 // sizes share one launch and each brick keeps the CTA decomposition it has alone.
 //
 // Per slot, on the device (the CTA that arrives last in a slot's launch decides):
-//   REFINE: x += s d (after an inner solve); r64 = b - A64 x and |r64| in FP64 (the
-//           grid stencil with the residual epilogue); converged (|r64| <= rtol |b|)
-//           -> DONE, refinement budget spent -> FAILED, else restart the inner solve:
-//           r = r64 / |r64| in FP32, d = 0, p = r / diag -> RUN.
-//   RUN:    one Jacobi-CG step in FP32: q = A32 p with p.q and alpha (grid stencil),
-//           d += alpha p, r -= alpha q with r.z, r.r and beta, p = z + beta p; inner
-//           tolerance reached (or the inner budget spent) -> REFINE.
-// A step is the refinement launches followed by `iterations` CG steps, for every
-// slot in use; a slot whose phase does not match a launch leaves it at once.  The
+//   REFINE: x += s d (after a stage); r64 = b - A64 x and |r64| in FP64 (the grid stencil
+//           with the residual epilogue); converged (|r64| <= rtol |b|) -> DONE, refinement
+//           budget spent -> FAILED, else the next stage: r = r64 / |r64| in FP32, d = 0 ->
+//           RUN.  An inner solve (down to inner_rtol; the budget counts these) is made of
+//           stages of equal reduction, and the search direction is kept from one to the
+//           next, made orthogonal to the new residual and scaled to its unit (reliable
+//           updates; a direction that cannot be continued restarts at z).
+//   RUN:    one Jacobi-CG step in FP32: d += alpha p of the step before and p = z + beta p
+//           + gamma r (gamma: the first step of a stage); q = A32 p with p.q and alpha
+//           (grid stencil); r -= alpha q with r.z, r.r and beta; stage tolerance reached
+//           (or the inner budget spent) -> REFINE.
+//
+// Bound: the HVP's instructions (29 us for 2.2 M nodes) and the traffic of the vector passes
+// (40 bytes a dof and step: 13 + 12 us; with d in the update, and an FP64 tree for the dots
+// in every warp, 23 + 9).  Restarting the inner CG at every refinement took 14,438 steps for
+// 24 requests of 16..64 a side, 170 ms with the warm-up; stages 13,134 and 126 ms.
+//
+// A step is `iterations` CG steps with the refinement launches before every 20th, for
+// every slot in use; a slot whose phase does not match a launch leaves it at once.  The
 // host only admits (writes a slot) and polls (reads the per-slot states) between
 // steps.  A slot's arithmetic depends on its own data alone -- fixed CTA
 // decomposition, fixed-order dot reductions, no atomics on values -- so a solve
@@ -36,6 +46,15 @@
 namespace tg {
 namespace {
 
+// A stage reduces |r| by at most STAGE_TOL before the FP64 residual replaces it.  24 requests
+// of 16..64 a side: 0.2 137 ms, 0.1 133, 0.03 130, 0.01 132 (a slot waits for the next
+// refinement launches after each stage; long stages lose the direction).
+constexpr double STAGE_TOL = 0.03;
+// Refinement launches every so many CG steps: 5 140 ms, 10 133, 20 130 (the launches cost
+// as much as two steps even where few slots take part).
+constexpr int REFINE_EVERY = 20;
+// Vector entries a CTA: 8192 135.7 ms, 4096 127.2, 3072 126.3, 2048 129.1.
+constexpr int BRICK_CHUNK = 3072;
 constexpr int BR_MAX = TG_BRICK_MAX_SLOTS;
 constexpr int PH_FREE = TG_BRICK_FREE, PH_REFINE = TG_BRICK_REFINE, PH_RUN = TG_BRICK_RUN,
               PH_DONE = TG_BRICK_DONE, PH_FAILED = TG_BRICK_FAILED;
@@ -53,14 +72,16 @@ struct BrickSlot {
   uint8_t* nmask;  // one byte per node, bit a: dof 3 n + a fixed
   double* part;
   double rtol, inner_rtol;
-  double tol2_inner;  // of the running inner solve (set at each refinement)
   int max_outer, max_inner;
   // written on the device
-  double scal[SCAL_N];
-  double s;   // |r64| of the current refinement: the scale of d
-  double bn;  // |b|
-  unsigned ticket[4];  // arrival counters: HVP, update, residual, restart
-  int inner_iters;
+  double bn;          // |b|
+  double s, s_prev;   // |r64| of the running stage and of the one before: the units of d, r, p
+  double target;      // |r64| at which the running inner solve ends
+  double tol2;        // |r|^2 at which its running stage ends
+  Scalar<float> rz, rz_prev;
+  float alpha, beta, gamma;  // of the last CG step; p = z + beta p + gamma r
+  int stages, last_stage, inner_iters;
+  unsigned ticket[4];  // arrival counters: HVP, update, residual, resume
 };
 
 struct Launch {
@@ -117,6 +138,24 @@ __device__ __forceinline__ void sum_parts(const double* part, int count, double 
   for (int k = 0; k < K; ++k) out[k] = sh[k];
 }
 
+// the same for float pairs
+template <int K, int NT>
+__device__ __forceinline__ void sum_parts(const Scalar<float>* part, int count,
+                                          Scalar<float> (&out)[K]) {
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = {0.f, 0.f};
+  for (int i = threadIdx.x; i < count; i += NT)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float2 t = __ldcg(reinterpret_cast<const float2*>(part + K * i + k));
+      out[k].add({t.x, t.y});
+    }
+  __shared__ Scalar<float> sh[K];
+  block_sum<K, NT>(out, sh);
+#pragma unroll
+  for (int k = 0; k < K; ++k) out[k] = sh[k];
+}
+
 // the entry, slot and CTA index of this CTA in the launch (recomputed from the launch
 // table where keeping them live would cost registers)
 __device__ __forceinline__ void reslot(const Launch& L, int& e, int& s, BrickSlot*& S, int& b,
@@ -142,17 +181,6 @@ __device__ __forceinline__ void copy_coefficients(GridCoef<T>* dst, const GridCo
   const int lo = part == GRID_XFACE ? FX : (part == GRID_YFACE ? FY : KE);
   const int hi = part == GRID_INTERIOR ? 0 : (part == GRID_XFACE ? FY : (part == GRID_YFACE ? KE : ALL));
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) d[i] = s[i];
-}
-
-__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  v[0] = t.x;
-  v[1] = t.y;
-  v[2] = t.z;
-  v[3] = t.w;
-}
-__device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // ------------------------------------------------------------------ admission
@@ -191,20 +219,22 @@ __global__ void __launch_bounds__(256) brick_admit_kernel(const __grid_constant_
 }
 
 // ------------------------------------------------------------------ refinement
-// x += s d after an inner solve
+// x += s d after a stage, d with its last step (alpha p) that no direction pass has added
 __global__ void __launch_bounds__(256) brick_xupdate_kernel(const __grid_constant__ Launch L,
                                                             const BrickSlot* __restrict__ slots,
                                                             const tg_brick_state* __restrict__ st) {
   const int e = find_entry(L, blockIdx.x);
   const int s = L.slot[e];
-  if (st[s].phase != PH_REFINE || st[s].outer == 0) return;
   const BrickSlot* S = slots + s;
+  if (st[s].phase != PH_REFINE || S->stages == 0) return;
   int64_t i0, i1;
   chunk_of(S->n_dofs, blockIdx.x - L.off[e], L.off[e + 1] - L.off[e], i0, i1);
   const double sc = S->s;
+  const float alpha = S->alpha;
   double* x = S->x;
-  const float* d = S->d;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) x[i] += sc * (double)d[i];
+  const float *d = S->d, *p = S->p;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x)
+    x[i] += sc * (double)fmaf(alpha, p[i], d[i]);
 }
 
 // r64 = b - A64 x (FP64 grid stencil, Dirichlet rows identity) and |r64|; the slot's
@@ -234,8 +264,12 @@ __global__ void __launch_bounds__(grid_threads<double>(), 2)
   if (threadIdx.x == 0) {
     const double rn = sqrt(rr[0]);
     tg_brick_state& q = st[s];
-    if (q.outer == 0) S->bn = rn;  // x = 0: the residual is b itself
+    const bool first = S->stages == 0;
+    if (first) S->bn = rn;  // x = 0: the residual is b itself
     const double bn = S->bn;
+    // an inner solve ends with its last stage, with its budget, or when a stage no longer
+    // pays (the residual proper did not even halve)
+    const bool fresh = first || S->last_stage || S->inner_iters >= S->max_inner || rn > 0.5 * S->s;
     q.rel_res = bn > 0.0 ? rn / bn : rn;
     if (!isfinite(rn)) {
       q.phase = PH_FAILED;
@@ -243,24 +277,36 @@ __global__ void __launch_bounds__(grid_threads<double>(), 2)
     } else if (rn <= S->rtol * bn || bn == 0.0) {
       q.phase = PH_DONE;
       q.status = TG_OK;
-    } else if (q.outer >= S->max_outer) {
+    } else if (fresh && q.outer >= S->max_outer) {
       q.phase = PH_FAILED;
       q.status = TG_ERR_NOT_CONVERGED;
     } else {
+      if (fresh) {
+        // the next inner solve reduces |r| only as far as the target still requires
+        // (factor-2 margin), at least by inner_rtol
+        double itol = 0.5 * S->rtol * bn / rn;
+        itol = itol < S->inner_rtol ? S->inner_rtol : (itol > 0.5 ? 0.5 : itol);
+        S->target = itol * rn;
+        S->inner_iters = 0;
+        q.outer += 1;
+      }
+      // the stages that are left, of equal reduction
+      const double left = S->target / rn;
+      const double k = ceil(log(left) / log(STAGE_TOL) - 1e-6);
+      S->last_stage = !(k > 1.0);
+      const double tol = !S->last_stage ? exp(log(left) / k) : (fresh || left < 0.5 ? left : 0.5);
+      S->tol2 = tol * tol;
+      S->s_prev = S->s;
       S->s = rn;
-      // the next inner solve reduces |r| only as far as the target still requires
-      // (factor-2 margin), at least by inner_rtol
-      double itol = 0.5 * S->rtol * bn / rn;
-      itol = itol < S->inner_rtol ? S->inner_rtol : (itol > 0.5 ? 0.5 : itol);
-      S->tol2_inner = itol * itol;
     }
   }
 }
 
-// r = r64 / |r64| (FP32), d = 0, p = z = r dinv, (r.z, r.r); last CTA: scalars, RUN
+// r = r64 / |r64| (FP32), d = 0 and the products that take the direction over; last CTA:
+// its coefficients, RUN
 __global__ void __launch_bounds__(DOT_THREADS)
-    brick_restart_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
-                         tg_brick_state* __restrict__ st) {
+    brick_resume_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
+                        tg_brick_state* __restrict__ st) {
   const int e = find_entry(L, blockIdx.x);
   const int s = L.slot[e];
   if (st[s].phase != PH_REFINE) return;
@@ -268,36 +314,79 @@ __global__ void __launch_bounds__(DOT_THREADS)
   const int b = blockIdx.x - L.off[e], count = L.off[e + 1] - L.off[e];
   int64_t i0, i1;
   chunk_of(S->n_dofs, b, count, i0, i1);
-  const double inv_s = 1.0 / S->s;  // one division per thread, not per element
+  __shared__ double inv_s;
+  if (threadIdx.x == 0) inv_s = 1.0 / S->s;
+  __syncthreads();
+  const bool first = S->stages == 0;
   const double* r64 = S->r64;
   float *r = S->r, *d = S->d, *p = S->p;
   const float* dinv = S->dinv;
-  DotAcc<float> a0, a1;
+  DotAcc<float> az, ar, ap;
   for (int64_t i = i0 + threadIdx.x; i < i1; i += DOT_THREADS) {
     const float ri = (float)(r64[i] * inv_s);
-    const float zi = ri * dinv[i];
     r[i] = ri;
     d[i] = 0.0f;
-    p[i] = zi;
-    a0.add(ri, zi);
-    a1.add(ri, ri);
+    if (first) p[i] = 0.0f;
+    else ap.add(p[i], ri);
+    az.add(ri, ri * dinv[i]);
+    ar.add(ri, ri);
   }
-  double v[2] = {a0.value(), a1.value()};
-  block_reduce_store<2, DOT_THREADS>(v, S->part + 2 * b);
+  Scalar<float> v[3] = {{az.hi, az.lo}, {ar.hi, ar.lo}, {ap.hi, ap.lo}};
+  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  block_sum<3, DOT_THREADS>(v, part + 3 * b);
   if (!last_of(&S->ticket[3], count)) return;
-  double w[2];
-  sum_parts<2, DOT_THREADS>(S->part, count, w);
+  sum_parts<3, DOT_THREADS>(part, count, v);
   if (threadIdx.x == 0) {
-    S->scal[SCAL_RZ] = w[0];
-    S->scal[SCAL_RR] = w[1];
-    S->scal[SCAL_FLAG] = 0.0;
-    S->inner_iters = 0;
-    st[s].outer += 1;
+    const double rz = v[0].value(), rr = v[1].value(), pr = v[2].value();
+    const double rz_k = first ? 0.0 : S->rz_prev.value(), scale = first ? 0.0 : S->s_prev / S->s;
+    const bool ok = rz_k > 0.0 && isfinite(rz_k) && rr > 0.0 && rz > 0.0 && isfinite(pr) &&
+                    isfinite(rz) && scale > 0.0 && isfinite(scale);
+    const double beta = ok ? rz / (rz_k * scale * scale) : 0.0;
+    S->beta = (float)(beta * scale);
+    S->gamma = ok ? (float)(-beta * scale * pr / rr) : 0.0f;
+    S->alpha = 0.0f;
+    S->rz = v[0];
+    S->stages += 1;
     st[s].phase = PH_RUN;
   }
 }
 
 // ------------------------------------------------------------------ one CG step
+// d += alpha p of the step before; p = r dinv + beta p + gamma r
+__global__ void __launch_bounds__(DOT_THREADS) brick_p_kernel(const __grid_constant__ Launch L,
+                                                              const BrickSlot* __restrict__ slots,
+                                                              const tg_brick_state* __restrict__ st) {
+  const int e = find_entry(L, blockIdx.x);
+  const int s = L.slot[e];
+  if (st[s].phase != PH_RUN) return;
+  const BrickSlot* S = slots + s;
+  int64_t i0, i1;
+  chunk_of(S->n_dofs, blockIdx.x - L.off[e], L.off[e + 1] - L.off[e], i0, i1);
+  const int64_t iv = i0 + ((i1 - i0) & ~int64_t(3));
+  const float alpha = S->alpha, beta = S->beta, gamma = S->gamma;
+  const float *r = S->r, *dinv = S->dinv;
+  float *p = S->p, *d = S->d;
+#pragma unroll 2
+  for (int64_t i = i0 + 4 * threadIdx.x; i < iv; i += 4 * DOT_THREADS) {
+    float rr[4], di[4], pp[4], dd[4];
+    ldv(r + i, rr);
+    ldv(dinv + i, di);
+    ldv(p + i, pp);
+    ldv(d + i, dd);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      dd[k] = fmaf(alpha, pp[k], dd[k]);
+      pp[k] = fmaf(beta, pp[k], fmaf(gamma, rr[k], rr[k] * di[k]));
+    }
+    stv(d + i, dd);
+    stv(p + i, pp);
+  }
+  for (int64_t i = iv + threadIdx.x; i < i1; i += DOT_THREADS) {
+    d[i] = fmaf(alpha, p[i], d[i]);
+    p[i] = fmaf(beta, p[i], fmaf(gamma, r[i], r[i] * dinv[i]));
+  }
+}
+
 // q = A32 p (grid stencil, Dirichlet rows identity) with p.q; last CTA: alpha
 __global__ void __launch_bounds__(grid_threads<float>(), grid_ctas_per_sm<float>())
     brick_hvp_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
@@ -314,27 +403,25 @@ __global__ void __launch_bounds__(grid_threads<float>(), grid_ctas_per_sm<float>
   __syncthreads();
   GridDotAcc<float> dot;
   grid_cta<float, TG_MODE_HVP, MASK_NODE_OUT, true>(P, b, S->p, S->p, S->nmask, S->q, sh, dot);
-  double v[1] = {dot.value()};
+  Scalar<float> v[1] = {{dot.hi, dot.lo}};
   reslot(L, e, s, S, b, count, slots);  // recomputed: not held in registers across the sweep
-  block_reduce_store<1, GR_THREADS>(v, S->part + b);
+  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  block_sum<1, GR_THREADS>(v, part + b);
   if (!last_of(&S->ticket[0], count)) return;
-  double w[1];
-  sum_parts<1, GR_THREADS>(S->part, count, w);
+  sum_parts<1, GR_THREADS>(part, count, v);
   if (threadIdx.x == 0) {
-    const double pq = w[0];
-    S->scal[SCAL_PQ] = pq;
-    if (!(pq > 0.0) || !isfinite(pq)) {
-      S->scal[SCAL_ALPHA] = 0.0;
+    if (!v[0].positive() || !v[0].finite()) {
+      S->alpha = 0.0f;
       st[s].phase = PH_FAILED;
       st[s].status = TG_ERR_BREAKDOWN;
     } else {
-      S->scal[SCAL_ALPHA] = S->scal[SCAL_RZ] / pq;
+      S->alpha = S->rz.over(v[0]);
     }
   }
 }
 
-// d += alpha p; r -= alpha q; (r.z, r.r) with z = r dinv; last CTA: beta, rz, and the
-// inner stopping test (|r| <= inner tolerance or the inner budget spent -> REFINE)
+// r -= alpha q; (r.z, r.r) with z = r dinv; last CTA: beta, rz, and the stage's stopping test
+// (|r| <= its tolerance or the inner budget spent -> REFINE)
 __global__ void __launch_bounds__(DOT_THREADS)
     brick_update_kernel(const __grid_constant__ Launch L, BrickSlot* __restrict__ slots,
                         tg_brick_state* __restrict__ st) {
@@ -346,88 +433,55 @@ __global__ void __launch_bounds__(DOT_THREADS)
   int64_t i0, i1;
   chunk_of(S->n_dofs, b, count, i0, i1);
   const int64_t iv = i0 + ((i1 - i0) & ~int64_t(3));
-  const float alpha = (float)S->scal[SCAL_ALPHA];
-  float *d = S->d, *r = S->r;
-  const float *p = S->p, *q = S->q, *dinv = S->dinv;
+  const float alpha = S->alpha;
+  float* r = S->r;
+  const float *q = S->q, *dinv = S->dinv;
   DotAcc<float> a0, a1;
 #pragma unroll 2
   for (int64_t i = i0 + 4 * threadIdx.x; i < iv; i += 4 * DOT_THREADS) {
-    float dd[4], pp[4], rr[4], qq[4], di[4];
-    ld4(d + i, dd);
-    ld4(p + i, pp);
-    ld4(r + i, rr);
-    ld4(q + i, qq);
-    ld4(dinv + i, di);
+    float rr[4], qq[4], di[4];
+    ldv(r + i, rr);
+    ldv(q + i, qq);
+    ldv(dinv + i, di);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      dd[k] += alpha * pp[k];
-      rr[k] = rr[k] - alpha * qq[k];
-    }
+    for (int k = 0; k < 4; ++k) rr[k] = fmaf(-alpha, qq[k], rr[k]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) a0.add(rr[k], rr[k] * di[k]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) a1.add(rr[k], rr[k]);
-    st4(d + i, dd);
-    st4(r + i, rr);
+    stv(r + i, rr);
   }
   for (int64_t i = iv + threadIdx.x; i < i1; i += DOT_THREADS) {
-    d[i] += alpha * p[i];
-    const float ri = r[i] - alpha * q[i];
+    const float ri = fmaf(-alpha, q[i], r[i]);
     r[i] = ri;
     a0.add(ri, ri * dinv[i]);
     a1.add(ri, ri);
   }
-  double v[2] = {a0.value(), a1.value()};
-  block_reduce_store<2, DOT_THREADS>(v, S->part + 2 * b);
+  Scalar<float> v[2] = {{a0.hi, a0.lo}, {a1.hi, a1.lo}};
+  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  block_sum<2, DOT_THREADS>(v, part + 2 * b);
   if (!last_of(&S->ticket[1], count)) return;
-  double w[2];
-  sum_parts<2, DOT_THREADS>(S->part, count, w);
+  sum_parts<2, DOT_THREADS>(part, count, v);
   if (threadIdx.x == 0) {
-    const double rz_new = w[0], rr = w[1];
     tg_brick_state& o = st[s];
     o.iterations += 1;
     S->inner_iters += 1;
-    S->scal[SCAL_RR] = rr;
-    if (!isfinite(rz_new) || !isfinite(rr)) {
+    if (!v[0].finite() || !v[1].finite()) {
       o.phase = PH_FAILED;
       o.status = TG_ERR_BREAKDOWN;
     } else {
-      S->scal[SCAL_BETA] = rz_new / S->scal[SCAL_RZ];
-      S->scal[SCAL_RZ] = rz_new;
-      if (rr <= S->tol2_inner || S->inner_iters >= S->max_inner) o.phase = PH_REFINE;
+      S->beta = v[0].over(S->rz);
+      S->gamma = 0.0f;
+      S->rz_prev = S->rz;
+      S->rz = v[0];
+      if (v[1].value() <= S->tol2 || S->inner_iters >= S->max_inner) o.phase = PH_REFINE;
     }
   }
 }
 
-// p = r dinv + beta p
-__global__ void __launch_bounds__(DOT_THREADS) brick_p_kernel(const __grid_constant__ Launch L,
-                                                              const BrickSlot* __restrict__ slots,
-                                                              const tg_brick_state* __restrict__ st) {
-  const int e = find_entry(L, blockIdx.x);
-  const int s = L.slot[e];
-  if (st[s].phase != PH_RUN) return;
-  const BrickSlot* S = slots + s;
-  int64_t i0, i1;
-  chunk_of(S->n_dofs, blockIdx.x - L.off[e], L.off[e + 1] - L.off[e], i0, i1);
-  const int64_t iv = i0 + ((i1 - i0) & ~int64_t(3));
-  const float beta = (float)S->scal[SCAL_BETA];
-  const float *r = S->r, *dinv = S->dinv;
-  float* p = S->p;
-  for (int64_t i = i0 + 4 * threadIdx.x; i < iv; i += 4 * DOT_THREADS) {
-    float rr[4], di[4], pp[4];
-    ld4(r + i, rr);
-    ld4(dinv + i, di);
-    ld4(p + i, pp);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) pp[k] = rr[k] * di[k] + beta * pp[k];
-    st4(p + i, pp);
-  }
-  for (int64_t i = iv + threadIdx.x; i < i1; i += DOT_THREADS) p[i] = r[i] * dinv[i] + beta * p[i];
-}
-
 // ------------------------------------------------------------------ host
 int brick_chunks(int64_t n_dofs) {
-  const int64_t c = (n_dofs + 8191) / 8192;
+  const int64_t c = (n_dofs + BRICK_CHUNK - 1) / BRICK_CHUNK;
   return (int)(c < 1 ? 1 : (c > DOT_CHUNKS ? DOT_CHUNKS : c));
 }
 
@@ -441,7 +495,7 @@ int64_t brick_grid_ctas(const int32_t nodes[3]) {
 size_t brick_part_doubles(const int32_t nodes[3]) {
   const int64_t n = 3 * (int64_t)nodes[0] * nodes[1] * nodes[2];
   const int64_t g32 = brick_grid_ctas<float>(nodes), g64 = brick_grid_ctas<double>(nodes);
-  const int64_t g = g32 > g64 ? g32 : g64, c = 2 * (int64_t)brick_chunks(n);
+  const int64_t g = g32 > g64 ? g32 : g64, c = 3 * (int64_t)brick_chunks(n);
   return (size_t)(g > c ? g : c);
 }
 
@@ -573,7 +627,6 @@ extern "C" int tg_brick_admit(tg_brick_batch* bt, const tg_brick_request* req, v
   h.part = (double*)take(brick_part_doubles(nd) * sizeof(double));
   h.rtol = req->rtol;
   h.inner_rtol = req->inner_rtol;
-  h.tol2_inner = req->inner_rtol * req->inner_rtol;
   h.max_outer = req->max_outer;
   h.max_inner = req->max_inner;
   tg_brick_state q;
@@ -634,15 +687,19 @@ extern "C" int tg_brick_step(tg_brick_batch* bt, int iterations, void* stream) {
     TG_TRY(launch_check("tg_brick_step: admission"));
   }
   auto enqueue = [&]() {
-    brick_xupdate_kernel<<<(unsigned)nc, 256, 0, st>>>(Lc, bt->d_slots, bt->d_state);
-    brick_resid_kernel<<<(unsigned)n64, grid_threads<double>(), 0, st>>>(L64, bt->d_slots,
-                                                                         bt->d_state);
-    brick_restart_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
+    auto refine = [&] {
+      brick_xupdate_kernel<<<(unsigned)nc, 256, 0, st>>>(Lc, bt->d_slots, bt->d_state);
+      brick_resid_kernel<<<(unsigned)n64, grid_threads<double>(), 0, st>>>(L64, bt->d_slots,
+                                                                           bt->d_state);
+      brick_resume_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
+    };
+    if (iterations == 0) refine();
     for (int it = 0; it < iterations; ++it) {
+      if (it % REFINE_EVERY == 0) refine();
+      brick_p_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
       brick_hvp_kernel<<<(unsigned)n32, grid_threads<float>(), 0, st>>>(L32, bt->d_slots,
                                                                         bt->d_state);
       brick_update_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
-      brick_p_kernel<<<(unsigned)nc, DOT_THREADS, 0, st>>>(Lc, bt->d_slots, bt->d_state);
     }
   };
   const bool can_capture = st != nullptr && st != cudaStreamLegacy && st != cudaStreamPerThread;

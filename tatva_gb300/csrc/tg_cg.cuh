@@ -136,6 +136,26 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[K], double* __res
   __syncthreads();
 }
 
+// The same for float pairs: warp k adds value k of all threads (a tree of pairs in every
+// warp would be several times the instructions).  Ends with a barrier.
+template <int K, int NT = DOT_THREADS>
+__device__ __forceinline__ void block_sum(Scalar<float> (&v)[K], Scalar<float>* __restrict__ out) {
+  __shared__ Scalar<float> part[K][NT];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) part[k][threadIdx.x] = v[k];
+  __syncthreads();
+  if (w < K) {
+    Scalar<float> t = part[w][lane];
+#pragma unroll
+    for (int j = 1; j < NT / 32; ++j) t.add(part[w][lane + 32 * j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t.add(t.down(o));
+    if (lane == 0) out[w] = t;
+  }
+  __syncthreads();
+}
+
 // Called by every thread after thread 0 stored this CTA's partials: true in the CTA
 // that arrives last, which then sees every CTA's partials (read them with __ldcg).
 // That CTA resets the ticket for the next launch.  An arrival counter, no waiting.
