@@ -44,27 +44,35 @@ __device__ __forceinline__ void add_tangent_block(T (&rb)[V][COLS], int b, T s, 
     }
 }
 
+// coordinates and, where the law needs them, displacements of an element's nodes
+template <int ET, int MAT, class T>
+struct ElementNodes {
+  static constexpr bool NH = MAT == TG_NEO_HOOKEAN;
+  T X[Elem<ET>::NN][Elem<ET>::D], U[Elem<ET>::NN][NH ? 3 : 1];
+  __device__ __forceinline__ void load(const T* __restrict__ coords, const T* __restrict__ u,
+                                       const int (&nid)[Elem<ET>::NN]) {
+    constexpr int D = Elem<ET>::D;
+#pragma unroll
+    for (int b = 0; b < Elem<ET>::NN; ++b)
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        X[b][d] = coords[(int64_t)nid[b] * D + d];
+        if constexpr (NH) U[b][d] = u[(int64_t)nid[b] * 3 + d];
+      }
+  }
+};
+
 // Row block K_e[(a, i), (b, k)] (i, k < V, b < NN) of element e's tangent at u,
-// rb[i][b V + k]; nid: the element's nodes
+// rb[i][b V + k]
 template <int ET, int MAT, class T>
 __device__ __forceinline__ void element_row_block(
-    const T* __restrict__ coords, const int32_t* __restrict__ conn, const T* __restrict__ u,
-    T p0, T p1, const T* __restrict__ eparam, int64_t e, int a,
-    T (&rb)[LawDims<MAT, Elem<ET>::D>::V][Elem<ET>::NN * LawDims<MAT, Elem<ET>::D>::V],
-    int (&nid)[Elem<ET>::NN]) {
+    ElementNodes<ET, MAT, T>& nodes, T p0, T p1, const T* __restrict__ eparam, int64_t e,
+    int a, T (&rb)[LawDims<MAT, Elem<ET>::D>::V][Elem<ET>::NN * LawDims<MAT, Elem<ET>::D>::V]) {
   using E = Elem<ET>;
   constexpr int NN = E::NN, D = E::D, V = LawDims<MAT, D>::V;
   constexpr bool NH = MAT == TG_NEO_HOOKEAN;
-  T X[NN][D], U[NN][NH ? 3 : 1];
-#pragma unroll
-  for (int b = 0; b < NN; ++b) nid[b] = __ldg(conn + e * NN + b);
-#pragma unroll
-  for (int b = 0; b < NN; ++b)
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      X[b][d] = coords[(int64_t)nid[b] * D + d];
-      if constexpr (NH) U[b][d] = u[(int64_t)nid[b] * 3 + d];
-    }
+  auto& X = nodes.X;  // (overwritten)
+  auto& U = nodes.U;
   const T mu = eparam ? eparam[e] : p0, lam = MAT == TG_POISSON ? T(0) : p1;
 #pragma unroll
   for (int i = 0; i < V; ++i)
@@ -229,7 +237,7 @@ __device__ __forceinline__ void element_row_block(
 // What bounds it is on chip: about 250 arithmetic instructions and 36 shared-memory adds
 // per (Tet4 element, corner) and the gathers of the element's nodes; the data is written
 // once and neither column indices nor colours are read.  Kuhn 56^3 jittered, Neo-Hookean
-// FP32 (1.05 M tets, 24 M values): 201 us; compressed Hessian and decompression, which it
+// FP32 (1.05 M tets, 24 M values): 187 us, 201 without the loads run ahead; compressed Hessian and decompression, which it
 // replaces on the mesh's own pattern, 717 + 125 us.
 template <int ET>
 constexpr int slot_pad() { return Elem<ET>::NN <= 4 ? 4 : 8; }
@@ -239,7 +247,7 @@ constexpr int CSR_SLAB = 16;   // row words a lane hands over at a time when wri
 template <int ET, int MAT, class T>
 __global__ void __launch_bounds__(32 * CSR_WARPS)
     hessian_csr_kernel(const T* __restrict__ coords, const int32_t* __restrict__ conn,
-                       const T* __restrict__ u, T p0, T p1, const T* __restrict__ eparam,
+                       bool conn16, const T* __restrict__ u, T p0, T p1, const T* __restrict__ eparam,
                        int64_t n_nodes, const int32_t* __restrict__ inc_ptr,
                        const int32_t* __restrict__ inc_idx, const uint16_t* __restrict__ slots,
                        const int32_t* __restrict__ indptr, int row_words, T* __restrict__ data) {
@@ -254,28 +262,74 @@ __global__ void __launch_bounds__(32 * CSR_WARPS)
   const int len = live ? __ldg(indptr + V * n + V) - base : 0;
   const int L = len / V;  // the length of each of the node's rows
   for (int k = 0; k < len; ++k) acc[k * 32 + lane] = T(0);
-  const int j1 = live ? __ldg(inc_ptr + n + 1) : 0;
-  for (int j = live ? __ldg(inc_ptr + n) : 0; j < j1; ++j) {
-    const int ea = __ldg(inc_idx + j);
-    const int64_t e = ea / NN;
-    const int a = ea - (int)(e * NN);
-    int sl[NP];
-    load_lconn<NP>(slots + (int64_t)j * NP, sl);
-    T rb[V][NN * V];
-    int nid[NN];
-    element_row_block<ET, MAT, T>(coords, conn, u, p0, p1, eparam, e, a, rb, nid);
+  const int j0 = live ? __ldg(inc_ptr + n) : 0, last = (live ? __ldg(inc_ptr + n + 1) : 0) - 1;
+  // The loads of an incidence entry depend on one another (entry, node ids and slots,
+  // coordinates), so they run ahead: the entry by two turns, ids and slots by one and, for
+  // simplices, the coordinates from before the adds of the turn before.  At 11 warps an SM
+  // (shared memory) their latency was a third of the time.  Scalar laws (a ninth of the adds
+  // and of the shared memory, hence more warps) lose by it: Poisson 81.7 -> 84.8 us.
+  constexpr bool AHEAD = V > 1, NODES_AHEAD = AHEAD && E::SIMPLEX;
+  auto ids = [&](int ea, int (&nid)[NN]) {
+    const int32_t* row = conn + (int64_t)(ea / NN) * NN;
+    if (NN % 4 == 0 && conn16) {
 #pragma unroll
-    for (int b = 0; b < NN; ++b) {
-      T* w = acc + (V * sl[b]) * 32 + lane;
-      T t[V][V];
+      for (int b = 0; b < NN / 4; ++b) {
+        const int4 c = __ldg(reinterpret_cast<const int4*>(row) + b);
+        nid[4 * b] = c.x;
+        nid[4 * b + 1] = c.y;
+        nid[4 * b + 2] = c.z;
+        nid[4 * b + 3] = c.w;
+      }
+    } else {
 #pragma unroll
-      for (int i = 0; i < V; ++i)
+      for (int b = 0; b < NN; ++b) nid[b] = __ldg(row + b);
+    }
+  };
+  if (j0 <= last) {
+    int ea = 0, ea1 = 0, nid[NN];
+    LconnRaw<NP> raw;
+    ElementNodes<ET, MAT, T> nodes;
+    if constexpr (AHEAD) {
+      ea = __ldg(inc_idx + j0);
+      ea1 = __ldg(inc_idx + min(j0 + 1, last));
+      ids(ea, nid);
+      raw.load(slots + (int64_t)j0 * NP);
+    }
+    if constexpr (NODES_AHEAD) nodes.load(coords, u, nid);
+    for (int j = j0; j <= last; ++j) {
+      if constexpr (!AHEAD) {
+        ea = __ldg(inc_idx + j);
+        raw.load(slots + (int64_t)j * NP);
+        ids(ea, nid);
+      }
+      if constexpr (!NODES_AHEAD) nodes.load(coords, u, nid);
+      int sl[NP], ea2 = 0;
+      raw.unpack(sl);
+      if constexpr (AHEAD) {
+        ea2 = __ldg(inc_idx + min(j + 2, last));
+        ids(ea1, nid);
+        raw.load(slots + (int64_t)min(j + 1, last) * NP);
+      }
+      T rb[V][NN * V];
+      element_row_block<ET, MAT, T>(nodes, p0, p1, eparam, ea / NN, ea % NN, rb);
+      if constexpr (NODES_AHEAD) nodes.load(coords, u, nid);
 #pragma unroll
-        for (int k = 0; k < V; ++k) t[i][k] = w[(i * L + k) * 32];
+      for (int b = 0; b < NN; ++b) {
+        T* w = acc + (V * sl[b]) * 32 + lane;
+        T t[V][V];
 #pragma unroll
-      for (int i = 0; i < V; ++i)
+        for (int i = 0; i < V; ++i)
 #pragma unroll
-        for (int k = 0; k < V; ++k) w[(i * L + k) * 32] = t[i][k] + rb[i][b * V + k];
+          for (int k = 0; k < V; ++k) t[i][k] = w[(i * L + k) * 32];
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+#pragma unroll
+          for (int k = 0; k < V; ++k) w[(i * L + k) * 32] = t[i][k] + rb[i][b * V + k];
+      }
+      if constexpr (AHEAD) {
+        ea = ea1;
+        ea1 = ea2;
+      }
     }
   }
   // write-out in slabs of CSR_SLAB words per node: each lane moves its slab from its own
@@ -411,7 +465,11 @@ __global__ void compressed_hessian_kernel(const T* __restrict__ coords,
       const int a = ea - (int)(e * NN);
       T rb[V][NN * V];
       int nid[NN];
-      element_row_block<ET, MAT, T>(coords, conn, u, p0, p1, eparam, e, a, rb, nid);
+#pragma unroll
+      for (int b = 0; b < NN; ++b) nid[b] = __ldg(conn + e * NN + b);
+      ElementNodes<ET, MAT, T> nodes;
+      nodes.load(coords, u, nid);
+      element_row_block<ET, MAT, T>(nodes, p0, p1, eparam, e, a, rb);
 #pragma unroll
       for (int b = 0; b < NN; ++b)
 #pragma unroll
@@ -668,9 +726,9 @@ extern "C" int tg_hessian_csr(int elem, int prec, const tg_material* mat, const 
                                                  (int)smem),
                             "tg_hessian_csr: shared memory"));
           kern<<<grid_for(n_nodes, 32 * CSR_WARPS), 32 * CSR_WARPS, smem, st>>>(
-              (const T*)coords, conn, (const T*)u, (T)mat->p0, (T)mat->p1,
-              (const T*)mat->elem_param, n_nodes, inc_ptr, inc_idx, slots, indptr, words,
-              (T*)data);
+              (const T*)coords, conn, reinterpret_cast<uintptr_t>(conn) % 16 == 0, (const T*)u,
+              (T)mat->p0, (T)mat->p1, (const T*)mat->elem_param, n_nodes, inc_ptr, inc_idx, slots,
+              indptr, words, (T*)data);
           return launch_check("tg_hessian_csr");
         });
       }
