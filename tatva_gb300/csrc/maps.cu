@@ -209,7 +209,8 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
 // thread and 4-byte accesses: eval 125 -> 20 us (82 MB written, 5.2 TB/s with the gathers),
 // grad 329 -> 65 us (248 MB, 4.2 TB/s), transpose of grad 156 -> 77 us for the elements, of
 // eval 236 -> 21 us for the elements + 38 us for the nodes.  61 x 67 x 59 distorted, FP64,
-// V = 1: grad 389 -> 263 us, its transpose 408 -> 282 us.
+// V = 1: grad 389 -> 263 us, its transpose 408 -> 282 us; with the adjugate instead of the
+// inverse (one value: three products by the reciprocal determinant, not nine) 240 and 246.
 template <int NV>
 constexpr int hex_group() { return NV ? NV : 3; }
 template <class T>
@@ -282,10 +283,16 @@ struct HexPlane {
 
 // the geometry of an element: scaled coordinate modes and, for a parallelepiped (bitwise
 // what the per-point evaluation gives), its one inverse
-template <class T>
+template <class T, bool UNSCALED>
 struct HexGeometry {
-  T mx[8][3], R[3][3];
+  T mx[8][3], R[3][3], r;
   bool constant;
+  // R: the inverse, or, UNSCALED, the adjugate, and r: the reciprocal determinant
+  __device__ __forceinline__ void invert(const T (&J)[3][3]) {
+    if constexpr (UNSCALED) r = T(1) / adjugate3(J, R);
+    else inv3(J, R);
+  }
+  __device__ __forceinline__ T scaled(T v) const { return UNSCALED ? v * r : v; }
   __device__ __forceinline__ void load(const T* __restrict__ coords,
                                        const int32_t* __restrict__ conn, int64_t e,
                                        int (&nid)[8]) {
@@ -297,7 +304,7 @@ struct HexGeometry {
       const T J[3][3] = {{mx[1][0], mx[1][1], mx[1][2]},
                          {mx[2][0], mx[2][1], mx[2][2]},
                          {mx[4][0], mx[4][1], mx[4][2]}};
-      inv3(J, R);
+      invert(J);
     }
   }
   __device__ __forceinline__ void plane(HexPlane<T, 3>& jx, T sz) const {
@@ -307,7 +314,7 @@ struct HexGeometry {
     if (!constant) {
       T J[3][3];
       jx.at(p, J);
-      inv3(J, R);
+      invert(J);
     }
   }
 };
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(128) hex_grad_kernel(const T* __restrict__ nod
   constexpr int G = hex_group<NV>(), NP = hex_planes<T>();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_elems) return;
-  HexGeometry<T> geo;
+  HexGeometry<T, NV == 1> geo;
   int nid[8];
   geo.load(coords, conn, e, nid);
   if (NV) V = NV;
@@ -361,7 +368,8 @@ __global__ void __launch_bounds__(128) hex_grad_kernel(const T* __restrict__ nod
 #pragma unroll
             for (int d = 0; d < 3; ++d)
               o[((z * 4 + p) * G + k) * 3 + d] =
-                  fma(geo.R[d][2], H[2][k], fma(geo.R[d][1], H[1][k], geo.R[d][0] * H[0][k]));
+                  geo.scaled(fma(geo.R[d][2], H[2][k],
+                                 fma(geo.R[d][1], H[1][k], geo.R[d][0] * H[0][k])));
         }
       }
       T* dst = out + ((e * 8 + z0 * 4) * V + v0) * 3;
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(128)
   constexpr int G = hex_group<NV>(), NP = hex_planes<T>();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n_elems) return;
-  HexGeometry<T> geo;
+  HexGeometry<T, NV == 1> geo;
   int nid[8];
   geo.load(coords, conn, e, nid);
   if (NV) V = NV;
@@ -426,7 +434,8 @@ __global__ void __launch_bounds__(128)
             T r[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i)
-              r[i] = fma(geo.R[2][i], t[2], fma(geo.R[1][i], t[1], geo.R[0][i] * t[0]));
+              r[i] = geo.scaled(
+                  fma(geo.R[2][i], t[2], fma(geo.R[1][i], t[1], geo.R[0][i] * t[0])));
             F.add(p, k, r[0], r[1], r[2]);
           }
         }
@@ -722,30 +731,37 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
 }
 
 // Phase 2: out[n] = the contributions of node n's incident (element, corner) pairs, in
-// the order of the incidence CSR (increasing element): deterministic.  Four pairs' loads
-// in flight (each waits for its index).
+// the order of the incidence CSR (increasing element): deterministic.  Each pair's load
+// waits for its index, so eight pairs are in flight (a Hex8 grid node has eight; FP32, 3
+// values, 881,000 nodes: 37.5 us with four, 31.7 with eight), four in FP64 (1 value, 253,000
+// nodes: 8.6 us, 10.2 with eight).
 template <class T>
 __global__ void transpose_node_kernel(const T* __restrict__ contrib, int64_t n_nodes, int V,
                                       const int32_t* __restrict__ inc_ptr,
                                       const int32_t* __restrict__ inc_idx, T* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_nodes * V) return;
-  const int64_t n = i / V;
+  const int64_t n = i < (int64_t)1 << 31 ? (int64_t)((unsigned)i / (unsigned)V) : i / V;
   const int v = (int)(i - n * V);
   T s = T(0);
   int k = __ldg(inc_ptr + n);
   const int k1 = __ldg(inc_ptr + n + 1);
-  for (; k + 4 <= k1; k += 4) {
-    int j[4];
-    T c[4];
+  auto run = [&](auto count) {
+    constexpr int C = decltype(count)::value;
+    for (; k + C <= k1; k += C) {
+      int j[C];
+      T c[C];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) j[t] = __ldg(inc_idx + k + t);
+      for (int t = 0; t < C; ++t) j[t] = __ldg(inc_idx + k + t);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) c[t] = __ldg(contrib + (int64_t)j[t] * V + v);
+      for (int t = 0; t < C; ++t) c[t] = __ldg(contrib + (int64_t)j[t] * V + v);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) s += c[t];
-  }
-  for (; k < k1; ++k) s += __ldg(contrib + (int64_t)__ldg(inc_idx + k) * V + v);
+      for (int t = 0; t < C; ++t) s += c[t];
+    }
+  };
+  if constexpr (sizeof(T) == 4) run(std::integral_constant<int, 8>{});
+  run(std::integral_constant<int, 4>{});
+  run(std::integral_constant<int, 1>{});
   out[i] = s;
 }
 

@@ -116,6 +116,20 @@ __device__ __forceinline__ T inv2(const T (&J)[2][2], T (&Ji)[2][2]) {
   return det;
 }
 
+// adjugate of J (its inverse times the determinant); returns the determinant
+template <class T>
+__device__ __forceinline__ T adjugate3(const T (&J)[3][3], T (&A)[3][3]) {
+  A[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+  A[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+  A[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+  A[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
+  A[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
+  A[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
+  A[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+  A[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
+  A[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+  return J[0][0] * A[0][0] + J[0][1] * A[1][0] + J[0][2] * A[2][0];
+}
 // inverse and determinant of J; r: the reciprocal of the determinant
 template <class T>
 __device__ __forceinline__ T inv3(const T (&J)[3][3], T (&Ji)[3][3], T& r) {
