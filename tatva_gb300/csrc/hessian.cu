@@ -1,4 +1,5 @@
-// Colored compressed Hessian (K6) and its decompression into CSR values.
+// Colored compressed Hessian (K6) and its decompression into CSR values, and the CSR
+// values straight from the element tangents (hessian_csr_kernel) on a mesh's own pattern.
 //
 // Reference (tatva/sparse/base.py):
 //   colored_jacobian_batch (:230-270): Jc[:, c] = jvp(grad E, u, seed_c),

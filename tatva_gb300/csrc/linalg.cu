@@ -7,7 +7,8 @@
 //     order, independent of the GPU and of the launch, so repeated solves are bitwise
 //     identical
 //   * Jacobi-preconditioned CG whose scalars never leave the device; `check_every`
-//     iterations are captured once in a CUDA graph and replayed between host
+//     iterations are captured once in a CUDA graph (on a structured brick of up to
+//     GRID_CG_MAX_DOFS unknowns: run as one cooperative launch) and replayed between host
 //     convergence checks; every loop is bounded by max_iter
 //   * mixed precision: FP32 CG inner solves (FP32 HVP, FP64 dots), FP64 iterative
 //     refinement on the true residual b - A64 x.
