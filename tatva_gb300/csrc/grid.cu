@@ -185,13 +185,16 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
 // for one that sums up.  Tiles and vector entries are taken by a fixed stride: the result
 // depends on the number of CTAs alone.
 // Three launches a step spent most of a small or mid-size brick's iteration between kernels
-// and in the arrival counters and last-CTA sums of their dots.  CG in FP32, us an iteration,
-// three launches -> one: 16^3 20.8 -> 12.7, 32^3 20.7 -> 13.9, 64^3 28.4 -> 21.3, 96^3 41.9 ->
-// 37.6.  At 64^3 the tiles take 12,000 clocks, the two vector passes 5,500 each and a barrier
-// 2,500 to 4,500.
+// and in the arrival counters and last-CTA sums of their dots.  The vectors that only their
+// own thread touches (r, 1 / diag, x, and its p) stay in shared memory as far as they fit.
+// CG in FP32, us an iteration, three launches -> one for 50 iterations -> vectors kept and one
+// for up to 800: 16^3 20.8 -> 12.8 -> 12.2, 32^3 20.7 -> 14.4 -> 13.9, 64^3 28.4 -> 21.3 -> 19.7,
+// 96^3 41.9 -> 38.6 -> 37.0.  At 64^3 the tiles take 11,500 clocks, the update 4,200, the
+// direction 2,000 and an exchange about 7,000 (fences and loads across the dies).
 // The barrier's wait ends after GRID_SPIN polls (a second or more); the kernel then reports
 // SCAL_FLAG = 2 and returns.
 constexpr unsigned GRID_SPIN = 1u << 22;
+constexpr int CG_SMEM = 220 * 1024;  // of the 227 KB a CTA can have; the rest: the sums'
 constexpr int CG_MAX_CTAS = DOT_CHUNKS / 2;  // partials: CTAs of A, then two per CTA of B
 template <class T>
 constexpr int cg_groups() { return grid_ctas_per_sm<T>(); }
@@ -207,6 +210,7 @@ struct GridCg {
   double *scal, *part;
   unsigned* count;  // zero before the launch
   int iters, n_items;
+  int cached, slabs;  // vectors kept in shared memory (of r, dinv, x, p), entries / (4 grid NT)
 };
 
 // The scalars of the recursion.  FP32 vectors: unevaluated float pairs throughout (two-sums,
@@ -343,6 +347,26 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
   bool done = G.scal[SCAL_DONE] != 0.0;
   int it = 0;
   const int64_t i0 = 4 * ((int64_t)blockIdx.x * NT + threadIdx.x), stride = 4 * (int64_t)gridDim.x * NT;
+  // entries i0 + j stride + 0..3 are this thread's throughout: vectors 0 (r), 1 (dinv), 2 (x), 3
+  // (p) in shared memory as far as they fit
+  T* const cache = reinterpret_cast<T*>(sh + NG) + 4 * threadIdx.x;
+  auto kept = [&](int v, int j) { return cache + ((size_t)v * G.slabs + j) * (4 * NT); };
+  auto get = [&](int v, const T* g, int64_t i, int j, T (&o)[4]) {
+    if (v < G.cached) ldv(kept(v, j), o);
+    else ld4n(g, i, G.n, o);
+  };
+  auto put = [&](int v, T* g, int64_t i, int j, const T (&o)[4]) {
+    if (v < G.cached) stv(kept(v, j), o);
+    else st4n(g, i, G.n, o);
+  };
+  for (int j = 0; j < G.slabs; ++j) {
+    const int64_t i = i0 + j * stride;
+    T t[4];  // zero beyond n
+    if (G.cached > 0) { ld4n(G.r, i, G.n, t); stv(kept(0, j), t); }
+    if (G.cached > 1) { ld4n(G.dinv, i, G.n, t); stv(kept(1, j), t); }
+    if (G.cached > 2) { ld4n(G.x, i, G.n, t); stv(kept(2, j), t); }
+    if (G.cached > 3) { ld4n(G.p, i, G.n, t); stv(kept(3, j), t); }
+  }
   while (it < G.iters && !done && flag == 0.0) {
     GridDotAcc<T> dot;
     for (int item = group * gridDim.x + blockIdx.x; item < G.n_items; item += NG * gridDim.x) {
@@ -367,18 +391,19 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
     }
     DotAcc<T> a0, a1;
 #pragma unroll 2
-    for (int64_t i = i0; i < G.n; i += stride) {
+    for (int j = 0; j < G.slabs; ++j) {
+      const int64_t i = i0 + j * stride;
       T rv[4], qv[4], dv[4];
-      ld4n(G.r, i, G.n, rv);
       ld4n(G.q, i, G.n, qv);
-      ld4n(G.dinv, i, G.n, dv);
+      get(0, G.r, i, j, rv);
+      get(1, G.dinv, i, j, dv);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         rv[k] = rv[k] - alpha * qv[k];
         a0.add(rv[k], rv[k] * dv[k]);
         a1.add(rv[k], rv[k]);
       }
-      st4n(G.r, i, G.n, rv);
+      put(0, G.r, i, j, rv);
     }
     const S v[2] = {scalar_of(a0), scalar_of(a1)};
     S s[2];
@@ -397,25 +422,35 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
     done = rr.at_most(tol2);
     const bool stop = done || flag != 0.0;  // the direction stays as it is
 #pragma unroll 2
-    for (int64_t i = i0; i < G.n; i += stride) {
+    for (int j = 0; j < G.slabs; ++j) {
+      const int64_t i = i0 + j * stride;
       T xv[4], pv[4], rv[4], dv[4];
-      ld4n(G.x, i, G.n, xv);
-      ld4n(G.p, i, G.n, pv);
-      ld4n(G.r, i, G.n, rv);
-      ld4n(G.dinv, i, G.n, dv);
+      get(2, G.x, i, j, xv);
+      get(3, G.p, i, j, pv);
+      get(0, G.r, i, j, rv);
+      get(1, G.dinv, i, j, dv);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         xv[k] += alpha * pv[k];
         pv[k] = rv[k] * dv[k] + beta * pv[k];
       }
-      st4n(G.x, i, G.n, xv);
-      if (!stop) st4n(G.p, i, G.n, pv);
+      put(2, G.x, i, j, xv);
+      if (!stop) {
+        st4n(G.p, i, G.n, pv);
+        if (G.cached > 3) stv(kept(3, j), pv);
+      }
     }
     if (stop || it == G.iters) break;
     if (!grid_barrier(G.count, target += gridDim.x)) {
       flag = 2.0;
       break;
     }
+  }
+  for (int j = 0; j < G.slabs; ++j) {
+    const int64_t i = i0 + j * stride;
+    T t[4];
+    if (G.cached > 0) { ldv(kept(0, j), t); st4n(G.r, i, G.n, t); }
+    if (G.cached > 2) { ldv(kept(2, j), t); st4n(G.x, i, G.n, t); }
   }
   if (it > 0 && blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read the scalars
     const double z1 = rz.value(), z0 = rz_old.value();
@@ -447,16 +482,21 @@ int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,
     const int64_t items = grid_setup<T>(plan, mu, lam, P, cg_groups<T>() * sms);
     if (items <= 0) return set_error(TG_ERR_VALUE, "grid CG: empty or too large grid");
     GridCg<T> G{(T*)x, (T*)r, (T*)p, (T*)q, (const T*)dinv, node_mask,
-                3 * (int64_t)P.nx * P.ny * P.nz, scal, part, count, iters, (int)items};
+                3 * (int64_t)P.nx * P.ny * P.nz, scal, part, count, iters, (int)items, 0, 0};
     const void* kern = node_mask ? (const void*)grid_cg_kernel<T, MASK_NODE_OUT>
                                  : (const void*)grid_cg_kernel<T, MASK_NONE>;
-    constexpr int smem = cg_groups<T>() * (int)sizeof(GridShared<T>);
-    TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                      "grid CG: shared memory"));
     // one CTA per SM (all resident), none without work
     const int64_t vec = (G.n + 4 * NT - 1) / (4 * NT), want = items > vec ? items : vec;
     int64_t ctas = sms < want ? sms : want;
     ctas = ctas < CG_MAX_CTAS ? ctas : CG_MAX_CTAS;
+    // the SM's shared memory holds as many of the vectors as fit
+    constexpr int tiles = cg_groups<T>() * (int)sizeof(GridShared<T>);
+    G.slabs = (int)((vec + ctas - 1) / ctas);
+    const int64_t vbytes = (int64_t)G.slabs * 4 * NT * sizeof(T), room = CG_SMEM - tiles;
+    G.cached = (int)(room / vbytes < 4 ? room / vbytes : 4);
+    const int smem = tiles + (int)(G.cached * vbytes);
+    TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM),
+                      "grid CG: shared memory"));
     TG_TRY(cuda_check(cudaMemsetAsync(count, 0, sizeof(unsigned), st), "grid CG: barrier"));
     void* args[] = {&P, &G};
     const cudaError_t e =

@@ -827,7 +827,10 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
   int rc = TG_OK;
   bool done = false;
   while (*iters < max_iter) {
-    const int k = (max_iter - *iters) < check_every ? (max_iter - *iters) : check_every;
+    // a persistent launch ends by itself when the solve has: 16 blocks in one, fewer reads
+    // of the scalars by the host (30 us each with the launch; 50 iterations take 600 at 16^3)
+    const int64_t block = (B.persistent ? 16 : 1) * (int64_t)check_every;
+    const int k = (max_iter - *iters) < block ? (max_iter - *iters) : (int)block;
     const int before = *iters;
     if (B.persistent) {
       rc = launch_grid_cg(op->plan, op->prec, op->mat.p0, op->mat.p1, B.nmask, x, B.r, B.p, B.q,

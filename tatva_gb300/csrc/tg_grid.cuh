@@ -63,7 +63,7 @@ namespace tg {
 // FP64: 256 threads, a column each (grid_interior), its kernels being FP64-pipe bound.
 constexpr int GR_DEEP_TZ = 11, GR_MAX_TZ = 15;
 // Unknowns up to which CG iterations run as one cooperative launch (grid_cg_kernel): at 96^3
-// (2.7 M) 37.6 against 41.9 us an iteration in three launches, at 128^3 (6.4 M), where the
+// (2.7 M) 37.0 against 41.9 us an iteration in three launches, at 128^3 (6.4 M), where the
 // vector passes want more loads in flight than one CTA per SM keeps, 90.1 against 81.5.
 constexpr int64_t GRID_CG_MAX_DOFS = 3500000;
 constexpr int GR_TX = 32, GR_TY = 8;
