@@ -445,7 +445,9 @@ TG_API int tg_operator_apply(const tg_operator_desc* op, const void* x, void* y,
                       size_t workspace_bytes, void* stream);
 
 /* Jacobi-preconditioned CG, all vectors of precision op->prec, scalars and dot
- * products in FP64 on the device.  Solves A x = b from the given x.  The loop runs
+ * products on the device to FP64's precision or better (FP32: exact products, pairs
+ * of floats over the few dozen entries of a thread, whose sum has to stay in FP32's
+ * range, then FP64, or three floats on a brick that runs as one launch).  Solves A x = b from the given x.  The loop runs
  * `check_every` iterations per CUDA graph replay between host convergence checks
  * and never exceeds max_iter; the stopping test itself runs on the device after
  * every iteration, so the result does not depend on check_every.  On a structured
@@ -457,7 +459,7 @@ TG_API int tg_cg_solve(const tg_operator_desc* op, const void* b, void* x, const
                 double rtol, int max_iter, int check_every, void* workspace,
                 size_t workspace_bytes, tg_solve_stats* stats, void* stream);
 
-/* Mixed precision: FP32 Jacobi-CG inner solves on op32 (FP32 HVP, FP64 dots),
+/* Mixed precision: FP32 Jacobi-CG inner solves on op32 (FP32 HVP, dots as there),
  * FP64 iterative refinement with the true residual r = b - A64 x on op64.
  * b, x, diag64 are FP64; converges to ||b - A64 x|| <= rtol ||b||.  b must be
  * 16-byte aligned (vector loads), else TG_ERR_VALUE.  Each inner solve reduces its

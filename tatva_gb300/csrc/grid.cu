@@ -182,7 +182,8 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
 // One CTA per SM holds the groups that would be separate CTAs, so that a barrier joins 152
 // arrivals and a dot 152 partials.  Every CTA adds the partials itself, in the same fixed
 // order, so all of them hold the same scalars and take the same decisions, and none waits
-// for one that sums up.  Tiles and vector entries are taken by a fixed stride: the result
+// for one that sums up.  The sums and scalars of FP32 vectors keep more than FP64's 53 bits
+// (Sum3); in float pairs, 48 bits, the iteration took as long.  Tiles and vector entries are taken by a fixed stride: the result
 // depends on the number of CTAs alone.
 // Three launches a step spent most of a small or mid-size brick's iteration between kernels
 // and in the arrival counters and last-CTA sums of their dots.  The vectors that only their
@@ -195,7 +196,7 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
 // SCAL_FLAG = 2 and returns.
 constexpr unsigned GRID_SPIN = 1u << 22;
 constexpr int CG_SMEM = 220 * 1024;  // of the 227 KB a CTA can have; the rest: the sums'
-constexpr int CG_MAX_CTAS = DOT_CHUNKS / 2;  // partials: CTAs of A, then two per CTA of B
+constexpr int CG_MAX_CTAS = DOT_CHUNKS / 4;  // partials: CTAs of A, then two per CTA of B
 template <class T>
 constexpr int cg_groups() { return grid_ctas_per_sm<T>(); }
 template <class T>
@@ -213,18 +214,38 @@ struct GridCg {
   int cached, slabs;  // vectors kept in shared memory (of r, dinv, x, p), entries / (4 grid NT)
 };
 
-// The scalars of the recursion.  FP32 vectors: unevaluated float pairs throughout (two-sums,
-// 48 bits, as the threads' accumulators): an FP64 addition takes about 100 clocks here and an
-// FP64 division in every warp 3,000, several times a whole brick's vector pass.  FP64 vectors:
-// FP64, the divisions in one thread.
-__device__ __forceinline__ Scalar<float> scalar_of(const GridDotAcc<float>& a) { return {a.hi, a.lo}; }
-__device__ __forceinline__ Scalar<float> scalar_of(const DotAcc<float>& a) { return {a.hi, a.lo}; }
-__device__ __forceinline__ Scalar<double> scalar_of(const GridDotAcc<double>& a) { return {a.v}; }
-__device__ __forceinline__ Scalar<double> scalar_of(const DotAcc<double>& a) { return {a.v}; }
+// The scalars of the recursion are totals (tg_cg.cuh): three floats for FP32 vectors (an
+// exchange is a chain of some 20 additions, 81 clocks each in FP64) and FP64 for FP64 vectors.
+// The floats' range is FP32's, where the three-launch path adds the threads' sums in FP64:
+// large totals are scaled down by more than the number of threads (CG_MAX_CTAS of them), so
+// that a total overflows no earlier than one thread's sum does.
+template <class T>
+__device__ __forceinline__ T total_scale(double v) {
+  return sizeof(T) == 4 && v > 0x1p60 ? T(0x1p-18) : T(1);
+}
+static_assert(CG_MAX_CTAS * cg_threads<float>() <= 1 << 18, "what total_scale allows for");
+
+// A thread's sum as it is handed to the warp that adds them up: a float pair or a double.
+template <class T>
+struct ThreadSum {
+  float hi, lo;
+  __device__ ThreadSum(const GridDotAcc<T>& a, float scale) : hi(a.hi * scale), lo(a.lo * scale) {}
+  __device__ ThreadSum(const DotAcc<T>& a, float scale) : hi(a.hi * scale), lo(a.lo * scale) {}
+  __device__ Total<T> total() const { return Total<T>::of(hi, lo); }
+  __device__ void add_to(Total<T>& t) const { t.add(hi, lo); }
+};
+template <>
+struct ThreadSum<double> {
+  double v;
+  __device__ ThreadSum(const GridDotAcc<double>& a, double) : v(a.v) {}
+  __device__ ThreadSum(const DotAcc<double>& a, double) : v(a.v) {}
+  __device__ Total<double> total() const { return {v}; }
+  __device__ void add_to(Total<double>& t) const { t.v += v; }
+};
 
 // sum over the warp's lanes (lane 0)
 template <class T>
-__device__ __forceinline__ Scalar<T> warp_total(Scalar<T> a) {
+__device__ __forceinline__ Total<T> warp_total(Total<T> a) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) a.add(a.down(o));
   return a;
@@ -241,61 +262,57 @@ __device__ __forceinline__ bool grid_arrive_wait(unsigned* count, unsigned targe
   return seen >= target;
 }
 
-// The CTA's K sums (v: the thread's) stored as its partials, a grid barrier, and the sums of
-// all CTAs' partials, the same in every thread of every CTA.  False where the wait ran out.
-// den: what v[0]'s total is divided by (quot = total / den) or, with INV, what divides it.
-template <class T, int K, int NT, bool INV>
-__device__ __forceinline__ bool grid_sum(const Scalar<T> (&v)[K], Scalar<T>* part, unsigned* count,
-                                         unsigned target, const Scalar<T>& den, Scalar<T> (&out)[K],
-                                         T& quot) {
-  constexpr int NW = NT / 32;
-  static_assert(NW <= 16, "one warp adds the warps' sums");
-  __shared__ Scalar<T> warps[K][NW], total[K];
-  __shared__ T ratio;
-  __shared__ bool ok;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  Scalar<T> a[K];
+// What the threads share of a recursion: the scalars, thread 0's but for tol2, and what the
+// exchanges decide.
+template <class T>
+struct CgShared {
+  Total<T> rz, rz_old, pq, rr, tol2;
+  T ratio;          // alpha, then beta
+  bool ok[2], bad;  // the wait ended; a sum is not positive (A) or not finite (B)
+  bool done;
+};
+
+// The K sums over all threads of all CTAs.  Warp k adds value k of its CTA's threads, stores
+// the CTA's total, waits for the other CTAs' (K arrivals each: everything the CTA has written
+// is then visible too) and adds those, in a fixed order: the same totals in every CTA.  (A tree
+// in every warp was more instructions: 64^3 21.3 us an iteration, 16^3 13.1.)
+// v: the thread's sums, handed over in `stage`, the shared memory of the groups' tiles.
+// finish(k, w): lane 0 of warp k with value k's total.
+template <class T, int K, int NT, class F>
+__device__ __forceinline__ bool grid_sum(const ThreadSum<T> (&v)[K], GridShared<T>* stage,
+                                         Total<T>* part, unsigned* count, unsigned target,
+                                         CgShared<T>& S, F&& finish) {
+  constexpr int NW = NT / 32, GT = grid_threads<T>();
+  const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+  auto slot = [&](int t, int kk) -> ThreadSum<T>& {
+    return reinterpret_cast<ThreadSum<T>*>(stage + t / GT)[kk * GT + t % GT];
+  };
 #pragma unroll
-  for (int k = 0; k < K; ++k) a[k] = warp_total<T>(v[k]);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) warps[k][warp] = a[k];
+  for (int kk = 0; kk < K; ++kk) slot(threadIdx.x, kk) = v[kk];
   __syncthreads();
-  if (warp == 0) {
+  if (k < K) {
+    Total<T> w = slot(lane, k).total();
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      a[k] = lane < NW ? warps[k][lane] : Scalar<T>::of(0.0);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) a[k].add(a[k].down(o));
-      if (lane == 0) part[K * blockIdx.x + k] = a[k];
-    }
+    for (int j = 1; j < NW; ++j) slot(lane + 32 * j, k).add_to(w);
+    w = warp_total<T>(w);
     bool here = true;
-    if (lane == 0) here = grid_arrive_wait(count, target);
-    here = __shfl_sync(0xffffffffu, (int)here, 0) != 0;
-    Scalar<T> w[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) w[k] = Scalar<T>::of(0.0);
-#pragma unroll 8
-    for (int i = lane; i < (int)gridDim.x; i += 32)
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const double raw = __ldcg(reinterpret_cast<const double*>(part) + K * i + k);
-        w[k].add(*reinterpret_cast<const Scalar<T>*>(&raw));
-      }
-#pragma unroll
-    for (int k = 0; k < K; ++k) w[k] = warp_total<T>(w[k]);
     if (lane == 0) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) total[k] = w[k];
-      ratio = INV ? den.over(w[0]) : w[0].over(den);
-      ok = here;
+      w.store(part + K * blockIdx.x + k);
+      here = grid_arrive_wait(count, target);
+    }
+    here = __shfl_sync(0xffffffffu, (int)here, 0) != 0;
+    w = Total<T>::of(0.0);
+#pragma unroll 8
+    for (int i = lane; i < (int)gridDim.x; i += 32) w.add(Total<T>::load(part + K * i + k));
+    w = warp_total<T>(w);
+    if (lane == 0) {
+      w.normalize();
+      S.ok[k] = here;
+      finish(k, w);
     }
   }
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = total[k];
-  quot = ratio;
-  return ok;
+  return S.ok[0] && S.ok[K - 1];
 }
 
 // grid barrier alone
@@ -334,14 +351,21 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
   constexpr int NT = cg_threads<T>(), NG = cg_groups<T>();
   extern __shared__ __align__(16) unsigned char cg_smem[];
   GridShared<T>* sh = reinterpret_cast<GridShared<T>*>(cg_smem);  // one per group
-  using S = Scalar<T>;
-  static_assert(sizeof(S) == sizeof(double), "a partial is one 8-byte slot");
+  using S = Total<T>;
+  static_assert(3 * CG_MAX_CTAS * sizeof(S) <= 2 * DOT_CHUNKS * sizeof(double), "partials fit");
   const int group = threadIdx.x / grid_threads<T>();
   S* part_a = reinterpret_cast<S*>(G.part);
   S* part_b = part_a + CG_MAX_CTAS;
+  __shared__ CgShared<T> C;
   unsigned target = 0;
-  S rz = S::of(G.scal[SCAL_RZ]), rr = S::of(G.scal[SCAL_RR]), pq = S::of(0.0), rz_old = rz;
-  const S tol2 = S::of(G.scal[SCAL_TOL2]);
+  const T sz = total_scale<T>(G.scal[SCAL_RZ]), sr = total_scale<T>(G.scal[SCAL_RR]);
+  if (threadIdx.x == 0) {
+    C.rz = S::of((double)sz * G.scal[SCAL_RZ]);
+    C.rr = S::of((double)sr * G.scal[SCAL_RR]);
+    C.tol2 = S::of((double)sr * G.scal[SCAL_TOL2]);
+    C.pq = S::of(0.0);
+    C.rz_old = C.rz;
+  }
   T alpha = T(0), beta = T(0);
   double flag = G.scal[SCAL_FLAG];
   bool done = G.scal[SCAL_DONE] != 0.0;
@@ -375,20 +399,25 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
       group_sync<T, true>();  // the next item restages the group's shared memory
     }
     {
-      const S v[1] = {scalar_of(dot)};
-      S s[1];
-      if (!grid_sum<T, 1, NT, true>(v, part_a, G.count, target += gridDim.x, rz, s, alpha)) {
+      const ThreadSum<T> v[1] = {{dot, sz}};
+      const bool met = grid_sum<T, 1, NT>(v, sh, part_a, G.count, target += gridDim.x, C,
+                                          [&](int, const S& w) {
+                                            C.pq = w;
+                                            C.bad = !w.positive() || !w.finite();
+                                            C.ratio = C.rz.over(w);
+                                          });
+      if (!met) {
         flag = 2.0;
         break;
       }
-      pq = s[0];
     }
     ++it;
-    if (!pq.positive() || !pq.finite()) {
+    if (C.bad) {
       flag = 1.0;
       alpha = T(0);
       break;
     }
+    alpha = C.ratio;
     DotAcc<T> a0, a1;
 #pragma unroll 2
     for (int j = 0; j < G.slabs; ++j) {
@@ -405,21 +434,31 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
       }
       put(0, G.r, i, j, rv);
     }
-    const S v[2] = {scalar_of(a0), scalar_of(a1)};
-    S s[2];
-    if (!grid_sum<T, 2, NT, false>(v, part_b, G.count, target += gridDim.x, rz, s, beta)) {
+    const ThreadSum<T> v[2] = {{a0, sz}, {a1, sr}};
+    const bool met = grid_sum<T, 2, NT>(v, sh, part_b, G.count, target += 2 * gridDim.x, C,
+                                        [&](int k, const S& w) {
+                                          if (k == 0) {
+                                            C.bad = !w.finite();
+                                            C.ratio = w.over(C.rz);
+                                            if (!C.bad) {
+                                              C.rz_old = C.rz;
+                                              C.rz = w;
+                                            }
+                                          } else {
+                                            C.rr = w;
+                                            C.done = w.at_most(C.tol2);
+                                          }
+                                        });
+    if (!met) {
       flag = 2.0;
       break;
     }
-    rr = s[1];
-    if (!s[0].finite()) {
+    done = C.done;
+    beta = C.ratio;
+    if (C.bad) {
       flag = 1.0;
       beta = T(0);
-    } else {
-      rz_old = rz;
-      rz = s[0];
     }
-    done = rr.at_most(tol2);
     const bool stop = done || flag != 0.0;  // the direction stays as it is
 #pragma unroll 2
     for (int j = 0; j < G.slabs; ++j) {
@@ -453,12 +492,12 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
     if (G.cached > 2) { ldv(kept(2, j), t); st4n(G.x, i, G.n, t); }
   }
   if (it > 0 && blockIdx.x == 0 && threadIdx.x == 0) {  // every CTA has read the scalars
-    const double z1 = rz.value(), z0 = rz_old.value();
-    G.scal[SCAL_PQ] = pq.value();
+    const double z1 = C.rz.value() / (double)sz, z0 = C.rz_old.value() / (double)sz;
+    G.scal[SCAL_PQ] = C.pq.value() / (double)sz;
     G.scal[SCAL_ALPHA] = (double)alpha;
     G.scal[SCAL_BETA] = flag == 0.0 ? z1 / z0 : 0.0;
     G.scal[SCAL_RZ] = z1;
-    G.scal[SCAL_RR] = rr.value();
+    G.scal[SCAL_RR] = C.rr.value() / (double)sr;
     G.scal[SCAL_DONE] = done ? 1.0 : 0.0;
     G.scal[SCAL_ITERS] += (double)it;
   }

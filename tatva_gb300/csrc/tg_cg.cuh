@@ -4,6 +4,7 @@
 #pragma once
 
 #include "tg_common.cuh"
+#include "tg_sum.h"
 
 namespace tg {
 
@@ -38,7 +39,7 @@ __device__ __forceinline__ void stv(double* p, const double (&v)[4]) {
 // FP32 vectors: each thread accumulates x_i y_i as an unevaluated pair (hi, lo) of
 // floats -- the product is split exactly with an FMA and added with a two-sum, so the
 // thread's partial keeps about 48 bits -- and only the per-thread partials enter the
-// FP64 tree reduction.  (This GPU's FP64 rate is a small fraction of FP32: per-element
+// tree reduction, in FP64 or in three floats (Sum3).  (This GPU's FP64 rate is a small fraction of FP32: per-element
 // FP64 conversions and multiply-adds made the dots several times slower than their
 // memory traffic.)  FP64 vectors accumulate in FP64.
 template <class T>
@@ -62,6 +63,58 @@ struct DotAcc<double> {
   double v = 0.0;
   __device__ __forceinline__ void add(double a, double b) { v += a * b; }
   __device__ __forceinline__ double value() const { return v; }
+};
+
+// The scalars of a recursion on vectors of T and their sums over threads: Sum3 for FP32,
+// FP64 for FP64.
+template <class T>
+struct Total;
+template <>
+struct Total<float> : Sum3 {
+  __device__ static Total of(double v) { return {Sum3::of(v)}; }
+  __device__ static Total of(float hi, float lo) { return {Sum3::of(hi, lo)}; }
+  __device__ Total down(int o) const {
+    return {{__shfl_down_sync(0xffffffffu, s, o), __shfl_down_sync(0xffffffffu, c, o),
+             __shfl_down_sync(0xffffffffu, cc, o)}};
+  }
+  // of a total that another CTA stored
+  __device__ static Total load(const Total* p) {
+    const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+    return {{t.x, t.y, t.z}};
+  }
+  __device__ void store(Total* p) const {
+    *reinterpret_cast<float4*>(p) = make_float4(s, c, cc, 0.f);
+  }
+  // the tests and the quotient take normalized totals
+  __device__ bool finite() const { return isfinite(s) && isfinite(c); }
+  __device__ bool positive() const { return s > 0.f; }
+  __device__ bool at_most(const Total& o) const {
+    return (s - o.s) + ((c - o.c) + (cc - o.cc)) <= 0.f;
+  }
+  // this / o, rounded to FP32: an approximate quotient and the quotient of its exact
+  // residual (a division in FP64 takes 580 clocks)
+  __device__ float over(const Total& o) const {
+    if (o.s < 0x1p-120f || o.s > 0x1p120f) return (float)(value() / o.value());
+    const float q = __fdividef(s, o.s);
+    if (!isfinite(q)) return q;
+    const float r = fmaf(-q, o.s, s) + (fmaf(-q, o.c, c) + fmaf(-q, o.cc, cc));
+    return q + __fdividef(r, o.s);
+  }
+};
+template <>
+struct Total<double> {
+  double v;
+  __device__ static Total of(double a) { return {a}; }
+  __device__ double value() const { return v; }
+  __device__ void add(const Total& o) { v += o.v; }
+  __device__ void normalize() {}
+  __device__ Total down(int o) const { return {__shfl_down_sync(0xffffffffu, v, o)}; }
+  __device__ static Total load(const Total* p) { return {__ldcg(&p->v)}; }
+  __device__ void store(Total* p) const { p->v = v; }
+  __device__ bool finite() const { return isfinite(v); }
+  __device__ bool positive() const { return v > 0.0; }
+  __device__ bool at_most(const Total& o) const { return v <= o.v; }
+  __device__ double over(const Total& o) const { return v / o.v; }
 };
 
 template <class T>
@@ -94,18 +147,6 @@ struct Scalar<float> {
     const float r = fmaf(-q, o.hi, hi) + fmaf(-q, o.lo, lo);
     return q + __fdividef(r, o.hi);
   }
-};
-template <>
-struct Scalar<double> {
-  double v;
-  __device__ static Scalar of(double a) { return {a}; }
-  __device__ double value() const { return v; }
-  __device__ void add(const Scalar& o) { v += o.v; }
-  __device__ Scalar down(int o) const { return {__shfl_down_sync(0xffffffffu, v, o)}; }
-  __device__ bool finite() const { return isfinite(v); }
-  __device__ bool positive() const { return v > 0.0; }
-  __device__ bool at_most(const Scalar& o) const { return v <= o.v; }
-  __device__ double over(const Scalar& o) const { return v / o.v; }
 };
 
 // ------------------------------------------------------------------ reductions
