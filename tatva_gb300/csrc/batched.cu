@@ -19,21 +19,22 @@
 // iteration.
 //
 // Bound: the latency of an iteration (two sums over the CTA or cluster, the SpMV's
-// dependent loads), 2.0 us for 289 rows, 3.2 us for 9,409 rows on a cluster; at full
+// dependent loads), 2.3 us for 289 rows, 3.3 us for 9,409 rows on a cluster; at full
 // load the shared-memory loads (2.5 per entry).  768 unit squares of 8..96 cells a side:
-// 28.5 -> 5.6 ms; 4,096 of them 59.7 -> 30.7; 4,096 of 6..24: 13.9 -> 1.6.  Before, one CTA
+// 28.5 -> 6.0 ms; 4,096 of them 59.7 -> 32.1; 4,096 of 6..24: 13.9 -> 1.8 (5.5, 29.8 and 1.6
+// with sums in float pairs, 48 bits).  Before, one CTA
 // streamed a system's matrix from the L2 and DRAM: 27 us an iteration for the largest, which
 // the whole batch waited for, and FP64 sums in every warp, 7 us for the smallest.  Clusters
 // of two: 10 ms, of eight: 14 (768 squares).
 //
 // Each system runs FP32 Jacobi-preconditioned CG on the residual direction
 // r64 / |r64| and FP64 iterative refinement on the true residual b - A64 x, until
-// |b - A64 x| <= rtol |b|.  Dots accumulate as exact-product float pairs (about 48 bits)
-// through the whole sum, in a fixed order, so each system's result depends only on its own
-// data and the block size -- not on which CTA took it, nor on what else ran.  Every loop is
-// bounded by max_outer / max_inner; CTAs wait for others of their cluster only, at cluster
-// barriers that all of it reach (every decision is taken on sums that are the same bits
-// in each).
+// |b - A64 x| <= rtol |b|.  Dots accumulate as exact-product float pairs in a thread and to
+// more than FP64's 53 bits (three floats, tg_sum.h) beyond it, in a fixed order, so each
+// system's result depends only on its own data and the block size -- not on which CTA took it,
+// nor on what else ran.  Every loop is bounded by max_outer / max_inner; CTAs wait for others
+// of their cluster only, at cluster barriers that all of it reach (every decision is taken on
+// sums that are the same bits in each).
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -50,11 +51,12 @@ constexpr int TEAM = 4;  // CTAs of a cluster
 // and 1 KB for the system are the CTA's own)
 constexpr int batch_smem(int nt, int per_sm) { return 228 * 1024 / per_sm - 2048 - 16 * nt; }
 // What one CTA solves alone: its FP32 matrix and p within half an SM's shared memory, its
-// vectors within its registers (10 rows a thread at 256 threads).  768 squares of 8..96: 5.6
-// ms with this limit, 5.9 with 80 KB, 7 with 54 KB (more work at cluster barriers).
+// vectors within its registers (10 rows a thread at 256 threads).  768 squares of 8..96, with
+// sums in float pairs: 5.6 ms with this limit, 5.9 with 80 KB, 7 with 54 KB (more work at
+// cluster barriers).
 constexpr int64_t SOLO_BYTES = 103 * 1024;
 constexpr int SOLO_ROWS = 2560;
-using Pair = Scalar<float>;
+using Total32 = Total<float>;
 
 struct BatchArgs {
   tg_batch_desc d;
@@ -96,30 +98,26 @@ __device__ __forceinline__ void put(unsigned addr, float v) {
 __device__ __forceinline__ void put(unsigned addr, int v) {
   asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void put(unsigned addr, Pair v) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.hi), "f"(v.lo) : "memory");
+__device__ __forceinline__ void put(unsigned addr, const Total32& v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.s),
+               "f"(v.c), "f"(v.cc), "f"(0.f)
+               : "memory");
 }
 __device__ __forceinline__ void put(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
-__device__ __forceinline__ Pair shfl_down(const Pair& v, int o) { return v.down(o); }
-__device__ __forceinline__ double shfl_down(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ Pair lane0(const Pair& v) {
-  return {__shfl_sync(0xffffffffu, v.hi, 0), __shfl_sync(0xffffffffu, v.lo, 0)};
-}
-__device__ __forceinline__ double lane0(double v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ void acc(Pair& a, const Pair& b) { a.add(b); }
-__device__ __forceinline__ void acc(double& a, double b) { a += b; }
 
 // The CTAs that solve one system: the whole cluster (size TEAM) or this CTA alone.
 template <int NT>
 struct Crew {
   static constexpr int NW = NT / 32;
   struct Shared {
-    Pair part[2][NT];          // the threads' partial sums
-    Pair total[2][2][TEAM];    // the CTAs' sums; two halves, used in turn
+    float2 part[2][NT];        // the threads' partial sums
+    Total32 total[2][2][TEAM]; // the CTAs' sums; two halves, used in turn
     double dtotal[2][TEAM];
     double scal[4];
+    float ratio;  // alpha or NaN, then beta
+    int state;    // of the residual: 0 goes on, 1 small enough, 2 not finite
     int lo[TEAM], hi[TEAM];  // window of every CTA
     int next;
   };
@@ -129,53 +127,74 @@ struct Crew {
   __device__ void sync() const {
     if (size > 1) cluster_sync(); else __syncthreads();
   }
-  __device__ Pair* part(Pair*, int k) const { return S.part[k]; }
-  __device__ double* part(double*, int k) const { return reinterpret_cast<double*>(S.part[k]); }
-  __device__ Pair* total(Pair*, int k) const { return S.total[flip][k]; }
-  __device__ double* total(double*, int) const { return S.dtotal[flip]; }
 
-  // Sum of K per-thread values over the crew in a fixed order; every thread gets it.
-  // Warp k adds value k for the whole CTA: a tree in every warp was more instructions
-  // than the rows of a mid-size system.  A CTA may be one sum ahead of the others (its
-  // total goes to the other half), not two (the sync).
-  // between(): work of the threads after warp K - 1 while those add.
-  template <class V, int K>
-  __device__ __forceinline__ void sum(V (&v)[K]) {
-    sum(v, [] {});
-  }
-  template <class V, int K, class F>
-  __device__ __forceinline__ void sum(V (&v)[K], F&& between) {
+  // Sums of K per-thread float pairs over the crew, in a fixed order and to more than FP64's
+  // precision.  Warp k adds value k for the whole CTA: a tree in every warp was more
+  // instructions than the rows of a mid-size system.  finish(k, sum): lane 0 of warp k with
+  // value k's sum, the same in every CTA; what it leaves in S the threads read after the call.  A CTA may be one sum ahead of the others (its total goes to the other half),
+  // not two (the sync).  between(): work of the threads after warp K - 1 while those add.
+  template <int K, class F, class G>
+  __device__ __forceinline__ void sum(const float2 (&v)[K], F&& between, G&& finish) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < K; ++k) part((V*)nullptr, k)[threadIdx.x] = v[k];
+    for (int k = 0; k < K; ++k) S.part[k][threadIdx.x] = v[k];
     __syncthreads();
     if (w < K) {
-      const V* in = part((V*)nullptr, w);
-      V t = in[lane];
+      const float2* in = S.part[w];
+      Total32 t = Total32::of(in[lane].x, in[lane].y);
 #pragma unroll
-      for (int j = 1; j < NW; ++j) acc(t, in[lane + 32 * j]);
+      for (int j = 1; j < NW; ++j) t.add(in[lane + 32 * j].x, in[lane + 32 * j].y);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc(t, shfl_down(t, o));
-      V* out = total((V*)nullptr, w) + rank;
+      for (int o = 16; o > 0; o >>= 1) t.add(t.down(o));
       if (size > 1) {
-        t = lane0(t);
-        if (lane < TEAM) put(remote(out, lane), t);
+        t.s = __shfl_sync(0xffffffffu, t.s, 0);
+        t.c = __shfl_sync(0xffffffffu, t.c, 0);
+        t.cc = __shfl_sync(0xffffffffu, t.cc, 0);
+        if (lane < TEAM) put(remote(S.total[flip][w] + rank, lane), t);
       } else if (lane == 0) {
-        *out = t;
+        finish(w, t);
       }
     } else {
       between();
     }
-    sync();
+    if (size > 1) {
+      cluster_sync();
+      if (w < K && lane == 0) {
+        Total32 t = S.total[flip][w][0];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const V* in = total((V*)nullptr, k);
-      v[k] = in[0];
-      if (size > 1)
-#pragma unroll
-        for (int t = 1; t < TEAM; ++t) acc(v[k], in[t]);
+        for (int r = 1; r < TEAM; ++r) t.add(S.total[flip][w][r]);
+        finish(w, t);
+      }
+      flip ^= 1;
     }
+    __syncthreads();
+  }
+  // the same for one FP64 value per thread; every thread gets the sum
+  __device__ __forceinline__ double sum(double v) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* part = reinterpret_cast<double*>(S.part[0]);
+    part[threadIdx.x] = v;
+    __syncthreads();
+    if (w == 0) {
+      double t = part[lane];
+#pragma unroll
+      for (int j = 1; j < NW; ++j) t += part[lane + 32 * j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+      if (size > 1) {
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (lane < TEAM) put(remote(S.dtotal[flip] + rank, lane), t);
+      } else if (lane == 0) {
+        S.dtotal[flip][0] = t;
+      }
+    }
+    sync();
+    v = S.dtotal[flip][0];
+    if (size > 1)
+#pragma unroll
+      for (int t = 1; t < TEAM; ++t) v += S.dtotal[flip][t];
     flip ^= 1;
+    return v;
   }
 };
 
@@ -357,7 +376,7 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
   };
 
   // set-up: inverse diagonal, x = 0, r64 = b, |b|^2; the matrix
-  double s2[1] = {0.0};
+  double s2 = 0.0;
   bool bad = false;
   {
     const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
@@ -391,15 +410,14 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
       x[i] = 0.0;
       const double bi = b[i];
       r64[i] = bi;
-      s2[0] += bi * bi;
+      s2 += bi * bi;
     }
   }
-  crew.sum(s2);  // also publishes the windows
-  Pair nbad[1] = {{bad ? 1.f : 0.f, 0.f}};
-  crew.sum(nbad);
+  s2 = crew.sum(s2);  // also publishes the windows
+  const double nbad = crew.sum(bad ? 1.0 : 0.0);
   // scal: |b|, |r|, |r| / |b|, 1 / |r|
   double* const scal = crew.S.scal;
-  if (tid == 0) scal[0] = scal[1] = sqrt(s2[0]);
+  if (tid == 0) scal[0] = scal[1] = sqrt(s2);
   __syncthreads();
   // What `pown` holds, to the CTAs whose windows have these rows: p into the window, or
   // z into hz (the window without that CTA's own rows).  By the warps from 2 on, after a
@@ -420,7 +438,7 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
     }
   };
   int status = TG_OK, it_total = 0, n_outer = 0;
-  if (nbad[0].hi > 0.f) {
+  if (nbad > 0.0) {
     status = TG_ERR_BREAKDOWN;  // a non-positive diagonal entry: not SPD
     if (tid == 0) scal[2] = 1.0;
   } else if (!(scal[0] > 0.0)) {
@@ -453,10 +471,12 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
         __syncthreads();
         publish(false);
       }
-      Pair t2[2] = {{rz_acc.hi, rz_acc.lo}, {rr_acc.hi, rr_acc.lo}};
-      crew.sum(t2);  // also publishes p
-      Pair rz = t2[0];
-      const Pair stop = Pair::of(a.inner_rtol * a.inner_rtol * t2[1].value());
+      const float2 t2[2] = {{rz_acc.hi, rz_acc.lo}, {rr_acc.hi, rr_acc.lo}};
+      Total32 kept;  // r.z in thread 0, the |r|^2 to stop at in thread 32
+      crew.sum(t2, [] {}, [&](int k, const Total32& t) {  // also publishes p
+        kept = t;
+        if (k == 1) kept = Total32::of(a.inner_rtol * a.inner_rtol * t.value());
+      });
       bool broke = false;
       for (int it = 0; it < a.max_inner; ++it) {
         DotAcc<float> pq_acc;
@@ -504,11 +524,13 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
             }
           }
         }
-        Pair t1[1] = {{pq_acc.hi, pq_acc.lo}};
-        crew.sum(t1);
+        const float2 t1[1] = {{pq_acc.hi, pq_acc.lo}};
+        crew.sum(t1, [] {}, [&](int, const Total32& t) {
+          crew.S.ratio = t.positive() && t.finite() ? kept.over(t) : NAN;
+        });
         ++it_total;
-        if (!t1[0].positive() || !t1[0].finite()) { broke = true; break; }
-        const float alpha = rz.over(t1[0]);
+        const float alpha = crew.S.ratio;
+        if (isnan(alpha)) { broke = true; break; }
         DotAcc<float> rz2, rr2;
         each([&](int j, int i, bool ok) {
           D(j, i) = fmaf(alpha, Pv(j, i), D(j, i));
@@ -520,14 +542,26 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
           rr2.add(ri, ri);
           if (PP > 0 && crew.size > 1 && ok) pown[i] = zi;  // p itself is in registers
         });
-        Pair t3[2] = {{rz2.hi, rz2.lo}, {rr2.hi, rr2.lo}};
-        crew.sum(t3, [&] {
-          if (PP > 0 && crew.size > 1) publish(true);
-        });
-        if (!t3[1].finite()) { broke = true; break; }
-        if (t3[1].at_most(stop)) break;
-        const float beta = t3[0].over(rz);
-        rz = t3[0];
+        const float2 t3[2] = {{rz2.hi, rz2.lo}, {rr2.hi, rr2.lo}};
+        crew.sum(
+            t3,
+            [&] {
+              if (PP > 0 && crew.size > 1) publish(true);
+            },
+            [&](int k, const Total32& t) {
+              if (k == 0) {
+                crew.S.ratio = t.over(kept);
+                kept = t;
+              } else {
+                crew.S.state = !t.finite() ? 2 : (t.at_most(kept) ? 1 : 0);
+              }
+            });
+        const int state = crew.S.state;
+        if (state) {
+          broke = state == 2;
+          break;
+        }
+        const float beta = crew.S.ratio;
         each([&](int j, int i, bool ok) {
           const float pi = fmaf(beta, Pv(j, i), PP > 0 ? Q(j, i) : R(j, i) * G(j, i));
           Pv(j, i) = pi;
@@ -559,7 +593,7 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
       });
       if (crew.size > 1) __threadfence();
       crew.sync();
-      double u2[1] = {0.0};
+      double u2 = 0.0;
       const double* xs = x - f0;
       const uint16_t* __restrict__ col = at_entry(a.d.ell_col);
       const double* __restrict__ v64 = at_entry(a.d.ell_val64);
@@ -573,10 +607,10 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
           s -= v64[e] * __ldcg(xs + col[e]);
         }
         rs[i] = s;
-        u2[0] += s * s;
+        u2 += s * s;
       }
-      crew.sum(u2);
-      if (tid == 0) scal[1] = sqrt(u2[0]);
+      u2 = crew.sum(u2);
+      if (tid == 0) scal[1] = sqrt(u2);
       __syncthreads();
       if (!isfinite(scal[1])) { status = TG_ERR_BREAKDOWN; break; }
     }
@@ -802,9 +836,10 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
     return launch_check("tg_batch_solve");
   };
   // Many small systems (two or more for every CTA at four to an SM): few registers and
-  // little shared memory, four CTAs of 256 on an SM instead of two.  4,096 squares of 6..24:
-  // 1.6 ms, 2.2 with two to an SM; 700 of 6..31: 0.88 ms, 0.52 with two (the largest systems
-  // then share an SM with fewer others).  The rows of a thread and every sum are the same.
+  // little shared memory, four CTAs of 256 on an SM instead of two.  With sums in float pairs,
+  // 4,096 squares of 6..24: 1.6 ms, 2.2 with two to an SM; 700 of 6..31: 0.88 ms, 0.52 with
+  // two (the largest systems then share an SM with fewer others).  The rows of a thread and
+  // every sum are the same.
   const bool many = desc->n_systems >= 8 * sms;
   switch (threads) {
     case 128:

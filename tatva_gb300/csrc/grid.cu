@@ -183,8 +183,8 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
 // arrivals and a dot 152 partials.  Every CTA adds the partials itself, in the same fixed
 // order, so all of them hold the same scalars and take the same decisions, and none waits
 // for one that sums up.  The sums and scalars of FP32 vectors keep more than FP64's 53 bits
-// (Sum3); in float pairs, 48 bits, the iteration took as long.  Tiles and vector entries are taken by a fixed stride: the result
-// depends on the number of CTAs alone.
+// (Sum3); in float pairs, 48 bits, the iteration took as long.  Tiles and vector entries are
+// taken by a fixed stride: the result depends on the number of CTAs alone.
 // Three launches a step spent most of a small or mid-size brick's iteration between kernels
 // and in the arrival counters and last-CTA sums of their dots.  The vectors that only their
 // own thread touches (r, 1 / diag, x, and its p) stay in shared memory as far as they fit.

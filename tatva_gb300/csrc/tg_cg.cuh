@@ -85,9 +85,8 @@ struct Total<float> : Sum3 {
   __device__ void store(Total* p) const {
     *reinterpret_cast<float4*>(p) = make_float4(s, c, cc, 0.f);
   }
-  // the tests and the quotient take normalized totals
-  __device__ bool finite() const { return isfinite(s) && isfinite(c); }
-  __device__ bool positive() const { return s > 0.f; }
+  __device__ bool finite() const { return isfinite(s + c); }
+  __device__ bool positive() const { return s + c > 0.f; }
   __device__ bool at_most(const Total& o) const {
     return (s - o.s) + ((c - o.c) + (cc - o.cc)) <= 0.f;
   }

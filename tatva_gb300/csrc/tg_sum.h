@@ -36,9 +36,8 @@ struct alignas(16) Sum3 {
   }
   TG_HD double value() const { return (double)s + ((double)c + (double)cc); }
   TG_HD void add(const Sum3& o) {
-    const float e = two_sum(s, o.s);
-    const float d = two_sum(c, o.c);
-    cc += o.cc + (d + two_sum(c, e));
+    cc += o.cc;
+    add(o.s, o.c);
   }
   // a float pair, as the threads' accumulators hold
   TG_HD void add(float hi, float lo) {
