@@ -25,8 +25,9 @@
 //
 // Bound: the HVP's instructions (29 us for 2.2 M nodes) and the traffic of the vector passes
 // (40 bytes a dof and step: 13 + 12 us; with d in the update, and an FP64 tree for the dots
-// in every warp, 23 + 9).  Restarting the inner CG at every refinement took 14,438 steps for
-// 24 requests of 16..64 a side, 170 ms with the warm-up; stages 13,134 and 126 ms.
+// in every warp, 23 + 9).  The dots' sums beyond a thread keep more than FP64's 53 bits
+// (tg_sum.h), and so do the scalars.  Restarting the inner CG at every refinement took 14,438 steps for
+// 24 requests of 16..64 a side, 170 ms with the warm-up; stages 13,134 and 130 ms.
 //
 // A step is `iterations` CG steps with the refinement launches before every 20th, for
 // every slot in use; a slot whose phase does not match a launch leaves it at once.  The
@@ -78,7 +79,7 @@ struct BrickSlot {
   double s, s_prev;   // |r64| of the running stage and of the one before: the units of d, r, p
   double target;      // |r64| at which the running inner solve ends
   double tol2;        // |r|^2 at which its running stage ends
-  Scalar<float> rz, rz_prev;
+  Total<float> rz, rz_prev;
   float alpha, beta, gamma;  // of the last CG step; p = z + beta p + gamma r
   int stages, last_stage, inner_iters;
   unsigned ticket[4];  // arrival counters: HVP, update, residual, resume
@@ -138,22 +139,22 @@ __device__ __forceinline__ void sum_parts(const double* part, int count, double 
   for (int k = 0; k < K; ++k) out[k] = sh[k];
 }
 
-// the same for float pairs
+// the same for the totals of FP32 vectors
 template <int K, int NT>
-__device__ __forceinline__ void sum_parts(const Scalar<float>* part, int count,
-                                          Scalar<float> (&out)[K]) {
+__device__ __forceinline__ void sum_parts(const Total<float>* part, int count,
+                                          Total<float> (&out)[K]) {
 #pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = {0.f, 0.f};
+  for (int k = 0; k < K; ++k) out[k] = Total<float>::of(0.0);
   for (int i = threadIdx.x; i < count; i += NT)
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float2 t = __ldcg(reinterpret_cast<const float2*>(part + K * i + k));
-      out[k].add({t.x, t.y});
-    }
-  __shared__ Scalar<float> sh[K];
+    for (int k = 0; k < K; ++k) out[k].add(Total<float>::load(part + K * i + k));
+  __shared__ Total<float> sh[K];
   block_sum<K, NT>(out, sh);
 #pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = sh[k];
+  for (int k = 0; k < K; ++k) {
+    out[k] = sh[k];
+    out[k].normalize();
+  }
 }
 
 // the entry, slot and CTA index of this CTA in the launch (recomputed from the launch
@@ -331,8 +332,8 @@ __global__ void __launch_bounds__(DOT_THREADS)
     az.add(ri, ri * dinv[i]);
     ar.add(ri, ri);
   }
-  Scalar<float> v[3] = {{az.hi, az.lo}, {ar.hi, ar.lo}, {ap.hi, ap.lo}};
-  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  Total<float> v[3] = {total_of(az), total_of(ar), total_of(ap)};
+  Total<float>* part = reinterpret_cast<Total<float>*>(S->part);
   block_sum<3, DOT_THREADS>(v, part + 3 * b);
   if (!last_of(&S->ticket[3], count)) return;
   sum_parts<3, DOT_THREADS>(part, count, v);
@@ -403,9 +404,9 @@ __global__ void __launch_bounds__(grid_threads<float>(), grid_ctas_per_sm<float>
   __syncthreads();
   GridDotAcc<float> dot;
   grid_cta<float, TG_MODE_HVP, MASK_NODE_OUT, true>(P, b, S->p, S->p, S->nmask, S->q, sh, dot);
-  Scalar<float> v[1] = {{dot.hi, dot.lo}};
+  Total<float> v[1] = {Total<float>::of(dot.hi, dot.lo)};
   reslot(L, e, s, S, b, count, slots);  // recomputed: not held in registers across the sweep
-  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  Total<float>* part = reinterpret_cast<Total<float>*>(S->part);
   block_sum<1, GR_THREADS>(v, part + b);
   if (!last_of(&S->ticket[0], count)) return;
   sum_parts<1, GR_THREADS>(part, count, v);
@@ -457,8 +458,8 @@ __global__ void __launch_bounds__(DOT_THREADS)
     a0.add(ri, ri * dinv[i]);
     a1.add(ri, ri);
   }
-  Scalar<float> v[2] = {{a0.hi, a0.lo}, {a1.hi, a1.lo}};
-  Scalar<float>* part = reinterpret_cast<Scalar<float>*>(S->part);
+  Total<float> v[2] = {total_of(a0), total_of(a1)};
+  Total<float>* part = reinterpret_cast<Total<float>*>(S->part);
   block_sum<2, DOT_THREADS>(v, part + 2 * b);
   if (!last_of(&S->ticket[1], count)) return;
   sum_parts<2, DOT_THREADS>(part, count, v);
@@ -492,10 +493,14 @@ int64_t brick_grid_ctas(const int32_t nodes[3]) {
   return grid_setup_dims<T>(nodes, h, 1.0, 1.0, P, true);
 }
 
-size_t brick_part_doubles(const int32_t nodes[3]) {
+// partials: a total per CTA of the HVP or a double per CTA of the residual, three totals per
+// chunk of the resume (the most a launch over chunks stores)
+size_t brick_part_bytes(const int32_t nodes[3]) {
+  constexpr int64_t W = sizeof(Total<float>);
   const int64_t n = 3 * (int64_t)nodes[0] * nodes[1] * nodes[2];
-  const int64_t g32 = brick_grid_ctas<float>(nodes), g64 = brick_grid_ctas<double>(nodes);
-  const int64_t g = g32 > g64 ? g32 : g64, c = 3 * (int64_t)brick_chunks(n);
+  const int64_t g32 = W * brick_grid_ctas<float>(nodes);
+  const int64_t g64 = (int64_t)sizeof(double) * brick_grid_ctas<double>(nodes);
+  const int64_t g = g32 > g64 ? g32 : g64, c = 3 * W * brick_chunks(n);
   return (size_t)(g > c ? g : c);
 }
 
@@ -528,7 +533,7 @@ extern "C" size_t tg_brick_workspace_bytes(const int32_t nodes[3]) {
   if (!nodes || nodes[0] < 2 || nodes[1] < 2 || nodes[2] < 2) return 0;
   const int64_t nn = (int64_t)nodes[0] * nodes[1] * nodes[2], n = 3 * nn;
   return al256((size_t)n * 8) + 5 * al256((size_t)n * 4) + al256((size_t)nn) +
-         al256(brick_part_doubles(nodes) * sizeof(double));
+         al256(brick_part_bytes(nodes));
 }
 
 extern "C" int tg_brick_batch_create(tg_brick_batch** out) {
@@ -624,7 +629,7 @@ extern "C" int tg_brick_admit(tg_brick_batch* bt, const tg_brick_request* req, v
   h.q = (float*)take((size_t)h.n_dofs * 4);
   h.dinv = (float*)take((size_t)h.n_dofs * 4);
   h.nmask = (uint8_t*)take((size_t)h.n_nodes);
-  h.part = (double*)take(brick_part_doubles(nd) * sizeof(double));
+  h.part = (double*)take(brick_part_bytes(nd));
   h.rtol = req->rtol;
   h.inner_rtol = req->inner_rtol;
   h.max_outer = req->max_outer;

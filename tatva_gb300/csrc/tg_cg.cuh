@@ -115,38 +115,10 @@ struct Total<double> {
   __device__ bool at_most(const Total& o) const { return v <= o.v; }
   __device__ double over(const Total& o) const { return v / o.v; }
 };
-
-template <class T>
-struct Scalar;
-template <>
-struct Scalar<float> {
-  float hi, lo;
-  __device__ static Scalar of(double v) {
-    const float h = (float)v;
-    return {h, (float)(v - (double)h)};
-  }
-  __device__ double value() const { return (double)hi + (double)lo; }
-  __device__ void add(const Scalar& o) {
-    const float s = hi + o.hi, b = s - hi;
-    lo += o.lo + ((hi - (s - b)) + (o.hi - b));
-    hi = s;
-  }
-  __device__ Scalar down(int o) const {
-    return {__shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o)};
-  }
-  __device__ bool finite() const { return isfinite(hi) && isfinite(lo); }
-  __device__ bool positive() const { return hi + lo > 0.f; }
-  __device__ bool at_most(const Scalar& o) const { return (hi - o.hi) + (lo - o.lo) <= 0.f; }
-  // this / o, rounded to FP32: an approximate quotient and the quotient of its exact
-  // residual (the division with IEEE rounding costs every warp some hundred clocks)
-  __device__ float over(const Scalar& o) const {
-    if (o.hi < 0x1p-120f || o.hi > 0x1p120f) return (float)(value() / o.value());
-    const float q = __fdividef(hi, o.hi);
-    if (!isfinite(q)) return q;
-    const float r = fmaf(-q, o.hi, hi) + fmaf(-q, o.lo, lo);
-    return q + __fdividef(r, o.hi);
-  }
-};
+// a thread's sum
+__device__ __forceinline__ Total<float> total_of(const DotAcc<float>& a) {
+  return Total<float>::of(a.hi, a.lo);
+}
 
 // ------------------------------------------------------------------ reductions
 // Sum of one value per thread of the CTA into out[k] (thread 0 writes): a fixed tree
@@ -176,22 +148,23 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[K], double* __res
   __syncthreads();
 }
 
-// The same for float pairs: warp k adds value k of all threads (a tree of pairs in every
+// The same for totals of FP32 vectors: warp k adds value k of all threads (a tree in every
 // warp would be several times the instructions).  Ends with a barrier.
 template <int K, int NT = DOT_THREADS>
-__device__ __forceinline__ void block_sum(Scalar<float> (&v)[K], Scalar<float>* __restrict__ out) {
-  __shared__ Scalar<float> part[K][NT];
+__device__ __forceinline__ void block_sum(const Total<float> (&v)[K],
+                                          Total<float>* __restrict__ out) {
+  __shared__ Total<float> part[K][NT];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < K; ++k) part[k][threadIdx.x] = v[k];
   __syncthreads();
   if (w < K) {
-    Scalar<float> t = part[w][lane];
+    Total<float> t = part[w][lane];
 #pragma unroll
     for (int j = 1; j < NT / 32; ++j) t.add(part[w][lane + 32 * j]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t.add(t.down(o));
-    if (lane == 0) out[w] = t;
+    if (lane == 0) t.store(out + w);
   }
   __syncthreads();
 }
