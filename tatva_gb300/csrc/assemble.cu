@@ -171,10 +171,7 @@ __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (
 #pragma unroll
   for (int m = 0; m < 8; ++m)
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      Y[m][i] = T(0);
-      if constexpr (NH_HVP) U[m][i] += X[m][i];  // modes of the deformed cell
-    }
+    for (int i = 0; i < V; ++i) Y[m][i] = T(0);
   // not unrolled: the four pairs differ in two signs, and one pair already holds a
   // Jacobian, a gradient and a flux per point
 #pragma unroll 1
@@ -192,10 +189,10 @@ __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (
       T J[3][3], R[3][3];  // 8 J and its inverse
       jx.at(up, J);
       if constexpr (NH_HVP) {
-        T j[3][3], D[3][3];
-        ju.at(up, j);
+        T Du[3][3], D[3][3];
+        ju.at(up, Du);
         jw.at(up, D);
-        nh_hvp_axes<T>(law.mu, law.lam, T(1.0 / 512), J, j, D, F[up]);
+        nh_hvp_axes<T>(law.mu, law.lam, T(1.0 / 512), J, Du, D, F[up]);
         continue;
       }
       const T wd = inv3(J, R) * T(1.0 / 512);
@@ -266,15 +263,15 @@ __device__ __forceinline__ void simplex_element(
     for (int d = 0; d < D; ++d) J[k][d] = X[k + 1][d] - X[0][d];
   T fsrc = T(0);
   if constexpr (MAT == TG_NEO_HOOKEAN && MODE == TG_MODE_HVP) {
-    T j[3][3], dw[3][3];
+    T du[3][3], dw[3][3];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        j[k][i] = J[k][i] + (U[k + 1][i] - U[0][i]);
+        du[k][i] = U[k + 1][i] - U[0][i];
         dw[k][i] = W[k + 1][i] - W[0][i];
       }
-    nh_hvp_axes<T>(law.mu, law.lam, E::template w<T>(0), J, j, dw, F);
+    nh_hvp_axes<T>(law.mu, law.lam, E::template w<T>(0), J, du, dw, F);
   } else {
     T R[D][D];
     const T wd = invD<T, D>(J, R) * E::template w<T>(0);

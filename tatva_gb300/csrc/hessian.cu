@@ -99,14 +99,17 @@ __device__ __forceinline__ void element_row_block(
     };
     T wd, c1;
     if constexpr (NH) {
-      T j[3][3], r[3][3], rdet;
+      T Du[3][3], j[3][3], r[3][3], rdet;
       wd = inv3(J, R, rdet) * E::template w<T>(0);
 #pragma unroll
       for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) j[k][d] = J[k][d] + (U[k + 1][d] - U[0][d]);
+        for (int d = 0; d < 3; ++d) {
+          Du[k][d] = U[k + 1][d] - U[0][d];
+          j[k][d] = J[k][d] + Du[k][d];
+        }
       const T dj = inv3(j, r);
-      c1 = wd * (mu - lam * log(dj * rdet));
+      c1 = wd * (mu - lam * log_volume_ratio(J, R, rdet, j, r, dj, Du));
       nodes_of(r, g);
     } else {
       wd = invD<T, D>(J, R) * E::template w<T>(0);
@@ -149,10 +152,6 @@ __device__ __forceinline__ void element_row_block(
     if constexpr (NH) {
       hex_modes8<T, 3>(U);
       hex_scale_gauss<T, 3>(U);
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) U[m][d] += X[m][d];  // modes of the deformed cell
     }
     const T sa[3] = {T(E::s(a, 0)), T(E::s(a, 1)), T(E::s(a, 2))};
 #pragma unroll 1
@@ -168,10 +167,15 @@ __device__ __forceinline__ void element_row_block(
       const T wd = inv3(J, R, rdet) * T(1.0 / 512);
       T c1 = wd * mu;
       if constexpr (NH) {
+        T Du[3][3], j[3][3];
         pr.set(U, sx, sy);
-        pr.at(up, J);
-        const T dj = inv3(J, r);
-        c1 = wd * (mu - lam * log(dj * rdet));
+        pr.at(up, Du);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int d = 0; d < 3; ++d) j[k][d] = J[k][d] + Du[k][d];
+        const T dj = inv3(j, r);
+        c1 = wd * (mu - lam * log_volume_ratio(J, R, rdet, j, r, dj, Du));
       }
       // f[l][side]: 1 + s x_l of the corners on that side along axis l
       const T f[3][2] = {{T(1) - sx * gp, T(1) + sx * gp},

@@ -13,6 +13,7 @@
 #pragma once
 
 #include "tg_common.cuh"
+#include "tg_volume.h"
 
 namespace tg {
 
@@ -181,23 +182,28 @@ struct Law<TG_NEO_HOOKEAN, 3, T> {
   __device__ T source() const { return T(0); }
 };
 
-// Neo-Hookean HVP at one point, in the element's own coordinates: J and j are the
-// Jacobians of the undeformed and the deformed cell, D of the direction (row k: derivative
-// along reference axis k), all with the same scale.  With the inverses R and r of J and j,
+// Neo-Hookean HVP at one point, in the element's own coordinates: J is the Jacobian of the
+// undeformed cell, Du and D those of the displacement and the direction (row k: derivative
+// along reference axis k), all with the same scale.  With the inverses R and r of J and of
+// the deformed cell's j = J + Du,
 // the spatial gradient of the direction g = dH F^-1 = sum_m D_m (x) r_m and the metric
 // C = R^T R of the undeformed axes,
 //   F_k = wd dP G_k = wd (mu sum_m C_mk D_m + c1 g^T r_k + lambda tr(g) r_k),
-//   c1 = mu - lambda ln(det j / det J),
+//   c1 = mu - lambda ln(det j / det J) (log_volume_ratio),
 // which is Lin::dflux above without forming F, its inverse or the 3 x 3 products with it.
 template <class T>
 __device__ __forceinline__ void nh_hvp_axes(T mu, T lam, T weight, const T (&J)[3][3],
-                                            const T (&j)[3][3], const T (&D)[3][3],
+                                            const T (&Du)[3][3], const T (&D)[3][3],
                                             T (&F)[3][3]) {
-  T R[3][3], r[3][3], rdet;
+  T R[3][3], r[3][3], j[3][3], rdet;
   const T det = inv3(J, R, rdet);
   const T wd = det * weight;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) j[k][d] = J[k][d] + Du[k][d];
   const T dj = inv3(j, r);
-  const T c1 = wd * (mu - lam * log(dj * rdet));
+  const T c1 = wd * (mu - lam * log_volume_ratio(J, R, rdet, j, r, dj, Du));
   const T m = wd * mu;
   T C[3][3], g[3][3];
 #pragma unroll
