@@ -66,6 +66,22 @@ __device__ __forceinline__ void load_run(const T* p, T (&v)[N]) {
   }
 }
 
+// Whether a value is infinite or NaN, on its bits (FP64: without the FP64 pipe).  The forms
+// that subtract a corner's value first turn one infinite nodal value into NaN all over its
+// element, and overflow from an eighth of the largest number on; an element with such a result
+// is done again as the weighted sum that defines it.
+__device__ __forceinline__ unsigned magnitude_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned magnitude_bits(double v) {
+  return (unsigned)__double2hiint(v) & 0x7fffffffu;
+}
+template <int N, class T>
+__device__ __forceinline__ bool any_nonfinite(const T (&v)[N]) {
+  unsigned m = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) m = max(m, magnitude_bits(v[k]));
+  return m >= (sizeof(T) == 4 ? 0x7f800000u : 0x7ff00000u);
+}
+
 // ------------------------------------------------------------------ eval
 template <int ET, class T>
 __global__ void eval_kernel(const T* __restrict__ nodal, int V, const int32_t* __restrict__ conn,
@@ -480,6 +496,29 @@ __device__ __forceinline__ void hex_scale_value(T (&m)[8][C]) {
   }
 }
 
+// the same sums as they are written: one element's components v0 .. v0 + nv - 1 of
+// sum_a N_a(xi_q) u[conn[e, a]] and of sum_q N_a(xi_q) quad[e, q]
+template <class T>
+__device__ __noinline__ void hex_eval_weighted(const T* __restrict__ nodal, int V, int v0, int nv,
+                                               const int32_t* __restrict__ conn, T* out) {
+  for (int q = 0; q < 8; ++q)
+    for (int k = 0; k < nv; ++k) {
+      T s = T(0);
+      for (int a = 0; a < 8; ++a)
+        s += Elem<TG_HEX8>::N<T>(q, a) * nodal[(int64_t)conn[a] * V + v0 + k];
+      out[q * V + k] = s;
+    }
+}
+template <class T>
+__device__ __noinline__ void hex_eval_transpose_weighted(const T* quad, int V, int nv, T* out) {
+  for (int a = 0; a < 8; ++a)
+    for (int k = 0; k < nv; ++k) {
+      T s = T(0);
+      for (int q = 0; q < 8; ++q) s += Elem<TG_HEX8>::N<T>(q, a) * quad[q * V + k];
+      out[a * V + k] = s;
+    }
+}
+
 // out[e, q, v] = sum_a N_a(xi_q) u[conn[e, a], v]
 template <class T, int NV, bool VEC>
 __global__ void __launch_bounds__(128)
@@ -507,6 +546,10 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int k = 0; k < G; ++k) o[q * G + k] = m[q][k] + base[k];
     T* dst = out + e * 8 * V + v0;
+    if (any_nonfinite(o)) {
+      hex_eval_weighted(nodal, V, v0, nv, conn + e * 8, dst);
+      continue;
+    }
     if constexpr (NV) {
       store_run<VEC>(dst, o);
     } else {
@@ -551,18 +594,22 @@ __global__ void __launch_bounds__(128)
     hex_scale_value<T, G>(m);
     hex_modes8_adjoint<T, G>(m);
     T* dst = contrib + e * 8 * V + v0;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int k = 0; k < G; ++k) f[a * G + k] = m[a][k];
+    if (any_nonfinite(f)) {
+      hex_eval_transpose_weighted(src, V, nv, dst);
+      continue;
+    }
     if constexpr (NV) {
-#pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int k = 0; k < G; ++k) f[a * G + k] = m[a][k];
       store_run<VEC>(dst, f);
     } else {
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
         for (int k = 0; k < G; ++k)
-          if (k < nv) dst[a * V + k] = m[a][k];
+          if (k < nv) dst[a * V + k] = f[a * G + k];
     }
   }
 }
