@@ -157,7 +157,8 @@ __device__ __forceinline__ void warp_load_runs(const T* __restrict__ src, T* til
 // Tri3 / Tet4: thread per element through the edge vectors from node 0 (gradient = R D f,
 // D_k f = f_{k+1} - f_0, R the inverse of the coordinates' D).  NV = V in {1, 2, 3}; NV = 0:
 // any V, a component at a time.  FP64 is bound by the FP64 pipe (about 95 operations for
-// V = 3), FP32 by memory.
+// V = 3), FP32 by memory.  A result that is not finite is done again as the sum over the nodes
+// (sum_a G_a f_a, with G_0 = -sum_k R_k): in the differences an infinite f_0 is in every term.
 template <int ET, class T>
 __device__ __forceinline__ void simplex_inverse(const T* __restrict__ coords,
                                                 const int32_t* __restrict__ conn, int64_t e,
@@ -171,6 +172,50 @@ __device__ __forceinline__ void simplex_inverse(const T* __restrict__ coords,
 #pragma unroll
     for (int d = 0; d < D; ++d) J[k][d] = X[k + 1][d] - X[0][d];
   invD<T, D>(J, R);
+}
+
+// the sums over the nodes, for one component (not inlined: the compiler would run them for
+// every element, FP64 Tri3 46 -> 74 us): its gradient, or node 0's share of a flux f
+template <class T, int D>
+struct SimplexVec {
+  T v[D];
+};
+template <int ET, class T>
+__device__ __noinline__ SimplexVec<T, Elem<ET>::D> simplex_grad_nodal(
+    const T* __restrict__ nodal, const T* __restrict__ coords, int V, int v,
+    const int32_t* __restrict__ conn, int64_t e) {
+  constexpr int D = Elem<ET>::D;
+  int nid[Elem<ET>::NN];
+  T R[D][D];
+  simplex_inverse<ET, T>(coords, conn, e, nid, R);
+  SimplexVec<T, D> g;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    T g0 = T(0);
+#pragma unroll
+    for (int k = 0; k < D; ++k) g0 -= R[d][k];
+    g.v[d] = g0 * nodal[(int64_t)nid[0] * V + v];
+#pragma unroll
+    for (int k = 0; k < D; ++k) g.v[d] += R[d][k] * nodal[(int64_t)nid[k + 1] * V + v];
+  }
+  return g;
+}
+template <int ET, class T>
+__device__ __noinline__ T simplex_node0_share(const T* __restrict__ flux,
+                                              const T* __restrict__ coords,
+                                              const int32_t* __restrict__ conn, int64_t e) {
+  constexpr int D = Elem<ET>::D;
+  int nid[Elem<ET>::NN];
+  T R[D][D], s = T(0);
+  simplex_inverse<ET, T>(coords, conn, e, nid, R);
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    T g0 = T(0);
+#pragma unroll
+    for (int k = 0; k < D; ++k) g0 -= R[d][k];
+    s += g0 * flux[d];
+  }
+  return s;
 }
 
 template <int ET, class T, int NV>
@@ -196,6 +241,11 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
       const T f = nodal[(int64_t)nid[k + 1] * V + v] - f0;
 #pragma unroll
       for (int d = 0; d < D; ++d) g[d] = k == 0 ? R[d][0] * f : fma(R[d][k], f, g[d]);
+    }
+    if (any_nonfinite(g)) {
+      const auto t = simplex_grad_nodal<ET, T>(nodal, coords, V, v, conn, ec);
+#pragma unroll
+      for (int d = 0; d < D; ++d) g[d] = t.v[d];
     }
 #pragma unroll
     for (int d = 0; d < D; ++d) o[d] = g[d];
@@ -741,7 +791,7 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
   int nid[NN];
   T R[D][D];
   simplex_inverse<ET, T>(coords, conn, ec, nid, R);
-  auto contribution = [&](const T* f, T (&c)[NN]) {
+  auto contribution = [&](const T* f, T (&c)[NN], int v) {
     T s = T(0);
 #pragma unroll
     for (int k = 0; k < D; ++k) {
@@ -752,6 +802,8 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
       s += t;
     }
     c[0] = -s;
+    if (any_nonfinite(c))  // infinities of both signs may have met in s
+      c[0] = simplex_node0_share<ET, T>(flux + (ec * V + v) * D, coords, conn, ec);
   };
   if constexpr (NV) {
     const int n_here = (int)(n_elems - e0 < 32 ? n_elems - e0 : 32);
@@ -761,7 +813,7 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       T c[NN];
-      contribution(f + v * D, c);
+      contribution(f + v * D, c, v);
 #pragma unroll
       for (int a = 0; a < NN; ++a) o[a * NV + v] = c[a];
     }
@@ -770,7 +822,7 @@ __global__ void __launch_bounds__(SIMPLEX_THREADS)
     if (e < n_elems)
       for (int v = 0; v < V; ++v) {
         T c[NN];
-        contribution(flux + (e * V + v) * D, c);
+        contribution(flux + (e * V + v) * D, c, v);
 #pragma unroll
         for (int a = 0; a < NN; ++a) contrib[(e * NN + a) * V + v] = c[a];
       }

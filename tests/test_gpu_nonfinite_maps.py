@@ -92,3 +92,52 @@ def test_hex_eval_transpose_of_infinite_and_nan_points(cuda, vals, dtype):
     np.add.at(want, e.ravel(), np.einsum("qa,eqv->eav", _weights(), flat).reshape(e.size, -1))
     _same_kinds(du, want.reshape(du.shape))
     assert np.isinf(want).any() and np.isnan(want).any()
+
+
+def _simplex(cuda, elem):
+    """A mesh whose shape gradients have no zero component, and G (e, a, d)."""
+    rng = np.random.default_rng(3)
+    c, e = om.unit_square(4, 3) if elem == "tri3" else om.kuhn_box((1, 1, 1), (3, 2, 2))
+    c = np.asarray(c, float) + 0.08 * rng.uniform(-1, 1, np.shape(c))
+    d = c.shape[1]
+    X = c[e]
+    R = np.linalg.inv(X[:, 1:] - X[:, :1])  # (e, d, k)
+    G = np.concatenate([-R.sum(2)[:, None], R.transpose(0, 2, 1)], 1)
+    assert np.abs(G).min() > 1e-4  # far above FP32's rounding of G: every sign is certain
+    cls = element.Tri3 if elem == "tri3" else element.Tetrahedron4
+    return Operator(Mesh(c, e, device=cuda), cls()), c, e, G, d
+
+
+@pytest.mark.parametrize("elem", ["tri3", "tet4"])
+@pytest.mark.parametrize("vals", [0, 3, 5])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_simplex_grad_of_infinite_and_nan_nodes(cuda, elem, vals, dtype):
+    op, c, e, G, d = _simplex(cuda, elem)
+    for corner in range(e.shape[1]):
+        u = np.random.default_rng(4).standard_normal((c.shape[0],) + _shape(vals))
+        flat = u.reshape(c.shape[0], -1)
+        flat[e[4, corner], 0], flat[e[-1, corner], -1] = np.inf, -np.inf
+        flat[e[9, corner], 0] = np.nan
+        with np.errstate(invalid="ignore"):
+            want = (flat[e][:, :, :, None] * G[:, :, None, :]).sum(1)  # (e, v, d)
+        _same_kinds(op.grad(torch.as_tensor(u, dtype=dtype, device=cuda)),
+                    want.reshape((e.shape[0], 1) + _shape(vals) + (d,)))
+        assert np.isinf(want).any() and np.isnan(want).any()
+
+
+@pytest.mark.parametrize("elem", ["tri3", "tet4"])
+@pytest.mark.parametrize("vals", [0, 3, 5])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_simplex_grad_transpose_of_infinite_and_nan_points(cuda, elem, vals, dtype):
+    op, c, e, G, d = _simplex(cuda, elem)
+    f = np.random.default_rng(5).standard_normal((e.shape[0], 1) + _shape(vals) + (d,))
+    flat = f.reshape(e.shape[0], -1, d)
+    flat[3, 0, 0], flat[-2, -1, 1], flat[10, 0, 0] = np.inf, -np.inf, np.nan
+    u = torch.zeros((c.shape[0],) + _shape(vals), dtype=dtype, device=cuda, requires_grad=True)
+    (du,) = torch.autograd.grad(op.grad(u), u, torch.as_tensor(f, dtype=dtype, device=cuda))
+    with np.errstate(invalid="ignore"):
+        per = (flat[:, None] * G[:, :, None, :]).sum(-1)  # (e, a, v)
+        want = np.zeros((c.shape[0], flat.shape[1]))
+        np.add.at(want, e.ravel(), per.reshape(e.size, -1))
+    _same_kinds(du, want.reshape(du.shape))
+    assert np.isinf(want).any() and np.isnan(want).any()
