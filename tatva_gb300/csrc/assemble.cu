@@ -1136,6 +1136,44 @@ __global__ void __launch_bounds__(APPLY_MAX_THREADS)
 }
 
 // ------------------------------------------------------------------ energy per element
+// A Hex8 element's energy from the sums over its nodes, for one whose modal form gave no finite
+// number: an infinite displacement is in every mode there (NaN), here it gives the infinity.
+template <int MAT, class T>
+__device__ __noinline__ T hex_energy_nodal(const T* __restrict__ coords,
+                                           const int32_t* __restrict__ conn,
+                                           const T* __restrict__ u, Law<MAT, 3, T> law) {
+  using E = Elem<TG_HEX8>;
+  constexpr int V = LawDims<MAT, 3>::V;
+  T acc = T(0);
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q) {
+    T J[3][3] = {}, R[3][3], H[V][3] = {}, uq = T(0);
+#pragma unroll 1
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          J[i][d] += E::template dN<T>(q, i, a) * coords[(int64_t)conn[a] * 3 + d];
+    const T wd = inv3(J, R) * E::template w<T>(q);
+#pragma unroll 1
+    for (int a = 0; a < 8; ++a) {
+      const T* ua = u + (int64_t)conn[a] * V;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        T g = T(0);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) g += R[d][i] * E::template dN<T>(q, i, a);
+#pragma unroll
+        for (int i = 0; i < V; ++i) H[i][d] += g * ua[i];
+      }
+      uq += E::template N<T>(q, a) * ua[0];
+    }
+    acc += wd * law.energy(H, uq);
+  }
+  return acc;
+}
+
 template <int ET, int MAT, class T>
 __global__ void energy_kernel(const T* __restrict__ coords, const int32_t* __restrict__ conn,
                               int64_t n_elems, const T* __restrict__ u, T p0, T p1,
@@ -1190,6 +1228,7 @@ __global__ void energy_kernel(const T* __restrict__ coords, const int32_t* __res
         acc += wd * law.energy(H, uq);
       }
     }
+    if (!isfinite(acc)) acc = hex_energy_nodal<MAT, T>(coords, conn + e * 8, u, law);
   } else {
 #pragma unroll
     for (int q = 0; q < E::Q; ++q) {
