@@ -447,14 +447,19 @@ TG_API int tg_operator_apply(const tg_operator_desc* op, const void* x, void* y,
 /* Jacobi-preconditioned CG, all vectors of precision op->prec, scalars and dot
  * products on the device to FP64's precision or better (FP32: exact products, pairs
  * of floats over the few dozen entries of a thread, whose sum has to stay in FP32's
- * range, then FP64, or three floats on a brick that runs as one launch).  Solves A x = b from the given x.  The loop runs
- * `check_every` iterations per CUDA graph replay between host convergence checks
- * and never exceeds max_iter; the stopping test itself runs on the device after
- * every iteration, so the result does not depend on check_every.  On a structured
- * brick with a Dirichlet mask, x is set to b on the fixed dofs first (the identity
- * rows of the masked system).  b and x must be 16-byte aligned (vector loads and
- * stores), else TG_ERR_VALUE.                                                  */
+ * range, then FP64, or three floats on a brick that runs as one launch).  Solves
+ * A x = b from the given x.  The loop runs tg_cg_check_interval iterations -- one
+ * CUDA graph replay or one cooperative launch -- between host convergence checks and
+ * never exceeds max_iter; the stopping test itself runs on the device after every
+ * iteration, so the result does not depend on check_every.  On a structured brick
+ * with a Dirichlet mask, x is set to b on the fixed dofs first (the identity rows of
+ * the masked system).  b and x must be 16-byte aligned (vector loads and stores),
+ * else TG_ERR_VALUE.                                                           */
 TG_API size_t tg_cg_workspace_bytes(const tg_operator_desc* op);
+/* HOST: CG iterations between two host checks with this operator: check_every (at
+ * least 1), or, where they run as one cooperative launch (linear elasticity on a
+ * structured brick of up to 3.5 M unknowns), 16 check_every, at most 65,536.     */
+TG_API int tg_cg_check_interval(const tg_operator_desc* op, int check_every);
 TG_API int tg_cg_solve(const tg_operator_desc* op, const void* b, void* x, const void* diag,
                 double rtol, int max_iter, int check_every, void* workspace,
                 size_t workspace_bytes, tg_solve_stats* stats, void* stream);

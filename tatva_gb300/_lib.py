@@ -218,6 +218,7 @@ SIGNATURES = {
     "tg_axpby": (I, [I, L, D, P, D, P, P]),
     "tg_convert": (I, [I, P, I, P, L, P]),
     "tg_cg_workspace_bytes": (S, [P]),
+    "tg_cg_check_interval": (I, [P, I]),
     "tg_cg_solve": (I, [P, P, P, P, D, I, I, P, S, P, P]),
     "tg_mixed_workspace_bytes": (S, [P, P]),
     "tg_mixed_solve": (I, [P, P, P, P, P, D, D, I, I, I, P, S, P, P]),

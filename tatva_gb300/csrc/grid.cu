@@ -224,6 +224,8 @@ __device__ __forceinline__ T total_scale(double v) {
   return sizeof(T) == 4 && v > 0x1p60 ? T(0x1p-18) : T(1);
 }
 static_assert(CG_MAX_CTAS * cg_threads<float>() <= 1 << 18, "what total_scale allows for");
+static_assert((int64_t)4 * CG_MAX_CTAS * GRID_CG_MAX_ITERS < (int64_t)1 << 31,
+              "a launch's arrivals fit the barrier's counter");
 
 // A thread's sum as it is handed to the warp that adds them up: a float pair or a double.
 template <class T>

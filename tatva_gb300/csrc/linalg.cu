@@ -712,6 +712,15 @@ static bool grid_op(const tg_operator_desc* op) {
          grid_cg_ctas(op->plan) > 0;
 }
 
+// CG iterations between two reads of the scalars by the host.  A persistent launch ends by
+// itself when the solve has: 16 blocks in one, fewer reads (30 us each with the launch; 50
+// iterations take 600 at 16^3).
+static int cg_block(bool persistent, int check_every) {
+  const int64_t every = check_every < 1 ? 1 : check_every;
+  if (!persistent) return (int)every;
+  return (int)(16 * every < GRID_CG_MAX_ITERS ? 16 * every : GRID_CG_MAX_ITERS);
+}
+
 static int64_t cg_part_doubles(const tg_operator_desc* op) {
   const int64_t g = grid_op(op) ? grid_cg_ctas(op->plan) : 0;
   return g > 2 * DOT_CHUNKS ? g : 2 * DOT_CHUNKS;
@@ -827,10 +836,8 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
   int rc = TG_OK;
   bool done = false;
   while (*iters < max_iter) {
-    // a persistent launch ends by itself when the solve has: 16 blocks in one, fewer reads
-    // of the scalars by the host (30 us each with the launch; 50 iterations take 600 at 16^3)
-    const int64_t block = (B.persistent ? 16 : 1) * (int64_t)check_every;
-    const int k = (max_iter - *iters) < block ? (max_iter - *iters) : (int)block;
+    const int block = cg_block(B.persistent, check_every);
+    const int k = max_iter - *iters < block ? max_iter - *iters : block;
     const int before = *iters;
     if (B.persistent) {
       rc = launch_grid_cg(op->plan, op->prec, op->mat.p0, op->mat.p1, B.nmask, x, B.r, B.p, B.q,
@@ -907,6 +914,10 @@ static int true_residual_norm(const tg_operator_desc* op, const T* bvec, const T
 }
 
 }  // namespace tg
+
+extern "C" int tg_cg_check_interval(const tg_operator_desc* op, int check_every) {
+  return cg_block(op && grid_op(op) && grid_cg_persistent(op->plan), check_every);
+}
 
 extern "C" size_t tg_cg_workspace_bytes(const tg_operator_desc* op) {
   return op ? cg_bytes(op) : 0;

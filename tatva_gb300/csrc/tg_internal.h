@@ -30,9 +30,12 @@ int64_t grid_cg_ctas(const tg_block_plan* plan);
 int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double lam,
                         const void* p, const uint8_t* node_mask, void* q, double* scal,
                         double* part, unsigned* ticket, cudaStream_t st);
-// Whether blocks of CG iterations on the plan's grid run as one launch (launch_grid_cg).
+// Whether blocks of CG iterations on the plan's grid run as one launch (launch_grid_cg), of at
+// most GRID_CG_MAX_ITERS: its barriers count their arrivals, four a CTA and iteration, in 32
+// bits.  (Results do not depend on where a solve is cut into launches.)
 bool grid_cg_persistent(const tg_block_plan* plan);
-// `iters` CG iterations (fewer when they converge or break down) from the residual r, the
+constexpr int GRID_CG_MAX_ITERS = 1 << 16;
+// `iters` <= GRID_CG_MAX_ITERS CG iterations (fewer when they converge or break down) from the residual r, the
 // direction p and the scalars scal (SCAL_*) on a structured brick, as one cooperative
 // launch; part: 2 DOT_CHUNKS doubles, count: one counter.  node_mask: NULL, or one byte per
 // node, bit d set when dof 3 n + d is fixed (pack_node_mask from the C ABI's per-dof mask);

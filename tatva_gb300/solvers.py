@@ -15,7 +15,8 @@ These wrappers drive the native solvers of the C ABI:
 
 All scalars stay on the GPU; the host reads one small vector every
 ``check_every`` iterations, which run as one captured CUDA graph (CG on a structured
-brick of up to 3.5 M unknowns: as one cooperative launch).
+brick of up to 3.5 M unknowns: every 16 ``check_every``, at most 65,536, which run as
+one cooperative launch).
 """
 
 from __future__ import annotations
