@@ -145,6 +145,9 @@ TG_API int tg_eval_transpose_ws(int elem, int prec, const void* quad, int64_t n_
  * stages its nodes in shared memory, accumulates element results in block-local
  * element-colour order, writes nodes it owns alone and leaves partial sums for
  * nodes shared with other blocks, which a second pass adds in fixed order.   */
+/* grid_flags of a plan: the CG's iterations as separate launches (captured in a graph)
+ * where they would run as one cooperative launch */
+#define TG_GRID_SEPARATE_LAUNCHES 1
 typedef struct tg_block_plan {
   int32_t n_blocks;
   int32_t n_elems;
@@ -186,7 +189,7 @@ typedef struct tg_block_plan {
    * in the reference corner order.  Linear-elastic residual / HVP then run as a
    * stencil over the grid (no element data read).  grid_nodes[0] = 0: not a brick. */
   int32_t grid_nodes[3];
-  int32_t grid_reserved;
+  int32_t grid_flags; /* TG_GRID_* */
   double grid_h[3];
 } tg_block_plan;
 
@@ -407,7 +410,8 @@ typedef struct tg_solve_stats {
   int32_t status;       /* TG_OK / TG_ERR_NOT_CONVERGED / TG_ERR_BREAKDOWN */
   int32_t iterations;   /* total (inner) CG iterations                      */
   int32_t outer;        /* refinement steps (mixed solve)                   */
-  int32_t reserved;
+  int32_t checks;       /* host checks in CG loops: cooperative launches, or
+                           graph replays (groups of launches)               */
   double rel_res;       /* final FP64 true relative residual ||b-Ax||/||b|| */
 } tg_solve_stats;
 

@@ -67,9 +67,12 @@ class BlockPlan(ctypes.Structure):
         ("n_lattice_blocks", c_int32),
         ("reserved0", c_int32),
         ("grid_nodes", c_int32 * 3),
-        ("grid_reserved", c_int32),
+        ("grid_flags", c_int32),
         ("grid_h", c_double * 3),
     ]
+
+
+TG_GRID_SEPARATE_LAUNCHES = 1
 
 
 class Material(ctypes.Structure):
@@ -89,7 +92,7 @@ class SolveStats(ctypes.Structure):
         ("status", c_int32),
         ("iterations", c_int32),
         ("outer", c_int32),
-        ("reserved", c_int32),
+        ("checks", c_int32),
         ("rel_res", c_double),
     ]
 

@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
 
 bool grid_cg_persistent(const tg_block_plan* plan) {
   const int64_t n = 3 * (int64_t)plan->grid_nodes[0] * plan->grid_nodes[1] * plan->grid_nodes[2];
-  return n <= GRID_CG_MAX_DOFS;
+  return n <= GRID_CG_MAX_DOFS && !(plan->grid_flags & TG_GRID_SEPARATE_LAUNCHES);
 }
 
 int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,

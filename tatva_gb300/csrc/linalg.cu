@@ -687,6 +687,7 @@ struct CgBuffers {
   // caller destroys it with cg_release)
   cudaGraphExec_t exec = nullptr;
   int graph_len = 0;
+  int checks = 0;  // launches or replays so far, each followed by a read of the scalars
 };
 
 static void cg_release(CgBuffers& B) {
@@ -836,6 +837,7 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
   int rc = TG_OK;
   bool done = false;
   while (*iters < max_iter) {
+    ++B.checks;
     const int block = cg_block(B.persistent, check_every);
     const int k = max_iter - *iters < block ? max_iter - *iters : block;
     const int before = *iters;
@@ -845,6 +847,7 @@ static int cg_run(const tg_operator_desc* op, const T* bvec, T* x, const T* diag
       if (rc == TG_ERR_UNSUPPORTED) {
         B.persistent = false;
         rc = TG_OK;
+        --B.checks;
         continue;
       }
       if (rc != TG_OK) break;
@@ -955,6 +958,7 @@ extern "C" int tg_cg_solve(const tg_operator_desc* op, const void* b, void* x, c
     if (stats) {
       stats->iterations = total;
       stats->outer = 0;
+      stats->checks = B.checks;
       stats->rel_res = bn > 0 ? rn / bn : rn;
     }
     if (rc == TG_OK && rn > tol) rc = set_error(TG_ERR_NOT_CONVERGED, "tg_cg_solve: not converged");
@@ -1071,6 +1075,7 @@ extern "C" int tg_mixed_solve(const tg_operator_desc* op64, const tg_operator_de
     stats->status = rc;
     stats->iterations = total_inner;
     stats->outer = outer;
+    stats->checks = B.checks;
     stats->rel_res = bn > 0 ? rn / bn : rn;
   }
   return rc;

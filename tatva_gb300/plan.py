@@ -150,6 +150,16 @@ class BlockPlan:
         mode) or back on, when the mesh is a brick."""
         self.struct.grid_nodes[:] = self.grid_nodes if on else (0, 0, 0)
 
+    @property
+    def persistent_cg(self) -> bool:
+        """True where the CG's iterations on the brick run as one cooperative launch (bricks
+        of up to 3.5 M unknowns, ``tg_cg_check_interval``), False: as separate launches."""
+        return not self.struct.grid_flags & _lib.TG_GRID_SEPARATE_LAUNCHES
+
+    @persistent_cg.setter
+    def persistent_cg(self, on: bool) -> None:
+        self.struct.grid_flags = 0 if on else _lib.TG_GRID_SEPARATE_LAUNCHES
+
     def stats(self) -> dict:
         s = dict(self.sizes)
         s.update(block_elems=self.block_elems, threads=self.threads, grid=self.grid,

@@ -43,6 +43,7 @@ class SolveResult:
     seconds: float
     history: list = field(default_factory=list)
     message: str = ""
+    checks: int = 0  # host checks in CG loops (``tg_solve_stats``)
 
     @property
     def converged(self) -> bool:
@@ -102,7 +103,8 @@ def cg(energy, b: torch.Tensor, x0: torch.Tensor | None = None, *, u=None, fixed
 
     stats, rc, dt, msg = _run(go, b.device, raise_on_fail)
     del keep
-    return SolveResult(x.view(b.shape), stats.iterations, 0, stats.rel_res, rc, dt, message=msg)
+    return SolveResult(x.view(b.shape), stats.iterations, 0, stats.rel_res, rc, dt, message=msg,
+                       checks=stats.checks)
 
 
 def mixed_cg(energy, b: torch.Tensor, x0: torch.Tensor | None = None, *, u=None, fixed=None,
@@ -135,7 +137,7 @@ def mixed_cg(energy, b: torch.Tensor, x0: torch.Tensor | None = None, *, u=None,
     stats, rc, dt, msg = _run(go, b.device, raise_on_fail)
     del k64, k32
     return SolveResult(x.view(b.shape), stats.iterations, stats.outer, stats.rel_res, rc, dt,
-                       message=msg)
+                       message=msg, checks=stats.checks)
 
 
 # id of a pattern's indices tensor -> (weak reference to it, node blocks or None)
@@ -203,7 +205,8 @@ def csr_cg(cm, b: torch.Tensor, x0=None, *, fixed=None, rtol: float = 1e-8,
                                       int(maxiter), int(check_every), ptr(ws), nb, stats, st)
 
     stats, rc, dt, msg = _run(go, b.device, raise_on_fail)
-    return SolveResult(x.view(b.shape), stats.iterations, 0, stats.rel_res, rc, dt, message=msg)
+    return SolveResult(x.view(b.shape), stats.iterations, 0, stats.rel_res, rc, dt, message=msg,
+                       checks=stats.checks)
 
 
 def newton(energy, u0: torch.Tensor, lifter, *, colored_matrix=None, rtol: float = 1e-10,
