@@ -40,6 +40,7 @@ Multi-GPU: replicas only (each rank runs the same workload on its own GPU).
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import subprocess
@@ -383,7 +384,7 @@ def _hvp_timing(en, v, y, flush, steps, warmup, dev):
 def run_ours(args):
     import torch
 
-    from tatva_gb300 import autotune, replicas, solvers
+    from tatva_gb300 import _lib, autotune, replicas, solvers
     from tatva_gb300.problems import clamped_brick
 
     ws, rank, local = replicas.world()
@@ -445,19 +446,20 @@ def run_ours(args):
     inner = results[-1].iterations
     outer = results[-1].outer
     # launches per mixed solve: per inner iteration 3 kernels on a structured brick (the
-    # HVP with p.q, the update, the direction; one per block of check_every iterations up
-    # to 3.5 M unknowns), else the HVP plus 3 CG kernels; per
-    # refinement the FP64 HVP, 3 residual/norm kernels, the scale-down, the inner
-    # residual (HVP + 2 kernels, + 2 for the packed Dirichlet mask on a brick), the
-    # direction (2 kernels at a restart, 3 at a reliable update) and the update; 3
-    # set-up kernels, and the Jacobi diagonal
+    # HVP with p.q, the update, the direction; up to 3.5 M unknowns one cooperative launch
+    # per host check), else the HVP plus 3 CG kernels; per refinement the FP64 HVP, 3
+    # residual/norm kernels, the scale-down, the inner residual (HVP + 2 kernels, + 2 for
+    # the packed Dirichlet mask on a brick), the direction (2 kernels at a restart, 3 at a
+    # reliable update) and the update; 3 set-up kernels, and the Jacobi diagonal
     per_inner = 3 if plan.grid else hvp_launches + 3
     resumes = max(outer - 1, 0) if args.inner_rtol >= 0.01 else 0
-    launches_per_solve = (inner * per_inner + (outer + 1) * (hvp_launches + 3)
+    desc, _keep = en.operator_desc(None, fixed, torch.float32)
+    interval = _lib.lib().tg_cg_check_interval(ctypes.byref(desc), args.check_every)
+    inner_launches = (results[-1].checks if interval > args.check_every
+                      else inner * per_inner)
+    launches_per_solve = (inner_launches + (outer + 1) * (hvp_launches + 3)
                           + outer * (hvp_launches + 6 + (2 if plan.grid else 0)) + resumes
                           + 3 + hvp_launches)
-    if plan.grid and ndof <= 3_500_000:
-        launches_per_solve += inner // args.check_every + outer - inner * per_inner
 
     # ---- e2e through the public API: each step's own right-hand side (the traction
     # scaled per step) from pinned host memory, its solution back to pinned host memory

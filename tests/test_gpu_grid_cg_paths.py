@@ -77,6 +77,17 @@ def test_blocks_checks_and_bits(cuda, dtype, persistent):
 
 
 @PATHS
+def test_checks_of_a_mixed_solve(cuda, persistent):
+    """k iterations of an inner solve take ceil(k / interval) checks."""
+    en, b, fixed = _problem((20, 17, 19), cuda)
+    en.plan().persistent_cg = persistent
+    m = solvers.mixed_cg(en, b, fixed=fixed, rtol=1e-10, check_every=20)
+    interval = 16 * 20 if persistent else 20
+    assert max(m.outer, m.iterations / interval) <= m.checks
+    assert m.checks <= m.outer + m.iterations // interval
+
+
+@PATHS
 def test_prescribed_values(cuda, persistent):
     """b nonzero on fixed dofs: x = b there exactly, the rest as the element-block CG's."""
     en, b, fixed = _problem((14, 9, 11), cuda)
