@@ -49,12 +49,13 @@ struct Supported {
   static constexpr bool value = !(MAT == TG_NEO_HOOKEAN && Elem<ET>::D != 3);
 };
 
-// ------------------------------------------------------------------ generic per-QP element
-template <int ET, int MAT, class T, int MODE>
-__device__ __forceinline__ void element_generic(
+// ------------------------------------------------------------------ diagonal
+// Y = the diagonal of an element's tangent, from the shape gradients at every point
+// (residual and HVP: hex_element_modal, simplex_element)
+template <int ET, int MAT, class T>
+__device__ __forceinline__ void element_diagonal(
     const Law<MAT, Elem<ET>::D, T>& law, const T (&X)[Elem<ET>::NN][Elem<ET>::D],
     const T (&U)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
-    const T (&W)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V],
     T (&Y)[Elem<ET>::NN][LawDims<MAT, Elem<ET>::D>::V]) {
   using E = Elem<ET>;
   using L = Law<MAT, E::D, T>;
@@ -71,7 +72,7 @@ __device__ __forceinline__ void element_generic(
     T G[NN][D];
     const T wd = qp_geometry<ET, T>(q, X, G) * E::template w<T>(q);
     T H[V][D];
-    if constexpr (MODE == TG_MODE_RESIDUAL || !L::LINEAR) {
+    if constexpr (!L::LINEAR) {
 #pragma unroll
       for (int i = 0; i < V; ++i)
 #pragma unroll
@@ -82,63 +83,22 @@ __device__ __forceinline__ void element_generic(
           H[i][d] = s;
         }
     }
-    if constexpr (MODE == TG_MODE_RESIDUAL) {
-      T P[V][D];
-      law.flux(H, P);
+    const auto lin = law.linearize(H);
 #pragma unroll
-      for (int a = 0; a < NN; ++a)
+    for (int a = 0; a < NN; ++a)
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-          T s = T(0);
+      for (int i = 0; i < V; ++i) {
+        T dH[V][D], dP[V][D];
 #pragma unroll
-          for (int d = 0; d < D; ++d) s += P[i][d] * G[a][d];
-          Y[a][i] += wd * s;
-        }
-      if constexpr (MAT == TG_POISSON) {
-        const T f = law.source();
+        for (int k = 0; k < V; ++k)
 #pragma unroll
-        for (int a = 0; a < NN; ++a) Y[a][0] -= wd * f * E::template N<T>(q, a);
+          for (int d = 0; d < D; ++d) dH[k][d] = (k == i) ? G[a][d] : T(0);
+        lin.dflux(dH, dP);
+        T s = T(0);
+#pragma unroll
+        for (int d = 0; d < D; ++d) s += dP[i][d] * G[a][d];
+        Y[a][i] += wd * s;
       }
-    } else if constexpr (MODE == TG_MODE_HVP) {
-      const auto lin = law.linearize(H);
-      T dH[V][D], dP[V][D];
-#pragma unroll
-      for (int i = 0; i < V; ++i)
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          T s = T(0);
-#pragma unroll
-          for (int a = 0; a < NN; ++a) s += G[a][d] * W[a][i];
-          dH[i][d] = s;
-        }
-      lin.dflux(dH, dP);
-#pragma unroll
-      for (int a = 0; a < NN; ++a)
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          T s = T(0);
-#pragma unroll
-          for (int d = 0; d < D; ++d) s += dP[i][d] * G[a][d];
-          Y[a][i] += wd * s;
-        }
-    } else {  // diagonal of the element tangent
-      const auto lin = law.linearize(H);
-#pragma unroll
-      for (int a = 0; a < NN; ++a)
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          T dH[V][D], dP[V][D];
-#pragma unroll
-          for (int k = 0; k < V; ++k)
-#pragma unroll
-            for (int d = 0; d < D; ++d) dH[k][d] = (k == i) ? G[a][d] : T(0);
-          lin.dflux(dH, dP);
-          T s = T(0);
-#pragma unroll
-          for (int d = 0; d < D; ++d) s += dP[i][d] * G[a][d];
-          Y[a][i] += wd * s;
-        }
-    }
   }
 }
 
@@ -146,8 +106,8 @@ __device__ __forceinline__ void element_generic(
 // Residual or HVP of a general (trilinear) Hex8 element in the modal form of tg_hex.cuh,
 // one z pair of Gauss points per trip.  The element arithmetic bounds these kernels (the
 // issue slots in FP32, the FP64 pipe in FP64).  Against nodal sums at every point, which
-// this replaces, on jittered bricks: linear-elastic FP32 HVP of 872,640 elements 142 ->
-// 94 us, Neo-Hookean FP64 energy and residual of 84,480 elements 1522 -> 1016 us; FP32
+// this replaces, on jittered bricks: linear-elastic FP32 HVP of 872,640 elements (the call)
+// 155 -> 106 us, Neo-Hookean FP64 energy and residual of 84,480 elements 1522 -> 1016 us; FP32
 // error against FP64 2.1e-6 -> 1.5e-6 (differences to corner 0).
 template <int MAT, class T, int MODE>
 __device__ __forceinline__ void hex_element_modal(const Law<MAT, 3, T>& law, T (&X)[8][3],
@@ -331,7 +291,9 @@ __device__ __forceinline__ void simplex_element(
 
 // ------------------------------------------------------------------ Hex8 affine modal path
 // node a <-> tensor index t = bx + 2 by + 4 bz (bits of the reference coordinates)
-__host__ __device__ constexpr int hex_t(int a) { return (a == 2) ? 3 : (a == 3) ? 2 : (a == 6) ? 7 : (a == 7) ? 6 : a; }
+__host__ __device__ constexpr int hex_t(int a) {
+  return (a == 2) ? 3 : (a == 3) ? 2 : (a == 6) ? 7 : (a == 7) ? 6 : a;
+}
 
 // in place: m[S] = sum_t v_t prod_{i in S} s_i(t), S = bit set over (x, y, z)
 template <class T>
@@ -714,12 +676,12 @@ __device__ __forceinline__ void element_apply(
     }
   } else {
     const Law<MAT, E::D, T> law(p0, p1);
-    if constexpr (ET == TG_HEX8 && MODE != TG_MODE_DIAG)
+    if constexpr (MODE == TG_MODE_DIAG)
+      element_diagonal<ET, MAT, T>(law, X, U, Y);
+    else if constexpr (ET == TG_HEX8)
       hex_element_modal<MAT, T, MODE>(law, X, U, W, Y);
-    else if constexpr (E::SIMPLEX && MODE != TG_MODE_DIAG)
-      simplex_element<ET, MAT, T, MODE>(law, X, U, W, Y);
     else
-      element_generic<ET, MAT, T, MODE>(law, X, U, W, Y);
+      simplex_element<ET, MAT, T, MODE>(law, X, U, W, Y);
   }
 }
 
