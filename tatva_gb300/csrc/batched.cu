@@ -131,8 +131,9 @@ struct Crew {
   // Sums of K per-thread float pairs over the crew, in a fixed order and to more than FP64's
   // precision.  Warp k adds value k for the whole CTA: a tree in every warp was more
   // instructions than the rows of a mid-size system.  finish(k, sum): lane 0 of warp k with
-  // value k's sum, the same in every CTA; what it leaves in S the threads read after the call.  A CTA may be one sum ahead of the others (its total goes to the other half),
-  // not two (the sync).  between(): work of the threads after warp K - 1 while those add.
+  // value k's sum, the same in every CTA; what it leaves in S the threads read after the
+  // call.  A CTA may be one sum ahead of the others (its total goes to the other half), not
+  // two (the sync).  between(): work of the threads after warp K - 1 while those add.
   template <int K, class F, class G>
   __device__ __forceinline__ void sum(const float2 (&v)[K], F&& between, G&& finish) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -203,7 +204,7 @@ struct Crew {
 __device__ __forceinline__ bool for_cluster(const tg_batch_desc& d, int sys) {
   const int64_t n = d.row_ofs[sys + 1] - d.row_ofs[sys];
   const int W = d.ell_width[sys];
-  return n > 0 && n <= d.max_rows && W >= 0 && 
+  return n > 0 && n <= d.max_rows && W >= 0 &&
          (n > SOLO_ROWS || n * (6 * (int64_t)W + 4) > SOLO_BYTES);
 }
 
@@ -265,8 +266,8 @@ __device__ __forceinline__ void spmv(float (&y)[NR], const float* __restrict__ p
   }
 }
 template <int NT, int P, int NR>
-__device__ __forceinline__ void spmv_pairs(int np, float (&y)[NR], const float* p, const float* sval,
-                                           const uint32_t* scol, int m, int half, int Ks, int W,
+__device__ __forceinline__ void spmv_pairs(int np, float (&y)[NR], const float* p,
+                                           const float* sval, const uint32_t* scol, int m, int half, int Ks, int W,
                                            int n, int wlo, const float* v32, const uint16_t* col) {
   if constexpr (P > 0) {
     if (np == P) return spmv<NT, P>(y, p, sval, scol, m, half, Ks, W, n, wlo, v32, col);
@@ -350,11 +351,26 @@ __device__ void solve_rows(const BatchArgs& a, int sys, float* smem, Crew<NT>& c
   // the thread's values (PP > 0); a row that does not exist holds zeros throughout
   constexpr int NR = PP ? 2 * PP : 4;
   float vr[NR] = {}, vd[NR] = {}, vg[NR] = {}, vq[NR] = {}, vp[NR] = {};
-  auto R = [&](int j, int i) -> float& { if constexpr (PP > 0) return vr[j]; else return mem[0][i]; };
-  auto D = [&](int j, int i) -> float& { if constexpr (PP > 0) return vd[j]; else return mem[1][i]; };
-  auto G = [&](int j, int i) -> float& { if constexpr (PP > 0) return vg[j]; else return mem[2][i]; };
-  auto Q = [&](int j, int i) -> float& { if constexpr (PP > 0) return vq[j]; else return mem[3][i]; };
-  auto Pv = [&](int j, int i) -> float& { if constexpr (PP > 0) return vp[j]; else return pown[i]; };
+  auto R = [&](int j, int i) -> float& {
+    if constexpr (PP > 0) return vr[j];
+    else return mem[0][i];
+  };
+  auto D = [&](int j, int i) -> float& {
+    if constexpr (PP > 0) return vd[j];
+    else return mem[1][i];
+  };
+  auto G = [&](int j, int i) -> float& {
+    if constexpr (PP > 0) return vg[j];
+    else return mem[2][i];
+  };
+  auto Q = [&](int j, int i) -> float& {
+    if constexpr (PP > 0) return vq[j];
+    else return mem[3][i];
+  };
+  auto Pv = [&](int j, int i) -> float& {
+    if constexpr (PP > 0) return vp[j];
+    else return pown[i];
+  };
   // f(j, i, exists) for the thread's rows i; with PP > 0 also for its places j without a row
   auto each = [&](auto&& f) {
     if constexpr (PP > 0) {
@@ -644,7 +660,8 @@ __device__ void solve_system(const BatchArgs& a, int sys, float* smem, Crew<NT>&
 }
 
 template <int NT, int PP, bool ALL, int PER_SM>
-__global__ void __launch_bounds__(NT, PER_SM) __cluster_dims__(TEAM, 1, 1) batch_solve_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(NT, PER_SM) __cluster_dims__(TEAM, 1, 1)
+    batch_solve_kernel(BatchArgs a) {
   extern __shared__ __align__(16) float smem[];
   __shared__ typename Crew<NT>::Shared S;
   const int me = (int)cluster_rank();
@@ -804,7 +821,8 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
   a.rel_res = rel_res;
   a.status = status;
   cudaStream_t st = as_stream(stream);
-  TG_TRY(cuda_check(cudaMemsetAsync(a.counter, 0, 2 * sizeof(unsigned), st), "tg_batch_solve: counter reset"));
+  TG_TRY(cuda_check(cudaMemsetAsync(a.counter, 0, 2 * sizeof(unsigned), st),
+                    "tg_batch_solve: counter reset"));
   int dev = 0, sms = 0;
   TG_TRY(cuda_check(cudaGetDevice(&dev), "cudaGetDevice"));
   TG_TRY(cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"));
@@ -820,7 +838,8 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
       std::lock_guard<std::mutex> g(mu);
       size_t& cur = attr[std::make_pair((const void*)kern, dev)];
       if (smem > cur) {
-        TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem),
                           "tg_batch_solve: shared memory attribute"));
         cur = smem;
       }
@@ -828,7 +847,8 @@ extern "C" int tg_batch_solve(const tg_batch_desc* desc, int64_t n_rows, const d
     int per_sm = 0;
     TG_TRY(cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem),
                       "tg_batch_solve: occupancy"));
-    if (per_sm <= 0) return set_error(TG_ERR_UNSUPPORTED, "tg_batch_solve: kernel does not fit on an SM");
+    if (per_sm <= 0)
+      return set_error(TG_ERR_UNSUPPORTED, "tg_batch_solve: kernel does not fit on an SM");
     const int want = ctas_per_sm > 0 ? std::min(ctas_per_sm, per_sm) : per_sm;
     const int clusters = std::max(1, std::min(desc->n_systems, sms * want / TEAM));
     const int grid = clusters * TEAM;

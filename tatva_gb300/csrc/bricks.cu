@@ -26,8 +26,8 @@
 // Bound: the HVP's instructions (29 us for 2.2 M nodes) and the traffic of the vector passes
 // (40 bytes a dof and step: 13 + 12 us; with d in the update, and an FP64 tree for the dots
 // in every warp, 23 + 9).  The dots' sums beyond a thread keep more than FP64's 53 bits
-// (tg_sum.h), and so do the scalars.  Restarting the inner CG at every refinement took 14,438 steps for
-// 24 requests of 16..64 a side, 170 ms with the warm-up; stages 13,134 and 130 ms.
+// (tg_sum.h), and so do the scalars.  Restarting the inner CG at every refinement took 14,438
+// steps for 24 requests of 16..64 a side, 170 ms with the warm-up; stages 13,134 and 130 ms.
 //
 // A step is `iterations` CG steps with the refinement launches before every 20th, for
 // every slot in use; a slot whose phase does not match a launch leaves it at once.  The
@@ -48,13 +48,15 @@ namespace tg {
 namespace {
 
 // A stage reduces |r| by at most STAGE_TOL before the FP64 residual replaces it.  24 requests
-// of 16..64 a side: 0.2 137 ms, 0.1 133, 0.03 130, 0.01 132 (a slot waits for the next
-// refinement launches after each stage; long stages lose the direction).
+// of 16..64 a side: 0.2 137 ms, 0.1 133, 0.03 130, 0.01 132, flat from 0.1 to 0.01 within the
+// runs' spread (a slot waits for the next refinement launches after each stage; long stages
+// lose the direction): the middle of it.
 constexpr double STAGE_TOL = 0.03;
 // Refinement launches every so many CG steps: 5 140 ms, 10 133, 20 130 (the launches cost
 // as much as two steps even where few slots take part).
 constexpr int REFINE_EVERY = 20;
-// Vector entries a CTA: 8192 135.7 ms, 4096 127.2, 3072 126.3, 2048 129.1.
+// Vector entries a CTA: 8192 135.7 ms, 4096 127.2, 3072 126.3, 2048 129.1 (the last three
+// within the runs' spread of 2 %).
 constexpr int BRICK_CHUNK = 3072;
 constexpr int BR_MAX = TG_BRICK_MAX_SLOTS;
 constexpr int PH_FREE = TG_BRICK_FREE, PH_REFINE = TG_BRICK_REFINE, PH_RUN = TG_BRICK_RUN,
@@ -180,7 +182,8 @@ __device__ __forceinline__ void copy_coefficients(GridCoef<T>* dst, const GridCo
   for (int i = threadIdx.x; i < FX; i += blockDim.x) d[i] = s[i];
   const GridPart part = grid_part(*src, b);
   const int lo = part == GRID_XFACE ? FX : (part == GRID_YFACE ? FY : KE);
-  const int hi = part == GRID_INTERIOR ? 0 : (part == GRID_XFACE ? FY : (part == GRID_YFACE ? KE : ALL));
+  const int hi =
+      part == GRID_INTERIOR ? 0 : (part == GRID_XFACE ? FY : (part == GRID_YFACE ? KE : ALL));
   for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) d[i] = s[i];
 }
 

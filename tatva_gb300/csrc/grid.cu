@@ -372,7 +372,8 @@ __global__ void __launch_bounds__(cg_threads<T>(), 1)
   double flag = G.scal[SCAL_FLAG];
   bool done = G.scal[SCAL_DONE] != 0.0;
   int it = 0;
-  const int64_t i0 = 4 * ((int64_t)blockIdx.x * NT + threadIdx.x), stride = 4 * (int64_t)gridDim.x * NT;
+  const int64_t i0 = 4 * ((int64_t)blockIdx.x * NT + threadIdx.x);
+  const int64_t stride = 4 * (int64_t)gridDim.x * NT;
   // entries i0 + j stride + 0..3 are this thread's throughout: vectors 0 (r), 1 (dinv), 2 (x), 3
   // (p) in shared memory as far as they fit
   T* const cache = reinterpret_cast<T*>(sh + NG) + 4 * threadIdx.x;
@@ -536,8 +537,9 @@ int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,
     const int64_t vbytes = (int64_t)G.slabs * 4 * NT * sizeof(T), room = CG_SMEM - tiles;
     G.cached = (int)(room / vbytes < 4 ? room / vbytes : 4);
     const int smem = tiles + (int)(G.cached * vbytes);
-    TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM),
-                      "grid CG: shared memory"));
+    TG_TRY(cuda_check(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM),
+        "grid CG: shared memory"));
     TG_TRY(cuda_check(cudaMemsetAsync(count, 0, sizeof(unsigned), st), "grid CG: barrier"));
     void* args[] = {&P, &G};
     const cudaError_t e =

@@ -242,8 +242,8 @@ __device__ __forceinline__ void element_row_block(
 // What bounds it is on chip: about 250 arithmetic instructions and 36 shared-memory adds
 // per (Tet4 element, corner) and the gathers of the element's nodes; the data is written
 // once and neither column indices nor colours are read.  Kuhn 56^3 jittered, Neo-Hookean
-// FP32 (1.05 M tets, 24 M values): 187 us, 201 without the loads run ahead; compressed Hessian and decompression, which it
-// replaces on the mesh's own pattern, 717 + 125 us.
+// FP32 (1.05 M tets, 24 M values): 187 us, 201 without the loads run ahead; compressed Hessian
+// and decompression, which it replaces on the mesh's own pattern, 717 + 125 us.
 template <int ET>
 constexpr int slot_pad() { return Elem<ET>::NN <= 4 ? 4 : 8; }
 constexpr int CSR_WARPS = 2;   // warps per CTA
@@ -252,7 +252,8 @@ constexpr int CSR_SLAB = 16;   // row words a lane hands over at a time when wri
 template <int ET, int MAT, class T>
 __global__ void __launch_bounds__(32 * CSR_WARPS)
     hessian_csr_kernel(const T* __restrict__ coords, const int32_t* __restrict__ conn,
-                       bool conn16, const T* __restrict__ u, T p0, T p1, const T* __restrict__ eparam,
+                       bool conn16, const T* __restrict__ u, T p0, T p1,
+                       const T* __restrict__ eparam,
                        int64_t n_nodes, const int32_t* __restrict__ inc_ptr,
                        const int32_t* __restrict__ inc_idx, const uint16_t* __restrict__ slots,
                        const int32_t* __restrict__ indptr, int row_words, T* __restrict__ data) {
@@ -651,7 +652,8 @@ extern "C" int tg_csr_slots(int elem, int n_vals, int64_t n_nodes, const int32_t
   if (n_vals > 3 || n_colors < 1 || n_colors > SLOT_MAX_COLORS)
     return set_error(TG_ERR_UNSUPPORTED, "tg_csr_slots: at most 3 values per node and %d colours",
                      SLOT_MAX_COLORS);
-  if (n_nodes == 0 || n_elems == 0) return set_error(TG_ERR_UNSUPPORTED, "tg_csr_slots: empty mesh");
+  if (n_nodes == 0 || n_elems == 0)
+    return set_error(TG_ERR_UNSUPPORTED, "tg_csr_slots: empty mesh");
   TG_TRY(check_ptr(conn, "conn"));
   TG_TRY(check_ptr(inc_ptr, "inc_ptr"));
   TG_TRY(check_ptr(inc_idx, "inc_idx"));

@@ -3,9 +3,10 @@
 // The reference has no solver: users compose jax.scipy.sparse.linalg.cg with the
 // matrix-free HVP (README.md:93).  Here:
 //   * CSR SpMV (layout of ColoredMatrix.to_csr, tatva/sparse/base.py:76-81)
-//   * deterministic FP64 dot products: a fixed partition (dot_chunks) and a fixed tree
-//     order, independent of the GPU and of the launch, so repeated solves are bitwise
-//     identical
+//   * deterministic dot products, so that repeated solves are bitwise identical: here a fixed
+//     partition (dot_chunks) and a fixed tree order in FP64, independent of the GPU and of
+//     the launch.  On a structured brick p.q (and, in a cooperative launch, every dot) follows
+//     the stencil's tiles and the CTAs, which are cut by the number of SMs (grid.cu)
 //   * Jacobi-preconditioned CG whose scalars never leave the device; `check_every`
 //     iterations are captured once in a CUDA graph (on a structured brick of up to
 //     GRID_CG_MAX_DOFS unknowns: run as one cooperative launch) and replayed between host

@@ -70,7 +70,9 @@ __device__ __forceinline__ void load_run(const T* p, T (&v)[N]) {
 // that subtract a corner's value first turn one infinite nodal value into NaN all over its
 // element, and overflow from an eighth of the largest number on; an element with such a result
 // is done again as the weighted sum that defines it.
-__device__ __forceinline__ unsigned magnitude_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned magnitude_bits(float v) {
+  return __float_as_uint(v) & 0x7fffffffu;
+}
 __device__ __forceinline__ unsigned magnitude_bits(double v) {
   return (unsigned)__double2hiint(v) & 0x7fffffffu;
 }

@@ -39,9 +39,9 @@ __device__ __forceinline__ void stv(double* p, const double (&v)[4]) {
 // FP32 vectors: each thread accumulates x_i y_i as an unevaluated pair (hi, lo) of
 // floats -- the product is split exactly with an FMA and added with a two-sum, so the
 // thread's partial keeps about 48 bits -- and only the per-thread partials enter the
-// tree reduction, in FP64 or in three floats (Sum3).  (This GPU's FP64 rate is a small fraction of FP32: per-element
-// FP64 conversions and multiply-adds made the dots several times slower than their
-// memory traffic.)  FP64 vectors accumulate in FP64.
+// tree reduction, in FP64 or in three floats (Sum3).  (This GPU's FP64 rate is a small
+// fraction of FP32: per-element FP64 conversions and multiply-adds made the dots several
+// times slower than their memory traffic.)  FP64 vectors accumulate in FP64.
 template <class T>
 struct DotAcc;
 template <>

@@ -25,8 +25,8 @@
 //
 // Schedule (one launch):
 //   * interior CTAs: a tile of 32 x 8 node columns (x, y) and a run of z planes.  Each
-//     thread owns one column (FP32: two, below) and sweeps z; the input plane (with a one-node halo, 34 x
-//     10 nodes, 3 components in a 16-byte slot) sits in shared memory; a plane adds its
+//     thread owns one column (FP32: two, below) and sweeps z; the input plane (with a
+//     one-node halo, 34 x 10 nodes, 3 components in a 16-byte slot) sits in shared memory; a plane adds its
 //     contributions to the outputs at z - 1, z, z + 1 (three accumulator sets), so each
 //     output is complete after its upper neighbour plane.  Planes arrive through
 //     registers two planes ahead (the Dirichlet mask is applied on the way) and are
@@ -115,7 +115,7 @@ struct GridCoef {
   T kxz[2], kyz[2];  // (lambda - mu)/4 M_y, M_x: the z faces' own-plane coupling
   int nx, ny, nz;    // nodes per axis
   int tiles_x, tiles_y, tiles_z, tz;  // tiling of the interior columns: tz planes per tile
-  int n_edge_ctas, edge_lanes;  // nodes on two or three faces, edge_lanes lanes each
+  int edge_lanes;        // lanes of a node on two or three faces
   int n_yface_ctas;      // y face nodes, one per thread
   int xt_y, xt_z;        // x-face patches per face along y and z
   int n_xface_ctas;      // 2 xt_y xt_z
@@ -163,7 +163,9 @@ __device__ __forceinline__ constexpr bool masks_input() {
 // p.q (or r.r) of a grid launch: per node the three products summed in T (FMAs), the node
 // sums accumulated in a fixed order -- FP64 in FP64; FP32 as an unevaluated float pair (one
 // two-sum per node, exact to 48 bits): a conversion and an addition in FP64 per node held
-// the FP64 pipe, 64 cycles a warp instruction, about as long as the stencil takes.
+// the FP64 pipe, 64 cycles a warp instruction, about as long as the stencil takes.  The error
+// of p.q is the node sums' rounding, 2^-24 each, with either (simulated: 9.4e-11 of the whole
+// at 200,000 nodes, the two 2e-18 apart).
 template <class T>
 struct GridDotAcc;
 template <>
@@ -464,8 +466,9 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
 // next to each other, so a neighbour costs one 16-byte and one 8-byte shared load for the
 // pair.  Planes arrive by 4-byte cp.async, GP_STAGES - 1 ahead, without holding registers;
 // one barrier per plane.
-// HVP of a brick without / with a Dirichlet mask, against a column per thread staged through
-// registers and element-matrix sums on all faces: 64^3 7.3 / 9.8 -> 6.6 / 8.9 us, 96^3 15.2 /
+// HVP of a brick without / with a Dirichlet mask, the launch alone (graph replays; the call at
+// 128^3 takes 32.8 us), against a column per thread staged through registers and
+// element-matrix sums on all faces: 64^3 7.3 / 9.8 -> 6.6 / 8.9 us, 96^3 15.2 /
 // 22.0 -> 12.8 / 18.2, 128^3 26.8 / 39.0 -> 22.7 / 30.5 us.  f32x2 runs at the scalar lane
 // rate on this chip (128 lane operations a clock and SM); what it saves is issue slots, of
 // which a plane of 64 nodes takes 330 (18 shared loads, 10 copies, 143 on the FMA pipe).
@@ -747,7 +750,8 @@ __device__ void grid_interior_pair(const GridCoef<float>& P, int item,
   for (int p = ps; p <= pe; ++p) {
     asm volatile("cp.async.wait_group %0;" ::"n"(GP_STAGES - 2) : "memory");
     apply_masks(p, st);
-    group_sync<float, COH>();  // plane p complete; every thread is done with the stage refilled below
+    // plane p complete; every thread is done with the stage refilled below
+    group_sync<float, COH>();
     issue(p + GP_STAGES - 1, (st + GP_STAGES - 1) % GP_STAGES);
     if constexpr (MASK_IN) load_masks(p + 1);
     const GridPairStage& S = stage[st];
@@ -901,7 +905,8 @@ __device__ void grid_yface(const GridCoef<T>& P, int64_t t0, const T* __restrict
         const T v2 = (m & 4) ? T(0) : ld_in<COH>(in + 3 * g + 2);
 #pragma unroll
         for (int a = 0; a < 3; ++a)
-          acc[a] = fma(P.fy[S][row][j][a][2], v2, fma(P.fy[S][row][j][a][1], v1, fma(P.fy[S][row][j][a][0], v0, acc[a])));
+          acc[a] = fma(P.fy[S][row][j][a][2], v2,
+                       fma(P.fy[S][row][j][a][1], v1, fma(P.fy[S][row][j][a][0], v0, acc[a])));
       }
   };
   if (high) stencil(std::integral_constant<int, 1>{});
@@ -955,7 +960,8 @@ __device__ void grid_xface(const GridCoef<T>& P, int item, const T* __restrict__
         const V4 v = sm[2 * ((lz + j / 3) * GR_XS + ly + j % 3) + col];
 #pragma unroll
         for (int a = 0; a < 3; ++a)
-          acc[a] = fma(P.fx[S][col][j][a][2], v.z, fma(P.fx[S][col][j][a][1], v.y, fma(P.fx[S][col][j][a][0], v.x, acc[a])));
+          acc[a] = fma(P.fx[S][col][j][a][2], v.z,
+                       fma(P.fx[S][col][j][a][1], v.y, fma(P.fx[S][col][j][a][0], v.x, acc[a])));
       }
   };
   if (face) stencil(std::integral_constant<int, 1>{});
@@ -1117,8 +1123,8 @@ static int grid_sm_count() {
 }
 
 // Coefficients and tiling of a brick of nodes[0] x nodes[1] x nodes[2] nodes with
-// spacings h; returns the launch's CTA count (edge and face CTAs first, then the interior
-// tiles), or -1 when it does not fit an int.
+// spacings h; returns the launch's CTA count (grid_cta's order: interior tiles, x faces, y
+// faces, edges), or -1 when it does not fit an int.
 // deep: always GR_DEEP_TZ planes per tile (launches shared by many bricks need no spreading
 // of one brick over the SMs, and deeper tiles reload fewer halo planes).
 // groups > 0: the tiles and faces are shared out among that many groups at once (the
@@ -1182,7 +1188,6 @@ static int64_t grid_setup_dims(const int32_t nodes[3], const double h[3], double
   P.tiles_z = (int)tiles_of(tz);
   const int64_t n_int = columns * P.tiles_z;
   if (n_int + faces > 0x7fffffff) return -1;
-  P.n_edge_ctas = (int)n_edge;
   P.n_yface_ctas = (int)n_y;
   P.n_xface_ctas = (int)n_x;
   return n_int + faces;

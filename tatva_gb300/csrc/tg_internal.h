@@ -35,12 +35,12 @@ int launch_grid_hvp_dot(const tg_block_plan* plan, int prec, double mu, double l
 // bits.  (Results do not depend on where a solve is cut into launches.)
 bool grid_cg_persistent(const tg_block_plan* plan);
 constexpr int GRID_CG_MAX_ITERS = 1 << 16;
-// `iters` <= GRID_CG_MAX_ITERS CG iterations (fewer when they converge or break down) from the residual r, the
-// direction p and the scalars scal (SCAL_*) on a structured brick, as one cooperative
-// launch; part: 2 DOT_CHUNKS doubles, count: one counter.  node_mask: NULL, or one byte per
-// node, bit d set when dof 3 n + d is fixed (pack_node_mask from the C ABI's per-dof mask);
-// p and dinv are zero on fixed dofs (grid_cg_fixed).  TG_ERR_UNSUPPORTED (nothing launched)
-// where the CTAs cannot all be resident.
+// `iters` <= GRID_CG_MAX_ITERS CG iterations (fewer when they converge or break down) from the
+// residual r, the direction p and the scalars scal (SCAL_*) on a structured brick, as one
+// cooperative launch; part: 2 DOT_CHUNKS doubles, count: one counter.  node_mask: NULL, or one
+// byte per node, bit d set when dof 3 n + d is fixed (pack_node_mask from the C ABI's per-dof
+// mask); p and dinv are zero on fixed dofs (grid_cg_fixed).  TG_ERR_UNSUPPORTED (nothing
+// launched) where the CTAs cannot all be resident.
 int launch_grid_cg(const tg_block_plan* plan, int prec, double mu, double lam,
                    const uint8_t* node_mask, void* x, void* r, void* p, void* q, const void* dinv,
                    double* scal, double* part, unsigned* count, int iters, cudaStream_t st);
