@@ -246,7 +246,7 @@ __device__ __forceinline__ void element_row_block(
 // and decompression, which it replaces on the mesh's own pattern, 717 + 125 us.
 template <int ET>
 constexpr int slot_pad() { return Elem<ET>::NN <= 4 ? 4 : 8; }
-constexpr int CSR_WARPS = 2;   // warps per CTA
+constexpr int CSR_WARPS = 2;   // warps per CTA, at most (csr_warps)
 constexpr int CSR_SLAB = 16;   // row words a lane hands over at a time when writing
 
 template <int ET, int MAT, class T>
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(32 * CSR_WARPS)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T* acc = reinterpret_cast<T*>(smem_raw) + (size_t)warp * row_words * 32;
-  const int64_t n = ((int64_t)blockIdx.x * CSR_WARPS + warp) * 32 + lane;
+  const int64_t n = ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * 32 + lane;
   const bool live = n < n_nodes;
   const int base = live ? __ldg(indptr + V * n) : 0;
   const int len = live ? __ldg(indptr + V * n + V) - base : 0;
@@ -687,6 +687,22 @@ static int csr_row_words(int V, int max_deg) {
   return (V * V * max_deg + CSR_SLAB - 1) / CSR_SLAB * CSR_SLAB;
 }
 
+// Warps of a CTA of hessian_csr_kernel with `warp_bytes` of row blocks a warp: the ones that
+// leave more warps on an SM.  FP64 Hex8 (65 KB a warp for three values: three CTAs of one warp
+// where one of two fits), Linear-Elastic 22^3 1,316 us with two and 877 with one, 30^3 2,625 and
+// 1,757, 48^3 10,504 and 7,017.  Where the count is about the same, FP64 Hex8 takes one, for a
+// last wave in finer grains (Poisson 24^3 395 and 374, 30^3 729 and 664, 48^3 2,326 and 2,320),
+// and the others two: an SM holds 32 CTAs at most (Tet4 Poisson 56^3 FP32 52 us and 67 with
+// one, Hex8 Linear-Elastic 36^3 FP32 112 and 120).
+static int csr_warps(int elem, int prec, size_t warp_bytes, int sm_bytes) {
+  auto resident = [&](int w) {
+    const int64_t ctas = sm_bytes / (int64_t)(w * warp_bytes + 1024);
+    return w * (ctas < 32 ? ctas : 32);
+  };
+  const int64_t one = resident(1), two = resident(CSR_WARPS);
+  return one > two || (one * 10 >= two * 9 && elem == TG_HEX8 && prec == TG_F64) ? 1 : CSR_WARPS;
+}
+
 extern "C" int tg_hessian_csr(int elem, int prec, const tg_material* mat, const void* coords,
                               int64_t n_nodes, const int32_t* conn, int64_t n_elems,
                               const void* u, const int32_t* inc_ptr, const int32_t* inc_idx,
@@ -706,8 +722,11 @@ extern "C" int tg_hessian_csr(int elem, int prec, const tg_material* mat, const 
   TG_TRY(check_ptr(data, "data"));
   if (reinterpret_cast<uintptr_t>(slots) % 16 != 0)
     return set_error(TG_ERR_VALUE, "tg_hessian_csr: slots must be 16-byte aligned");
-  int dev = 0, cta_bytes = 0;
+  int dev = 0, cta_bytes = 0, sm_bytes = 0;
   TG_TRY(cuda_check(cudaGetDevice(&dev), "tg_hessian_csr: device"));
+  TG_TRY(cuda_check(
+      cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev),
+      "tg_hessian_csr: shared memory per SM"));
   TG_TRY(cuda_check(cudaDeviceGetAttribute(&cta_bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
                     "tg_hessian_csr: shared memory per CTA"));
   const size_t word = prec == TG_F32 ? 4 : 8;
@@ -727,12 +746,14 @@ extern "C" int tg_hessian_csr(int elem, int prec, const tg_material* mat, const 
           constexpr int V = LawDims<MAT, Elem<ET>::D>::V;
           if (!Law<MAT, Elem<ET>::D, T>::LINEAR) TG_TRY(check_ptr(u, "u"));
           const int words = csr_row_words(V, max_deg);
-          const size_t smem = (size_t)words * 32 * CSR_WARPS * sizeof(T);
+          const int warps =
+              csr_warps(elem, prec, (size_t)words * 32 * sizeof(T), sm_bytes);
+          const size_t smem = (size_t)words * 32 * warps * sizeof(T);
           auto kern = hessian_csr_kernel<ET, MAT, T>;
           TG_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem),
                             "tg_hessian_csr: shared memory"));
-          kern<<<grid_for(n_nodes, 32 * CSR_WARPS), 32 * CSR_WARPS, smem, st>>>(
+          kern<<<grid_for(n_nodes, 32 * warps), 32 * warps, smem, st>>>(
               (const T*)coords, conn, reinterpret_cast<uintptr_t>(conn) % 16 == 0, (const T*)u,
               (T)mat->p0, (T)mat->p1, (const T*)mat->elem_param, n_nodes, inc_ptr, inc_idx, slots,
               indptr, words, (T*)data);
