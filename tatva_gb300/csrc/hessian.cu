@@ -366,21 +366,24 @@ __global__ void __launch_bounds__(32 * CSR_WARPS)
 // Checks that a CSR pattern has the form hessian_csr_kernel writes and that a colouring
 // separates its columns: per node, V rows of the same ascending columns in groups of V
 // dofs of one node, all of different colours (then Jc[i, colour(j)] is H[i, j] alone).
-// info[0] |= 1 where it does not; info[1]: the most columns (nodes) of a row.  A warp per
-// node; the colours seen so far as bits in shared memory.
+// info[0] |= 1 where it does not; info[1]: the most columns (nodes) of a row.  CHECK_LANES
+// lanes per node (rows of 7 to 81 columns); the colours seen so far as bits in shared memory.
+// A node whose row is no longer than info[1] already was leaves it alone: one address, and
+// most rows have the same length.
 constexpr int SLOT_MAX_COLORS = 1024;
+constexpr int CHECK_LANES = 8, CHECK_NODES = 128 / CHECK_LANES;
 template <int V>
 __global__ void __launch_bounds__(128)
     csr_pattern_check_kernel(int64_t n_nodes, int64_t nnz, const int32_t* __restrict__ indptr,
                              const int32_t* __restrict__ indices,
                              const int32_t* __restrict__ colors, int n_colors,
                              int32_t* __restrict__ info) {
-  __shared__ unsigned seen[4][SLOT_MAX_COLORS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t n = (int64_t)blockIdx.x * 4 + warp;
-  if (n >= n_nodes) return;
-  for (int k = lane; k < SLOT_MAX_COLORS / 32; k += 32) seen[warp][k] = 0u;
+  __shared__ unsigned seen[CHECK_NODES][SLOT_MAX_COLORS / 32 + 1];
+  const int lane = threadIdx.x % CHECK_LANES, own = threadIdx.x / CHECK_LANES;
+  const int64_t n = (int64_t)blockIdx.x * CHECK_NODES + own;
+  for (int k = lane; k < SLOT_MAX_COLORS / 32; k += CHECK_LANES) seen[own][k] = 0u;
   __syncwarp();
+  if (n >= n_nodes) return;
   const int64_t N = n_nodes * V;
   const int64_t r0 = __ldg(indptr + V * n);
   const int64_t L = __ldg(indptr + V * n + 1) - r0;
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(128)
     good = good && (__ldg(indptr + V * n + i + 1) - __ldg(indptr + V * n + i) == L);
   if (n == n_nodes - 1) good = good && r0 + V * L == nnz;
   if (good) {
-    for (int64_t p = lane; p < L; p += 32) {
+    for (int64_t p = lane; p < L; p += CHECK_LANES) {
       const int64_t c = __ldg(indices + r0 + p);
       bool ok = c >= 0 && c < N;
       for (int i = 1; i < V; ++i) ok = ok && __ldg(indices + r0 + i * L + p) == c;
@@ -398,45 +401,54 @@ __global__ void __launch_bounds__(128)
       if (ok) {
         const int col = __ldg(colors + c);
         ok = col >= 0 && col < n_colors;
-        if (ok) ok = !(atomicOr(&seen[warp][col >> 5], 1u << (col & 31)) >> (col & 31) & 1u);
+        if (ok) ok = !(atomicOr(&seen[own][col >> 5], 1u << (col & 31)) >> (col & 31) & 1u);
       }
       good = good && ok;
     }
   }
   if (!good) atomicOr(info, 1);
-  if (lane == 0 && good) atomicMax(info + 1, (int)(L / V));
+  if (lane == 0 && good && (int)(L / V) > *(volatile int32_t*)(info + 1))
+    atomicMax(info + 1, (int)(L / V));
 }
 
-// slots of the incidence entries (a thread per node); info[0] |= 2 where a node of an
+// slots of the incidence entries (a thread per entry); info[0] |= 2 where a node of an
 // element is not among the columns.  Runs after the check, on rows it found ascending.
+// Bound: the chain of dependent loads of the searches; a thread per node went through them
+// one after another.  Jacobian made and called once with this and the check, FP32 Poisson:
+// Kuhn 40^3 292 -> 139 us, Tri3 400^2 275 -> 122 (the compressed Hessian's: 145 and 132).
 template <int ET, int V>
-__global__ void csr_slots_kernel(int64_t n_nodes, const int32_t* __restrict__ conn,
+__global__ void csr_slots_kernel(int64_t n_nodes, int64_t n_entries,
+                                 const int32_t* __restrict__ conn,
                                  const int32_t* __restrict__ inc_ptr,
                                  const int32_t* __restrict__ inc_idx,
                                  const int32_t* __restrict__ indptr,
                                  const int32_t* __restrict__ indices,
                                  uint16_t* __restrict__ slots, int32_t* __restrict__ info) {
   constexpr int NN = Elem<ET>::NN, NP = slot_pad<ET>();
-  const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= n_nodes || (*(volatile int32_t*)info & 1)) return;
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n_entries || j >= __ldg(inc_ptr + n_nodes) || (*(volatile int32_t*)info & 1)) return;
+  const int64_t ea = __ldg(inc_idx + j), n = __ldg(conn + ea);
   const int64_t r0 = __ldg(indptr + V * n);
   const int deg = (int)((__ldg(indptr + V * n + 1) - r0) / V);
-  for (int j = __ldg(inc_ptr + n); j < __ldg(inc_ptr + n + 1); ++j) {
-    const int64_t e = __ldg(inc_idx + j) / NN;
-    for (int b = 0; b < NN; ++b) {
-      const int64_t want = (int64_t)V * __ldg(conn + e * NN + b);
-      int lo = 0, hi = deg;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(indices + r0 + (int64_t)V * mid) < want) lo = mid + 1;
-        else hi = mid;
-      }
-      const bool found = lo < deg && lo < 65536 && __ldg(indices + r0 + (int64_t)V * lo) == want;
-      if (!found) atomicOr(info, 2);
-      slots[(int64_t)j * NP + b] = (uint16_t)(found ? lo : 0);
+  alignas(8) uint16_t row[NP];
+#pragma unroll
+  for (int b = 0; b < NP; ++b) {
+    row[b] = 0;
+    if (b >= NN) continue;
+    const int64_t want = (int64_t)V * __ldg(conn + ea / NN * NN + b);
+    int lo = 0, hi = deg;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(indices + r0 + (int64_t)V * mid) < want) lo = mid + 1;
+      else hi = mid;
     }
-    for (int b = NN; b < NP; ++b) slots[(int64_t)j * NP + b] = 0;
+    const bool found = lo < deg && lo < 65536 && __ldg(indices + r0 + (int64_t)V * lo) == want;
+    if (!found) atomicOr(info, 2);
+    row[b] = (uint16_t)(found ? lo : 0);
   }
+#pragma unroll
+  for (int b = 0; b < NP; b += 4)
+    *reinterpret_cast<uint2*>(slots + j * NP + b) = *reinterpret_cast<const uint2*>(row + b);
 }
 
 // Thread t of the CTA owns node n0 + t.  ACC_SMEM: its V x C row block sits in shared
@@ -670,10 +682,11 @@ extern "C" int tg_csr_slots(int elem, int n_vals, int64_t n_nodes, const int32_t
     constexpr int ET = decltype(et)::value;
     auto go = [&](auto vc) -> int {
       constexpr int V = decltype(vc)::value;
-      csr_pattern_check_kernel<V><<<grid_for(n_nodes, 4), 128, 0, st>>>(
+      csr_pattern_check_kernel<V><<<grid_for(n_nodes, CHECK_NODES), 128, 0, st>>>(
           n_nodes, nnz, indptr, indices, colors, n_colors, info);
-      csr_slots_kernel<ET, V><<<grid_for(n_nodes, 128), 128, 0, st>>>(
-          n_nodes, conn, inc_ptr, inc_idx, indptr, indices, slots, info);
+      const int64_t entries = n_elems * Elem<ET>::NN;
+      csr_slots_kernel<ET, V><<<grid_for(entries, 128), 128, 0, st>>>(
+          n_nodes, entries, conn, inc_ptr, inc_idx, indptr, indices, slots, info);
       return launch_check("tg_csr_slots");
     };
     if (n_vals == 1) return go(IntC<1>{});

@@ -210,6 +210,8 @@ class Energy:
                   ptr(Jc), stream())
         return Jc
 
+    MAX_COLORS = 1024  # of csr_slots
+
     def csr_slots(self, colored_matrix, n_colors: int):
         """(slots, max_deg) for ``tangent_csr`` on the pattern and colouring of
         ``colored_matrix``, or None where it takes the compressed Hessian: patterns that are
@@ -217,7 +219,7 @@ class Energy:
         row's columns, rows too long for shared memory."""
         cm, op, V = colored_matrix, self.op, self.n_values
         index = (cm.indptr, cm.indices, cm.colors)
-        if (op.n_elements == 0 or not 1 <= n_colors <= 1024
+        if (op.n_elements == 0 or not 1 <= n_colors <= self.MAX_COLORS
                 or tuple(cm.shape) != (self.n_dofs, self.n_dofs)
                 or not all(t.is_cuda and t.dtype == torch.int32 and t.is_contiguous()
                            for t in index)

@@ -174,18 +174,21 @@ def jacfwd(fn: Callable, colored_matrix: ColoredMatrix, *, color_batch_size: int
     """Sparse Jacobian of ``fn`` on the pattern of ``colored_matrix`` (base.py:139-176)."""
     from .materials import Energy
 
-    nb_colors = colored_matrix.n_colors
     require_cuda(colored_matrix.indptr)
     energy = _fused_energy(fn)
-    # a fused energy on a pattern of its mesh: the values straight from the element tangents
-    slots = (energy.csr_slots(colored_matrix, nb_colors) if isinstance(energy, Energy)
+    # a fused energy on a pattern of its mesh: the values straight from the element tangents.
+    # The number of colours is a read from the device that only the other route needs
+    # (csr_slots refuses colours of MAX_COLORS and above by itself).
+    slots = (energy.csr_slots(colored_matrix, Energy.MAX_COLORS) if isinstance(energy, Energy)
              else None)
+    nb_colors = colored_matrix.n_colors if slots is None else None
     row_colors = compute_rows_cols(colored_matrix) if slots is None else None
 
     def _wrapped_jacfwd(u: torch.Tensor, *args, **kwargs) -> ColoredMatrix:
         if slots is not None and not args and not kwargs:
             return replace(colored_matrix, data=energy.tangent_csr(u, colored_matrix, slots))
-        Jc = colored_jacobian(fn, u, colored_matrix.colors, nb_colors, color_batch_size, *args,
+        n_colors = colored_matrix.n_colors if nb_colors is None else nb_colors
+        Jc = colored_jacobian(fn, u, colored_matrix.colors, n_colors, color_batch_size, *args,
                               **kwargs)
         rows, col_colors = row_colors or compute_rows_cols(colored_matrix)
         return replace(colored_matrix, data=decompress(Jc, rows, col_colors))
