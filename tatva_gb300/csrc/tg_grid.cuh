@@ -262,14 +262,21 @@ __device__ __forceinline__ void stencil_plane(const GridCoef<T>& P,
   const T ym[3] = {v[0][1].x, v[0][1].y, v[0][1].z}, yp[3] = {v[2][1].x, v[2][1].y, v[2][1].z};
   const T mm[3] = {v[0][0].x, v[0][0].y, v[0][0].z}, pm[3] = {v[0][2].x, v[0][2].y, v[0][2].z};
   const T mp[3] = {v[2][0].x, v[2][0].y, v[2][0].z}, pp[3] = {v[2][2].x, v[2][2].y, v[2][2].z};
-  T own[3];  // to the outputs in this plane
+  // a face plane adds half of these sums to the outputs in it (and the terms at the end): what
+  // was there before enters twice and the whole is halved, both exact, so that the other
+  // planes pay nothing for it (sums of their own cost 3 of 93 FP64 instructions)
+  if (side) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) accP[a] += accP[a];
+  }
   // diagonal blocks grouped by |dx|, |dy|
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     ctr[a] = a0[a];
     const T gx = xm[a] + xp[a], gy = ym[a] + yp[a];
     const T gc = (mm[a] + mp[a]) + (pm[a] + pp[a]);
-    own[a] = fma(P.c[a][3], gc, fma(P.c[a][2], gy, fma(P.c[a][1], gx, P.c[a][0] * a0[a])));
+    accP[a] = fma(P.c[a][3], gc,
+                  fma(P.c[a][2], gy, fma(P.c[a][1], gx, fma(P.c[a][0], a0[a], accP[a]))));
     const T s1 = fma(P.c[a][7], gc, fma(P.c[a][6], gy, fma(P.c[a][5], gx, P.c[a][4] * a0[a])));
     accM[a] += s1;
     accN[a] += s1;
@@ -277,24 +284,12 @@ __device__ __forceinline__ void stencil_plane(const GridCoef<T>& P,
   // x-y blocks: C = qxy(|dz|) dx dy, the cross sum of the in-plane corners
   const T wx = (pp[0] - pm[0]) - (mp[0] - mm[0]);
   const T wy = (pp[1] - pm[1]) - (mp[1] - mm[1]);
-  own[0] = fma(P.qxy[0], wy, own[0]);
+  accP[0] = fma(P.qxy[0], wy, accP[0]);
   accM[0] = fma(P.qxy[1], wy, accM[0]);
   accN[0] = fma(P.qxy[1], wy, accN[0]);
-  own[1] = fma(P.qxy[0], wx, own[1]);
+  accP[1] = fma(P.qxy[0], wx, accP[1]);
   accM[1] = fma(P.qxy[1], wx, accM[1]);
   accN[1] = fma(P.qxy[1], wx, accN[1]);
-  if (side) {  // half the interior's own-plane entries and the corner entries of G_z
-    const T sg = T(side);
-    const T zx = fma(P.kxz[1], ((pm[2] - mm[2]) + (pp[2] - mp[2])), P.kxz[0] * (xp[2] - xm[2]));
-    const T xx = fma(P.kxz[1], ((pm[0] - mm[0]) + (pp[0] - mp[0])), P.kxz[0] * (xp[0] - xm[0]));
-    const T zy = fma(P.kyz[1], ((mp[2] - mm[2]) + (pp[2] - pm[2])), P.kyz[0] * (yp[2] - ym[2]));
-    const T yy = fma(P.kyz[1], ((mp[1] - mm[1]) + (pp[1] - pm[1])), P.kyz[0] * (yp[1] - ym[1]));
-    own[0] = fma(sg, zx, T(0.5) * own[0]);
-    own[1] = fma(sg, zy, T(0.5) * own[1]);
-    own[2] = fma(-sg, xx + yy, T(0.5) * own[2]);
-  }
-#pragma unroll
-  for (int a = 0; a < 3; ++a) accP[a] += own[a];
   // x-z blocks: C = qxz(|dy|) dx dz: odd in x, summed over dy with M_y
   const T uz_x = fma(P.qxz[1], ((pm[2] - mm[2]) + (pp[2] - mp[2])), P.qxz[0] * (xp[2] - xm[2]));
   const T ux_x = fma(P.qxz[1], ((pm[0] - mm[0]) + (pp[0] - mp[0])), P.qxz[0] * (xp[0] - xm[0]));
@@ -310,6 +305,16 @@ __device__ __forceinline__ void stencil_plane(const GridCoef<T>& P,
   accN[1] -= uz_y;
   accM[2] += uy_y;
   accN[2] -= uy_y;
+  if (side) {  // half the interior's own-plane entries and the corner entries of G_z
+    const T sg = T(side);
+    const T zx = fma(P.kxz[1], ((pm[2] - mm[2]) + (pp[2] - mp[2])), P.kxz[0] * (xp[2] - xm[2]));
+    const T xx = fma(P.kxz[1], ((pm[0] - mm[0]) + (pp[0] - mp[0])), P.kxz[0] * (xp[0] - xm[0]));
+    const T zy = fma(P.kyz[1], ((mp[2] - mm[2]) + (pp[2] - pm[2])), P.kyz[0] * (yp[2] - ym[2]));
+    const T yy = fma(P.kyz[1], ((mp[1] - mm[1]) + (pp[1] - pm[1])), P.kyz[0] * (yp[1] - ym[1]));
+    accP[0] = fma(sg, zx, T(0.5) * accP[0]);
+    accP[1] = fma(sg, zy, T(0.5) * accP[1]);
+    accP[2] = fma(-sg, xx + yy, T(0.5) * accP[2]);
+  }
 }
 
 // Tile of interior columns: thread (lx, ly) owns node column (x0 + lx, y0 + ly), planes
@@ -379,8 +384,14 @@ __device__ void grid_interior(const GridCoef<T>& P, int item, const T* __restric
   const int c0 = (lx + 1) + GR_PX * (ly + 1);
 
   T ctr[3];  // the column's value in the current plane
+  // A warp whose row of columns is outside the grid has nothing to add: its arithmetic would
+  // only take the FP64 pipe from the others' (4^3, three of eight rows exist: HVP 23 -> 13 us;
+  // in the persistent CG, whose CTAs hold one tile, the branch costs 3 % at 96^3).  A face
+  // plane that is another tile's output counts as an inner one.
+  const bool row = COH || yy <= ny - 2;
   auto plane_step = [&](const V4* buf, int p) {
-    stencil_plane<T>(P, buf, c0, accM, accP, accN, ctr, p == 0 ? 1 : (p == nz - 1 ? -1 : 0));
+    const int side = p == 0 && zs == 0 ? 1 : (p == nz - 1 && ze == nz ? -1 : 0);
+    if (row) stencil_plane<T>(P, buf, c0, accM, accP, accN, ctr, side);
   };
 
   // pc: the node's own input (the column's value in the output plane, masked): with
@@ -765,7 +776,9 @@ __device__ void grid_interior_pair(const GridCoef<float>& P, int item,
     m_out = out_mask(p);
     const f2 pc[3] = {prev[0], prev[1], prev[2]};  // the pair's values in plane p - 1
     f2 out[3];
-    pair_plane(K, S, c0, below, here, prev, out, p == 0 ? 1 : (p == nz - 1 ? -1 : 0));
+    // (a face plane that is another tile's output counts as an inner one)
+    pair_plane(K, S, c0, below, here, prev, out,
+               p == 0 && zs == 0 ? 1 : (p == nz - 1 && ze == nz ? -1 : 0));
     if (p > zs) emit(p - 1, out, pc, m_now);
     st = (st + 1) % GP_STAGES;
   }
@@ -1162,14 +1175,25 @@ static int64_t grid_setup_dims(const int32_t nodes[3], const double h[3], double
       tz = (2 * columns * nz + 5 * sms - 1) / (5 * sms);
       tz = tz < 2 ? 2 : (tz > GR_MAX_TZ ? GR_MAX_TZ : tz);
     } else {
-      // Two CTAs share an SM's FP64 pipe: the fewest planes for the busiest SM (with one tile
-      // per SM some still hold two of the launch's CTAs).  HVP at 64^3: 4 planes 86 us, 6
-      // planes 112; 96^3: 13 planes 217 us, 25 planes 339; 128^3: 19 planes 448 us, 13
-      // planes 497.
+      // Two CTAs share an SM's FP64 pipe: the fewest planes for the busiest SM, in sweep steps
+      // (7.2 us each).  One tile per SM costs a step and a half more at most where face CTAs
+      // and a short last layer are its neighbours, and 1.6 times its own steps where these
+      // are so many that some SMs hold two tiles.  HVP with a mask: 24^3 1 plane 23.9 us, 2
+      // planes 31.1; 38^3 4 planes 46.3, 2 planes 57.7; 50^3 5 planes 63.7, 3 planes 71.2;
+      // 64^3 7 planes 79.8, 4 planes 85.5; 96^3 13 planes 218, 25 planes 339; 128^3 19
+      // planes 451, 13 planes 497.
       double best = -1.0;
-      for (int64_t c = 2; c <= 24; ++c) {
-        const int64_t r = (columns * tiles_of(c) + sms - 1) / sms;
-        const double cost = (r <= 1 ? 1.6 : (double)r) * (double)(c + 2);
+      for (int64_t c = 1; c <= 24; ++c) {
+        const int64_t tiles = columns * tiles_of(c), last = nz % c;
+        const int64_t full = columns * (last == 1 || last == 2 ? nz / c : tiles_of(c));
+        const double steps = (double)(c + 2);
+        double cost;
+        if (full <= sms && 4 * (tiles + faces) <= 7 * sms) {
+          cost = tiles + faces <= sms ? steps : steps + (steps < 6.0 ? steps / 4 : 1.5);
+        } else {
+          const int64_t r = (tiles + sms - 1) / sms;
+          cost = (r <= 1 ? 1.6 : (double)r) * steps;
+        }
         if (best < 0.0 || cost < best) {
           best = cost;
           tz = c;
