@@ -26,8 +26,8 @@
 // Schedule (one launch):
 //   * interior CTAs: a tile of 32 x 8 node columns (x, y) and a run of z planes.  Each
 //     thread owns one column (FP32: two, below) and sweeps z; the input plane (with a
-//     one-node halo, 34 x 10 nodes, 3 components in a 16-byte slot) sits in shared memory; a plane adds its
-//     contributions to the outputs at z - 1, z, z + 1 (three accumulator sets), so each
+//     one-node halo, 34 x 10 nodes, 3 components in a 16-byte slot) sits in shared memory; a
+//     plane adds its contributions to the outputs at z - 1, z, z + 1 (three accumulator sets), so each
 //     output is complete after its upper neighbour plane.  Planes arrive through
 //     registers two planes ahead (the Dirichlet mask is applied on the way) and are
 //     double-buffered in shared memory: one barrier per plane.  Per node and plane:
